@@ -8,89 +8,208 @@
 // between layers.  torch's Conv1d is a cross-correlation:
 //   out[co][x] = b[co] + sum_ci sum_k W[co][ci][k] in[ci][(x + k - 2) mod N].
 //
-// Layout: one CTA holds R = max(1, 512 / N) rows, N threads per row.  The
-// solver stage keeps one cell per thread (the wide-row layout of
-// burgers_kernels.cuh, stages through a shared row).  In the convolution
-// stages thread g computes 4 output channels (group g / (N/8)) x 8 contiguous
-// cells (8 * (g % (N/8)) ...): per input channel it reads 12 activations as
-// three float4 and 20 weights as five broadcast float4, then does 160 FMAs.
-// Activations live in shared memory, two buffers of [R][32][row], cell x of a
-// row at apad(x + 2) with x in [-2, N + 2) (the circular halo is stored); the
-// 4-float pad per 32 makes the float4 reads conflict-free.  All weights
-// (42.6 KB) sit in shared memory for the whole launch.
-#include "burgers_cnn.cuh"
+// Layout: one thread per cell, one row per CTA (two for rows of 64 cells).  The first
+// layer (5 products per channel) and the last (5 partial sums per cell, exchanged once)
+// run on the FP32 pipes from registers; the hidden layers are matrix products on the
+// tensor cores (burgers_cnn_tc.cuh), with three-piece operands whose rounding is below
+// that of an FP32 multiply-add chain (tc.cuh).  A thread turns its cell's 32
+// activations into pieces with one power-of-two scale per row (the row's max |a|, one
+// warp reduction and one barrier), a thread per 128 cells issues the products, and each
+// thread reads its cell's 32 sums back from tensor memory.
+//
+// What bounds a step: the FP32 and integer work around the products (96 GELUs, the
+// splits and the first and last layers, about 2,900 instructions per cell) with the
+// products themselves (2 x 1,490 cycles per 128 cells) beside it; two CTAs per SM
+// overlap the two.
+#include "burgers_cnn_tc.cuh"
 
 namespace inc {
 namespace burgers {
 namespace cnn {
 
 template <int N>
-__global__ void __launch_bounds__(512) k_cnn_rollout(Args a, const float* __restrict__ wts,
-                                                     float* __restrict__ corr, float* __restrict__ acts) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    Smem<N>& S = *reinterpret_cast<Smem<N>*>(smraw);
-    constexpr int R = rows_per_cta<N>();
-    constexpr int LPG = N / 8;  // lanes per channel group
-    const int rl = threadIdx.x / N;
-    const int g = threadIdx.x % N;
-    const int cg = g / LPG;
-    const int L = g % LPG;
+struct FwdSmem {
+    using Cfg = TcCfg<N>;
+    alignas(128) unsigned char w[2][W_LAYER];          // W2, W3 in pieces
+    union {
+        alignas(128) unsigned char act[3 * 4 * Cfg::PLANE];  // activations in pieces
+        struct {                                             // outside the hidden layers
+            float part[Cfg::R][KW][N];  // the last layer's sums
+            WideSmem<1, N> sh[Cfg::R];  // the solver's rows
+        } o;
+    };
+    float w1[KW][C], b[3][C], w4[KW][C];               // tap-major: channels contiguous
+    float u[Cfg::R][N + 4];
+    float red[2][Cfg::T / 32];
+    uint64_t bar[Cfg::TILES];
+    uint32_t tmem;
+};
+
+template <int N>
+__global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
+    k_cnn_rollout(Args a, const float* __restrict__ wts, float* __restrict__ corr, float* __restrict__ acts) {
+    using Cfg = TcCfg<N>;
+    constexpr int T = Cfg::T, R = Cfg::R;
+    extern __shared__ __align__(128) unsigned char smraw[];
+    FwdSmem<N>& S = *reinterpret_cast<FwdSmem<N>*>(smraw);
+    float(*part)[KW][N] = S.o.part;
+    const int t = threadIdx.x, rl = t / N, g = t % N;
+    const int tile = N < 128 ? rl : t / 128;
+    const bool leader = N < 128 ? g == 0 : t % 128 == 0;
     const int row = blockIdx.x * R + rl;
     const bool valid = row < a.rows;
-    for (int i = threadIdx.x; i < W_FLOATS; i += blockDim.x) S.w[i] = __ldg(wts + i);
+    if (t < 32) tc::tmem_alloc(&S.tmem, Cfg::COLS);
+    if (t == 0) {
+#pragma unroll
+        for (int i = 0; i < Cfg::TILES; ++i) tc::mbar_init(&S.bar[i], 1);
+        tc::mbar_init_fence();
+    }
+    for (int i = t; i < KW * C; i += T) {
+        S.w1[i / C][i % C] = __ldg(wts + OFF_W1 + (i % C) * KW + i / C);
+        S.w4[i / C][i % C] = __ldg(wts + OFF_W4 + (i % C) * KW + i / C);
+    }
+    if (t < C) {
+        S.b[0][t] = __ldg(wts + OFF_B1 + t);
+        S.b[1][t] = __ldg(wts + OFF_B2 + t);
+        S.b[2][t] = __ldg(wts + OFF_B3 + t);
+    }
+    float ws[2];
+    ws[0] = stage_weights<T, false>(S.w[0], wts + OFF_W2, S.red[0]);
+    ws[1] = stage_weights<T, false>(S.w[1], wts + OFF_W3, S.red[0]);
+    const float b4 = __ldg(wts + OFF_B4);
+    tc::fence_smem();
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    // this warp's lanes of its tile's accumulators
+    const uint32_t acc = S.tmem + 96 * tile + ((uint32_t)(t & 96) << 16);
     Ctx<1> cx;
     make_ctx<1, N>(a, valid ? row : 0, g, true, cx);
     cx.has_s = true;
     float u[1], cmp[1] = {0.f};  // cmp: compensation carried from step to step (see advance)
     u[0] = valid ? __ldg(a.u + (int64_t)row * N + g) : 0.f;
     int parity = 0;
-    float (*act0)[row_len<N>()] = S.act[0][rl];
-    float (*act1)[row_len<N>()] = S.act[1][rl];
+    uint32_t phase = 0;
+    bool fail = false;  // a wait for the tensor cores ran out: the outputs turn to NaN
     const int nseg = a.ckpt_every > 0 ? (a.steps + a.ckpt_every - 1) / a.ckpt_every : 0;
     for (int k = 0; k < a.steps; ++k) {
         if (a.ckpts && valid && k % a.ckpt_every == 0)
             a.ckpts[((int64_t)row * nseg + k / a.ckpt_every) * N + g] = u[0];
-        put_cell<N>(act0[0], g, u[0]);
-        __syncthreads();  // also: the weights are in place (first step)
-        conv_first<N>(S.w, act0[0], act1, cg, L);
+        S.u[rl][g + 2] = u[0];
+        if (g < 2) S.u[rl][N + 2 + g] = u[0];
+        if (g >= N - 2) S.u[rl][g - N + 2] = u[0];
         __syncthreads();
-        if (acts) {  // training: the hidden layers' pre-activations recorded for the backward
-            float acc[4][8];
-            conv_mid_acc<N>(S.w + OFF_W2, S.w + OFF_B2, act1, acc, cg, L);
-            if (valid) put_acts(acts, row, a.steps, k, 0, acc, cg, L, N);
-            store_tile<N, true>(act0, acc, cg, L);
+        float v[C];
+        {  // layer 1
+            float2 uu[KW];
+#pragma unroll
+            for (int q = 0; q < KW; ++q) uu[q] = f2s(S.u[rl][g + q]);
+#pragma unroll
+            for (int c = 0; c < C; c += 4) {
+                const float4 b = lds4(&S.b[0][c]);
+                float2 z0 = f2(b.x, b.y), z1 = f2(b.z, b.w);
+#pragma unroll
+                for (int q = 0; q < KW; ++q) {
+                    const float4 w = lds4(&S.w1[q][c]);
+                    z0 = __ffma2_rn(f2(w.x, w.y), uu[q], z0);
+                    z1 = __ffma2_rn(f2(w.z, w.w), uu[q], z1);
+                }
+                z0 = act::gelu2(z0);
+                z1 = act::gelu2(z1);
+                v[c] = z0.x; v[c + 1] = z0.y; v[c + 2] = z1.x; v[c + 3] = z1.y;
+            }
+        }
+#pragma unroll 1
+        for (int l = 0; l < 2; ++l) {  // layers 2 and 3
+            const float m = row_absmax<N>(v, S.red[l], fail, rl);
+            if (fail) break;
+            const float s = tc::pow2_above(m);
+            store_cell<N>(S.act, v, 256.f / s, rl, g);
+            tc::fence_smem();
+            tc::fence_before();
             __syncthreads();
-            conv_mid_acc<N>(S.w + OFF_W3, S.w + OFF_B3, act0, acc, cg, L);
-            if (valid) put_acts(acts, row, a.steps, k, 1, acc, cg, L, N);
-            store_tile<N, true>(act1, acc, cg, L);
-        } else {
-            conv_mid<N>(S.w + OFF_W2, S.w + OFF_B2, act1, act0, cg, L);
-            __syncthreads();
-            conv_mid<N>(S.w + OFF_W3, S.w + OFF_B3, act0, act1, cg, L);
+            if (leader) {
+                tc::fence_after();
+                issue_layer<N>(S.tmem + 96 * tile, S.act, S.w[l], tile);
+                tc::commit(&S.bar[tile]);
+            }
+            fail = !tc::mbar_wait(&S.bar[tile], phase);
+            phase ^= 1;
+            tc::fence_after();
+            const float f = s * (1.f / 256.f) * ws[l];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float z[16];
+                read_layer16(acc, 16 * h, f, z);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) z[i] += S.b[l + 1][16 * h + i];
+                if (acts && valid) {
+                    float* p = acts_tile(acts, row, a.steps, k, l, 16 * h, N) + g;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) p[(int64_t)i * N] = z[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const float2 y = act::gelu2(f2(z[i], z[i + 1]));
+                    v[16 * h + i] = y.x;
+                    v[16 * h + i + 1] = y.y;
+                }
+            }
+            tc::fence_before();  // the accumulators are read before the next layer overwrites them
+        }
+        if (__syncthreads_or(fail)) {  // (also: every tile's products have read the activations)
+            fail = true;
+            break;
+        }
+        {  // layer 4: this cell's share of its five neighbours' sums
+            float2 q[KW];
+#pragma unroll
+            for (int i = 0; i < KW; ++i) q[i] = f2s(0.f);
+#pragma unroll
+            for (int c = 0; c < C; c += 4) {
+#pragma unroll
+                for (int i = 0; i < KW; ++i) {
+                    const float4 w = lds4(&S.w4[i][c]);
+                    q[i] = __ffma2_rn(f2(w.x, w.y), f2(v[c], v[c + 1]), q[i]);
+                    q[i] = __ffma2_rn(f2(w.z, w.w), f2(v[c + 2], v[c + 3]), q[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < KW; ++i) part[rl][i][g] = q[i].x + q[i].y;
         }
         __syncthreads();
-        conv_last_partial<N>(S.w + OFF_W4, act1, act0, cg, L);
-        __syncthreads();
-        float s = S.w[OFF_B4];
+        float s = b4;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) s += act0[q][apad(g + 2)];
+        for (int i = 0; i < KW; ++i) s += part[rl][i][(g + i - 2 + N) & (N - 1)];
         cx.s[0] = s;
         const int64_t at = ((int64_t)row * a.steps + k) * N + g;
         if (corr && valid) corr[at] = s;
-        // the stage's first barrier also orders these reads of act0 before the next step's writes
-        advance_wide<1, N>(a, cx, u, cmp, cx.t + k * cx.dt, S.sh[rl], parity, g);
+        // the stage's first barrier also orders these reads of the sums before the next step's writes
+        advance_wide<1, N>(a, cx, u, cmp, cx.t + k * cx.dt, S.o.sh[rl], parity, g);
         if (a.frames && valid) a.frames[at] = u[0];
     }
+    if (fail && valid) {
+        const float nan = __int_as_float(0x7fffffff);
+        u[0] = nan;
+        for (int k = 0; k < a.steps; ++k) {
+            const int64_t at = ((int64_t)row * a.steps + k) * N + g;
+            if (corr) corr[at] = nan;
+            if (a.frames) a.frames[at] = nan;
+        }
+    }
     if (a.out && valid) a.out[(int64_t)row * N + g] = u[0];
+    tc::fence_before();
+    __syncthreads();
+    if (t < 32) tc::tmem_free(S.tmem, Cfg::COLS);
 }
 
 template <int N>
 int launch(const Args& a, const float* w, float* corr, float* acts, cudaStream_t st) {
-    constexpr int R = rows_per_cta<N>();
-    const size_t smem = sizeof(Smem<N>);
-    static_assert(sizeof(Smem<N>) <= 227 * 1024, "shared memory");
+    constexpr int R = TcCfg<N>::R;
+    const size_t smem = sizeof(FwdSmem<N>);
+    static_assert(sizeof(FwdSmem<N>) <= (N == 512 ? 227 : 113) * 1024, "shared memory");
     cudaFuncSetAttribute(k_cnn_rollout<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_cnn_rollout<N><<<(a.rows + R - 1) / R, R * N, smem, st>>>(a, w, corr, acts);
+    k_cnn_rollout<N><<<(a.rows + R - 1) / R, TcCfg<N>::T, smem, st>>>(a, w, corr, acts);
     return check_launch("burgers_cnn_rollout");
 }
 

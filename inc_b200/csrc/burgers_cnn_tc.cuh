@@ -1,0 +1,149 @@
+// The periodic CNN corrector's hidden layers on the tensor cores: shared by the
+// forward rollout and its backward.
+//
+// A circular convolution of 32 channels to 32 channels, kernel 5, is five matrix
+// products [cells x 32] x [32 x 32], one per tap, on the same activation tile
+// shifted by one cell.  Activations sit in shared memory in the core-matrix layout of
+// tc.cuh, one slot (16 bytes per 8 channels and piece) per cell, with the two halo
+// cells of each side stored, so a tap is a start address 16 bytes further.  The
+// weights' three pieces are stacked as 96 columns: the activations' hi piece takes
+// all 96 in one instruction, mid 64 (hi, mid) and lo 32 (hi), so the accumulator
+// columns are hi.hi | first-order | second-order sums (see tc.cuh).  One instruction of
+// N = 96 issues in 56 cycles, N = 64 in 48, N = 32 in 45 (measured, M = 128, K = 16):
+// 1,490 cycles for a layer of 128 cells against 6,550 on the FP32 pipes at their peak.
+#pragma once
+#include "burgers_cnn.cuh"
+#include "gelu.cuh"
+#include "tc.cuh"
+
+namespace inc {
+namespace burgers {
+namespace cnn {
+
+// One thread per cell, 128 or more threads: rows of at most 128 cells have a tile of
+// 128 accumulator lanes each (a row of 64 cells leaves half of its tile unused; the
+// second row of the CTA uses the upper half so that its threads' warps can read it).
+template <int N>
+struct TcCfg {
+    static constexpr int T = N < 128 ? 128 : N;
+    static constexpr int R = T / N;                  // rows per CTA
+    static constexpr int SLOTS = R * (N + 4);        // cells with halos
+    static constexpr int PLANE = SLOTS * 16;         // bytes of 8 channels of one piece
+    static constexpr int TILES = N < 128 ? R : N / 128;
+    static constexpr int COLS = TILES <= 1 ? 128 : TILES <= 2 ? 256 : 512;  // 96 used per tile
+    static constexpr int WARPS_PER_ROW = N / 32;
+};
+constexpr int W_TAP = 96 * 32 * 2;             // bytes of one tap's stacked weight pieces
+constexpr int W_LAYER = KW * W_TAP;            // bytes of one layer's
+constexpr int W_PLANE = 96 * 16;
+
+// Packed FP32 weights of a hidden layer ([ci][co][k]) -> stacked pieces, tap-major:
+// tap k holds rows (piece, co), contraction ci.  TRANS: the layer's adjoint, rows
+// (piece, ci), contraction co, taps reversed.  Returns 2^e / 256 with 2^e >= max|w|.
+template <int T, bool TRANS>
+INC_DEV float stage_weights(unsigned char* dst, const float* __restrict__ w, float* red) {
+    float m = 0.f;
+    for (int i = threadIdx.x; i < C * C * KW; i += T) m = fmaxf(m, fabsf(__ldg(w + i)));
+    m = group_max_nonneg<32>(m);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < T / 32; ++i) m = fmaxf(m, red[i]);
+    __syncthreads();  // red is free again
+    const float s = tc::pow2_above(m), inv = 256.f / s;
+    // item: tap k, row r (the product's output channel), 8 contraction channels c8
+    for (int i = threadIdx.x; i < KW * C * (C / 8); i += T) {
+        const int k = i / (C * (C / 8)), r = i % C, c8 = (i / C) % (C / 8);
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = 8 * c8 + j;
+            const int ci = TRANS ? r : c, co = TRANS ? c : r, tap = TRANS ? KW - 1 - k : k;
+            v[j] = __ldg(w + (ci * C + co) * KW + tap) * inv;
+        }
+        uint4 hi, mid, lo;
+        tc::split8(v, hi, mid, lo);
+        unsigned char* p = dst + k * W_TAP + c8 * W_PLANE + r * 16;
+        *reinterpret_cast<uint4*>(p) = hi;
+        *reinterpret_cast<uint4*>(p + 32 * 16) = mid;
+        *reinterpret_cast<uint4*>(p + 64 * 16) = lo;
+    }
+    return s * (1.f / 256.f);
+}
+
+// This thread's 32 channels at cell g of row rl, scaled by inv, into the slot and the
+// halo copies that the row's ends own.  act: [3 pieces][4 planes][SLOTS][16 bytes].
+template <int N>
+INC_DEV void store_cell(unsigned char* act, const float (&v)[C], float inv, int rl, int g) {
+    constexpr int PL = TcCfg<N>::PLANE;
+    const int slot = rl * (N + 4) + g + 2;
+    const int halo = g < 2 ? N : (g >= N - 2 ? -N : 0);
+#pragma unroll
+    for (int c8 = 0; c8 < 4; ++c8) {
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = v[8 * c8 + j] * inv;
+        uint4 q[3];
+        tc::split8(x, q[0], q[1], q[2]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            unsigned char* d = act + (p * 4 + c8) * PL + slot * 16;
+            *reinterpret_cast<uint4*>(d) = q[p];
+            if (halo != 0) *reinterpret_cast<uint4*>(d + halo * 16) = q[p];
+        }
+    }
+}
+
+// One layer's products for one tile: 5 taps x 2 channel halves, accumulators at
+// columns d .. d + 95 of the tile's 128 lanes; one thread issues.
+template <int N>
+INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned char* w, int tile) {
+    constexpr int PL = TcCfg<N>::PLANE;
+    // (rows of 64 cells: the second row's tile starts 64 slots early, see TcCfg)
+    const int slot0 = N < 128 ? tile * (N + 4) - tile * 64 : tile * 128;
+    const uint32_t a0 = tc::smem_u32(act) + slot0 * 16, b0 = tc::smem_u32(w);
+    constexpr uint32_t i96 = tc::instr_desc(128, 96), i64 = tc::instr_desc(128, 64), i32 = tc::instr_desc(128, 32);
+#pragma unroll 1
+    for (int k = 0; k < KW; ++k) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint64_t b = tc::smem_desc(b0 + k * W_TAP + 2 * h * W_PLANE, W_PLANE, 128);
+            const uint32_t a = a0 + k * 16 + 2 * h * PL;
+            tc::mma(d, tc::smem_desc(a, PL, 128), b, i96, k + h > 0);
+            tc::mma(d + 32, tc::smem_desc(a + 4 * PL, PL, 128), b, i64, true);
+            tc::mma(d + 64, tc::smem_desc(a + 8 * PL, PL, 128), b, i32, true);
+        }
+    }
+}
+
+// 16 channels (c0 .. c0 + 15) of this thread's cell: (hi.hi + (first + second order)) f
+INC_DEV void read_layer16(uint32_t d, int c0, float f, float (&z)[16]) {
+    float v0[16], v1[16], v2[16];
+    tc::tmem_ld16(d + c0, v0);
+    tc::tmem_ld16(d + 32 + c0, v1);
+    tc::tmem_ld16(d + 64 + c0, v2);
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) z[i] = (v0[i] + (v1[i] + v2[i])) * f;
+}
+
+// max |v| over this thread's channels and its row (a barrier of the CTA inside; fails
+// is or-ed over the CTA)
+template <int N>
+INC_DEV float row_absmax(const float (&v)[C], float* red, bool& fail, int rl) {
+    float m = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) m = fmaxf(m, fabsf(v[c]));
+    m = group_max_nonneg<32>(m);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    fail = __syncthreads_or(fail);
+    constexpr int WPR = TcCfg<N>::WARPS_PER_ROW;
+    m = 0.f;
+#pragma unroll
+    for (int i = 0; i < WPR; ++i) m = fmaxf(m, red[rl * WPR + i]);
+    return m;
+}
+
+}  // namespace cnn
+}  // namespace burgers
+}  // namespace inc

@@ -1,0 +1,151 @@
+// Fifth-generation tensor-core (tcgen05) helpers for FP32-accurate contractions.
+//
+// An FP32 operand is split into three bf16 pieces in fixed point: with a power of
+// two s >= max|x| of the operand's scale group (the elements that share one scale
+// along the contraction), x / s * 256 = hi + mid + lo, where hi is an integer of
+// magnitude <= 256, mid a multiple of 2^-9 of magnitude <= 1/2 and lo a multiple
+// of 2^-18 of magnitude <= 2^-10: all exact in bf16, the remainder at most 2^-19
+// (2^-27 of s).  Six of the nine piece products are accumulated (the dropped ones
+// are below 2^-27 of s_a s_b per term) in two FP32 accumulators: hi.hi alone, whose
+// partial sums are integers below 2^24 for up to 256 full-scale terms, so the
+// accumulator's truncation never acts on it; and the five others, 2^-9 smaller, on
+// which it acts at 2^-33.  The two are added once in FP32.  The result is a rounded
+// exact sum of products of 27-bit inputs; an FP32 fused multiply-add chain of the
+// same length rounds at every term.
+//
+// Operand tiles live in shared memory as [rows][K] bf16 in 8-row x 16-byte core
+// matrices without swizzle: element (r, k) at (k / 8) * plane + r * 16 + (k % 8) * 2
+// bytes, plane = rows * 16.  A row is 16 bytes from the next, so a tile shifted by
+// one row (a convolution tap) is the same tile with the start address moved by 16.
+#pragma once
+#include <cuda_bf16.h>
+
+#include "common.cuh"
+
+namespace inc {
+namespace tc {
+
+INC_DEV uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// generic-proxy writes to shared memory visible to the tensor core's reads
+INC_DEV void fence_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+INC_DEV void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+INC_DEV void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// ---- tensor memory -------------------------------------------------------------
+// One warp allocates ncols (a power of two >= 32) columns; the base goes to *dst (shared).
+INC_DEV void tmem_alloc(uint32_t* dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+INC_DEV void tmem_free(uint32_t base, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(ncols) : "memory");
+}
+// 16 consecutive columns of this warp's 32 lanes (lane = accumulator row)
+INC_DEV void tmem_ld16(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+INC_DEV void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---- mbarrier --------------------------------------------------------------------
+INC_DEV void mbar_init(uint64_t* b, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+INC_DEV void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+// Waits for the phase of this parity; false when it did not complete within the limit
+// (try_wait suspends for a while by itself, so the limit is seconds).
+INC_DEV bool mbar_wait(uint64_t* b, uint32_t parity) {
+    const uint32_t a = smem_u32(b);
+    for (int i = 0; i < (1 << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// ---- matrix instructions -----------------------------------------------------------
+// Shared-memory descriptor of a tile in core matrices without swizzle: `lead` and
+// `stride` are the byte distances of neighbouring core matrices along K and along the
+// rows (K-major), or along the rows' 8-groups of K and along the columns (MN-major).
+INC_DEV uint64_t smem_desc(uint32_t addr, uint32_t lead, uint32_t stride) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lead >> 4) & 0x3FFFu) << 16) |
+           ((uint64_t)((stride >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+// FP32 accumulator, bf16 operands, M x N tile; a_mn / b_mn: operand stored MN-major
+__host__ __device__ constexpr uint32_t instr_desc(int M, int N, bool a_mn = false, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// D[tmem] (+)= A B^T over K = 16; one thread issues
+INC_DEV void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+// arrives on `b` when every matrix instruction this thread issued has finished
+INC_DEV void commit(uint64_t* b) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
+                 : "memory");
+}
+
+// ---- the three-piece split -----------------------------------------------------------
+// A power of two >= m (m >= 0, finite) as a float bit pattern's exponent: scale() gives
+// s / 256 and inv() 256 / s for the group.  m = 0 and the smallest values use 2^-100
+// (the pieces are then zero or exact below the smallest magnitudes that matter to a
+// product); the largest finite m keeps s finite.
+INC_DEV float pow2_above(float m) {
+    const uint32_t e = (__float_as_uint(m) + 0x007FFFFFu) & 0x7F800000u;
+    return fminf(fmaxf(__uint_as_float(e), 7.888609052210118e-31f), 1.7014118346046923e38f);
+}
+
+// x (already scaled to |x| <= 256) -> hi, mid, lo (exact in bf16)
+INC_DEV void split3(float x, float& hi, float& mid, float& lo) {
+    const float M0 = 12582912.f;              // 1.5 * 2^23: rounds to integers
+    const float M1 = 12582912.f / 512.f;      // to multiples of 2^-9
+    const float M2 = 12582912.f / 262144.f;   // to multiples of 2^-18
+    hi = __fsub_rn(__fadd_rn(x, M0), M0);
+    const float r = __fsub_rn(x, hi);
+    mid = __fsub_rn(__fadd_rn(r, M1), M1);
+    const float q = __fsub_rn(r, mid);
+    lo = __fsub_rn(__fadd_rn(q, M2), M2);
+}
+// the upper halves of two floats (exact bf16 values) packed as (a, b)
+INC_DEV uint32_t pack_bf16(float a, float b) {
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+// eight scaled values -> 16 bytes of each piece
+INC_DEV void split8(const float (&x)[8], uint4& hi, uint4& mid, uint4& lo) {
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float h0, m0, l0, h1, m1, l1;
+        split3(x[2 * i], h0, m0, l0);
+        split3(x[2 * i + 1], h1, m1, l1);
+        h[i] = pack_bf16(h0, h1);
+        m[i] = pack_bf16(m0, m1);
+        l[i] = pack_bf16(l0, l1);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    mid = make_uint4(m[0], m[1], m[2], m[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+}  // namespace tc
+}  // namespace inc

@@ -350,3 +350,26 @@ def test_fused_training_gradients_are_deterministic(cuda, N, B):
     a, b = run(), run()
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("N", [64, 128, 256, 512])
+def test_fused_cnn_rows_of_different_magnitude(cuda, N):
+    """The hidden layers' operands share one scale per row: rows of zeros, of tiny and of large
+    states and a row that turns non-finite, side by side (two rows share a CTA at n = 64), each
+    as accurate as on its own and none disturbed by the non-finite one."""
+    from inc_b200.fused import burgers_cnn_rollout
+    from inc_b200.solvers import BurgersSolverTorch
+    p = _params(N)
+    u0 = _u0(6, N, seed=N) * np.array([0.0, 1e-6, 1.0, 1.0, 2.0, 0.1])[:, None]
+    net = _net(8)
+    ref_f, ref_c = _fp64_loop(net, p, u0, 4, "ssprk3")
+    u0[2, N // 3] = np.inf
+    solver = BurgersSolverTorch(_sim_params(p, 6, "ssprk3", cuda))
+    with torch.no_grad():
+        frames, corr = burgers_cnn_rollout(net.float().to(cuda), solver,
+                                           torch.tensor(u0, dtype=torch.float32, device=cuda), 4)
+    frames, corr = frames.cpu().numpy(), corr.cpu().numpy()
+    assert not np.isfinite(frames[2, -1]).any()
+    for r in (0, 1, 3, 4, 5):
+        assert rel_l2(corr[r], ref_c[r]) < TOL, r
+        assert rel_l2(frames[r], ref_f[r]) < TOL, r
