@@ -139,20 +139,21 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
             const float f = s * (1.f / 256.f) * ws[l];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                float z[16];
-                read_layer16(acc, 16 * h, f, z);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) z[i] += S.b[l + 1][16 * h + i];
+                float2 z[8];
+                read_layer16(acc, 16 * h, f, S.b[l + 1], z);
                 if (acts && valid) {
                     float* p = acts_tile(acts, row, a.steps, k, l, 16 * h, N) + g;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) p[(int64_t)i * N] = z[i];
+                    for (int i = 0; i < 8; ++i) {
+                        p[(int64_t)(2 * i) * N] = z[i].x;
+                        p[(int64_t)(2 * i + 1) * N] = z[i].y;
+                    }
                 }
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    const float2 y = act::gelu2(f2(z[i], z[i + 1]));
-                    v[16 * h + i] = y.x;
-                    v[16 * h + i + 1] = y.y;
+                for (int i = 0; i < 8; ++i) {
+                    const float2 y = act::gelu2(z[i]);
+                    v[16 * h + 2 * i] = y.x;
+                    v[16 * h + 2 * i + 1] = y.y;
                 }
             }
             tc::fence_before();  // the accumulators are read before the next layer overwrites them

@@ -59,10 +59,10 @@ INC_DEV float stage_weights(unsigned char* dst, const float* __restrict__ w, flo
         for (int j = 0; j < 8; ++j) {
             const int c = 8 * c8 + j;
             const int ci = TRANS ? r : c, co = TRANS ? c : r, tap = TRANS ? KW - 1 - k : k;
-            v[j] = __ldg(w + (ci * C + co) * KW + tap) * inv;
+            v[j] = __ldg(w + (ci * C + co) * KW + tap);
         }
         uint4 hi, mid, lo;
-        tc::split8(v, hi, mid, lo);
+        tc::split8(v, inv, hi, mid, lo);
         unsigned char* p = dst + k * W_TAP + c8 * W_PLANE + r * 16;
         *reinterpret_cast<uint4*>(p) = hi;
         *reinterpret_cast<uint4*>(p + 32 * 16) = mid;
@@ -82,9 +82,9 @@ INC_DEV void store_cell(unsigned char* act, const float (&v)[C], float inv, int 
     for (int c8 = 0; c8 < 4; ++c8) {
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = v[8 * c8 + j] * inv;
+        for (int j = 0; j < 8; ++j) x[j] = v[8 * c8 + j];
         uint4 q[3];
-        tc::split8(x, q[0], q[1], q[2]);
+        tc::split8(x, inv, q[0], q[1], q[2]);
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             unsigned char* d = act + (p * 4 + c8) * PL + slot * 16;
@@ -116,15 +116,23 @@ INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned ch
     }
 }
 
-// 16 channels (c0 .. c0 + 15) of this thread's cell: (hi.hi + (first + second order)) f
-INC_DEV void read_layer16(uint32_t d, int c0, float f, float (&z)[16]) {
+// 16 channels (c0 .. c0 + 15) of this thread's cell: bias + (hi.hi + (first + second order)) f
+INC_DEV void read_layer16(uint32_t d, int c0, float f, const float* bias, float2 (&z)[8]) {
     float v0[16], v1[16], v2[16];
     tc::tmem_ld16(d + c0, v0);
     tc::tmem_ld16(d + 32 + c0, v1);
     tc::tmem_ld16(d + 64 + c0, v2);
     tc::tmem_ld_wait();
 #pragma unroll
-    for (int i = 0; i < 16; ++i) z[i] = (v0[i] + (v1[i] + v2[i])) * f;
+    for (int i = 0; i < 8; i += 2) {
+        const float4 b = lds4(bias + c0 + 2 * i);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int e = 2 * (i + j);
+            const float2 s = __fadd2_rn(f2(v0[e], v0[e + 1]), __fadd2_rn(f2(v1[e], v1[e + 1]), f2(v2[e], v2[e + 1])));
+            z[i + j] = __ffma2_rn(s, f2s(f), j == 0 ? f2(b.x, b.y) : f2(b.z, b.w));
+        }
+    }
 }
 
 // max |v| over this thread's channels and its row (a barrier of the CTA inside; fails

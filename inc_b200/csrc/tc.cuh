@@ -106,42 +106,37 @@ INC_DEV void commit(uint64_t* b) {
 }
 
 // ---- the three-piece split -----------------------------------------------------------
-// A power of two >= m (m >= 0, finite) as a float bit pattern's exponent: scale() gives
-// s / 256 and inv() 256 / s for the group.  m = 0 and the smallest values use 2^-100
-// (the pieces are then zero or exact below the smallest magnitudes that matter to a
-// product); the largest finite m keeps s finite.
+// A power of two >= m (m >= 0): the scale s of a group with max|x| = m.  Groups below
+// 2^-100 use that (a product of two such groups is below FP32's smallest normal number);
+// above 2^127, and for a non-finite m, 2^127, so that 256 / s stays a normal number.
 INC_DEV float pow2_above(float m) {
     const uint32_t e = (__float_as_uint(m) + 0x007FFFFFu) & 0x7F800000u;
     return fminf(fmaxf(__uint_as_float(e), 7.888609052210118e-31f), 1.7014118346046923e38f);
 }
 
-// x (already scaled to |x| <= 256) -> hi, mid, lo (exact in bf16)
-INC_DEV void split3(float x, float& hi, float& mid, float& lo) {
-    const float M0 = 12582912.f;              // 1.5 * 2^23: rounds to integers
-    const float M1 = 12582912.f / 512.f;      // to multiples of 2^-9
-    const float M2 = 12582912.f / 262144.f;   // to multiples of 2^-18
-    hi = __fsub_rn(__fadd_rn(x, M0), M0);
-    const float r = __fsub_rn(x, hi);
-    mid = __fsub_rn(__fadd_rn(r, M1), M1);
-    const float q = __fsub_rn(r, mid);
-    lo = __fsub_rn(__fadd_rn(q, M2), M2);
+// two values packed as bf16, rounded to nearest (a in the low half)
+INC_DEV uint32_t cvt_bf16x2(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
 }
-// the upper halves of two floats (exact bf16 values) packed as (a, b)
-INC_DEV uint32_t pack_bf16(float a, float b) {
-    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+// x * inv (a power of two, |x * inv| <= 256) of two values -> their pieces, packed.
+// The products inside the fused operations are exact.
+INC_DEV void split2(float2 x, float2 inv, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const float2 M = make_float2(12582912.f, 12582912.f);  // 1.5 * 2^23: rounds to integers
+    const float2 h = __fadd2_rn(__ffma2_rn(x, inv, M), make_float2(-M.x, -M.y));
+    const float2 r = __ffma2_rn(x, inv, make_float2(-h.x, -h.y));
+    hi = __byte_perm(__float_as_uint(h.x), __float_as_uint(h.y), 0x7632);  // integers <= 256: exact
+    mid = cvt_bf16x2(r.x, r.y);
+    const float2 q = __fadd2_rn(r, make_float2(-__uint_as_float(mid << 16), -__uint_as_float(mid & 0xffff0000u)));
+    lo = cvt_bf16x2(q.x, q.y);
 }
-// eight scaled values -> 16 bytes of each piece
-INC_DEV void split8(const float (&x)[8], uint4& hi, uint4& mid, uint4& lo) {
+// eight values -> 16 bytes of each piece
+INC_DEV void split8(const float (&x)[8], float inv, uint4& hi, uint4& mid, uint4& lo) {
     uint32_t h[4], m[4], l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float h0, m0, l0, h1, m1, l1;
-        split3(x[2 * i], h0, m0, l0);
-        split3(x[2 * i + 1], h1, m1, l1);
-        h[i] = pack_bf16(h0, h1);
-        m[i] = pack_bf16(m0, m1);
-        l[i] = pack_bf16(l0, l1);
-    }
+    for (int i = 0; i < 4; ++i)
+        split2(make_float2(x[2 * i], x[2 * i + 1]), make_float2(inv, inv), h[i], m[i], l[i]);
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     mid = make_uint4(m[0], m[1], m[2], m[3]);
     lo = make_uint4(l[0], l[1], l[2], l[3]);
