@@ -48,6 +48,17 @@ class KSPlan(C.Structure):
                 ("reserved", C.c_int32), ("dt", C.c_double), ("dev", _vp)]
 
 
+class FNODesc(C.Structure):
+    _fields_ = [("rows", C.c_int32), ("n", C.c_int32), ("width", C.c_int32), ("modes", C.c_int32),
+                ("grid_stride", C.c_int64), ("grid", _vp), ("fc0_w", _vp), ("fc0_b", _vp), ("modes_w", _vp * 4),
+                ("w", _vp * 4), ("b", _vp * 4), ("fc1_w", _vp), ("fc1_b", _vp), ("fc2_w", _vp), ("fc2_b", _vp)]
+
+
+class FNOGrads(C.Structure):
+    _fields_ = [("u", _vp), ("fc0_w", _vp), ("fc0_b", _vp), ("modes_w", _vp * 4), ("w", _vp * 4), ("b", _vp * 4),
+                ("fc1_w", _vp), ("fc1_b", _vp), ("fc2_w", _vp), ("fc2_b", _vp)]
+
+
 # name -> (restype, argtypes); the full export list of include/inc_b200.h
 SIGNATURES = {
     "inc_version": (C.c_int32, []),
@@ -92,6 +103,10 @@ SIGNATURES = {
                                           _vp]),
     "inc_bias_gelu": (C.c_int, [_vp, _vp, _vp, C.c_int32, C.c_int32, C.c_int32, _vp]),
     "inc_bias_gelu_bwd": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_int32, C.c_int32, C.c_int32, _vp]),
+    "inc_fno_work_size": (C.c_int64, [C.POINTER(FNODesc), C.c_int32]),
+    "inc_fno_forward": (C.c_int, [C.POINTER(FNODesc), _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "inc_fno_backward_work_size": (C.c_int64, [C.POINTER(FNODesc)]),
+    "inc_fno_backward": (C.c_int, [C.POINTER(FNODesc), _vp, _vp, _vp, _vp, _vp, C.POINTER(FNOGrads), _vp, _vp]),
     "inc_burgers_rollout_grad_noalloc": (C.c_int, [C.POINTER(BurgersDesc), _vp, _vp, _vp, C.c_double, C.c_int32,
                                                    C.c_int32, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "inc_burgers_cnn_rollout": (C.c_int, [C.POINTER(BurgersDesc), _vp, _vp, _vp, C.c_double, C.c_int32, _vp, _vp,

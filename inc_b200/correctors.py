@@ -21,6 +21,8 @@ take torch's FFTs.  The CNN runs inside the Burgers solver kernel when
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -245,6 +247,73 @@ def _channel_linear(lin: nn.Linear, x):
     return _channel_mm(lin.weight, x) + lin.bias[:, None]
 
 
+FNO_N = (64, 128, 256, 512)
+_FNO_LAYERS = ("conv0", "conv1", "conv2", "conv3"), ("w0", "w1", "w2", "w3")
+
+
+class FNOFn(torch.autograd.Function):
+    """The whole FNO1D forward (``inc_fno_forward``) and its backward
+    (``inc_fno_backward``): u [B, n], the grid [B, n] and the parameters in FNO1D's order."""
+
+    @staticmethod
+    def _desc(u, grid, params):
+        fc0_w, fc0_b, *rest = params
+        modes_w, ws, bs, (fc1_w, fc1_b, fc2_w, fc2_b) = rest[0:4], rest[4:12:2], rest[5:12:2], rest[12:]
+        d = nat.FNODesc()
+        d.rows, d.n = u.shape
+        d.width, d.modes = fc0_w.shape[0], modes_w[0].shape[-1]
+        d.grid_stride, d.grid = grid.stride(0), grid.data_ptr()
+        d.fc0_w, d.fc0_b = fc0_w.data_ptr(), fc0_b.data_ptr()
+        for i in range(4):
+            d.modes_w[i], d.w[i], d.b[i] = modes_w[i].data_ptr(), ws[i].data_ptr(), bs[i].data_ptr()
+        d.fc1_w, d.fc1_b, d.fc2_w, d.fc2_b = (t.data_ptr() for t in (fc1_w, fc1_b, fc2_w, fc2_b))
+        return d
+
+    @staticmethod
+    def forward(ctx, u, grid, record, *params):
+        u = u.contiguous()
+        params = [p.contiguous() for p in params]
+        d = FNOFn._desc(u, grid, params)
+        B, n, W, M = d.rows, d.n, d.width, d.modes
+        y = torch.empty_like(u)
+        z = xm = tmax = None
+        if record:  # for the backward: the layers' sums before GELU, their inputs' modes, magnitudes
+            z = u.new_empty(4, B, W, n)
+            xm = u.new_empty(4, M, B, W, 2)
+            tmax = u.new_empty(4, max(1, n // 128), B)
+        lib = nat.lib()
+        work = u.new_empty(lib.inc_fno_work_size(C.byref(d), int(record)))
+        with nat.on_device(u.device):
+            rc = lib.inc_fno_forward(C.byref(d), u.data_ptr(), y.data_ptr(), nat.ptr(z), nat.ptr(xm), nat.ptr(tmax),
+                                     work.data_ptr(), nat.stream_of(u.device))
+        nat.check(rc, "inc_fno_forward")
+        if record:
+            ctx.save_for_backward(u, grid, z, xm, tmax, *params)
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        u, grid, z, xm, tmax, *params = ctx.saved_tensors
+        gy = gy.contiguous()
+        d = FNOFn._desc(u, grid, params)
+        need = ctx.needs_input_grad
+        gu = torch.empty_like(u) if need[0] else None
+        grads = [torch.empty_like(p) for p in params]
+        g = nat.FNOGrads()
+        g.u = nat.ptr(gu)
+        g.fc0_w, g.fc0_b = grads[0].data_ptr(), grads[1].data_ptr()
+        for i in range(4):
+            g.modes_w[i], g.w[i], g.b[i] = (grads[j].data_ptr() for j in (2 + i, 6 + 2 * i, 7 + 2 * i))
+        g.fc1_w, g.fc1_b, g.fc2_w, g.fc2_b = (t.data_ptr() for t in grads[14:])
+        lib = nat.lib()
+        work = u.new_empty(lib.inc_fno_backward_work_size(C.byref(d)))
+        with nat.on_device(u.device):
+            rc = lib.inc_fno_backward(C.byref(d), u.data_ptr(), gy.data_ptr(), z.data_ptr(), xm.data_ptr(),
+                                      tmax.data_ptr(), C.byref(g), work.data_ptr(), nat.stream_of(u.device))
+        nat.check(rc, "inc_fno_backward")
+        return (gu, None, None) + tuple(t if need[3 + i] else None for i, t in enumerate(grads))
+
+
 class FNO1D(nn.Module):
     """The reference's FNO corrector (models/models_1d/fno.py:39-105), same constructor
     ``FNO1D(L=16, modes=16, width=64)``, same submodules and parameter names (fc0,
@@ -276,9 +345,48 @@ class FNO1D(nn.Module):
         self.fc1 = nn.Linear(self.width, 128)
         self.fc2 = nn.Linear(128, 1)
 
+    def _layer_params(self):
+        """The parameters in FNOFn's order."""
+        convs, ws = _FNO_LAYERS
+        out = [self.fc0.weight, self.fc0.bias] + [getattr(self, c).weights1 for c in convs]
+        for w in ws:
+            out += [getattr(self, w).weight, getattr(self, w).bias]
+        return out + [self.fc1.weight, self.fc1.bias, self.fc2.weight, self.fc2.bias]
+
+    def _fused(self, x, L) -> bool:
+        """True when FNOFn computes this call: FP32 CUDA states of 64..512 cells, width 32 or
+        64 and at most 16 modes, the plain layers (nothing hooked, replaced or reshaped), no
+        autocast, no gradient to L."""
+        if not (isinstance(x, torch.Tensor) and x.is_cuda and x.dtype == torch.float32 and x.dim() == 2
+                and x.shape[0] > 0 and x.shape[1] in FNO_N and self.width in (32, 64) and 1 <= self.modes1 <= 16):
+            return False
+        if torch.is_autocast_enabled("cuda") or (isinstance(L, torch.Tensor) and (L.requires_grad or not L.is_cuda)):
+            return False
+        W, M = self.width, self.modes1
+        convs, ws = _FNO_LAYERS
+        for name in convs:
+            m = getattr(self, name)
+            if type(m) is not SpectralConv1d or m.modes1 != M or "forward" in m.__dict__:
+                return False
+            if (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                    or torch.nn.modules.module._has_any_global_hook()):
+                return False
+        shapes = [(W, 2), (W,)] + [(W, W, M)] * 4 + [(W, W, 1), (W,)] * 4 + [(128, W), (128,), (1, 128), (1,)]
+        for i, (p, shape) in enumerate(zip(self._layer_params(), shapes)):
+            if (not isinstance(p, torch.Tensor) or tuple(p.shape) != shape or p.device != x.device
+                    or p.dtype != (torch.complex64 if 2 <= i < 6 else torch.float32)):
+                return False
+        return True
+
     def forward(self, x, L=None):
         L = L if L is not None else self.L
         grid = get_grid(x, L)
+        if self._fused(x, L):
+            params = self._layer_params()
+            record = torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in params))
+            if grid.stride(1) != 1:
+                grid = grid.contiguous()
+            return FNOFn.apply(x, grid, record, *params)
         h = _channel_linear(self.fc0, torch.stack([x, grid], dim=1))  # [B, width, D]
         layers = ((self.conv0, self.w0), (self.conv1, self.w1), (self.conv2, self.w2), (self.conv3, self.w3))
         for i, (conv, w) in enumerate(layers):

@@ -1,0 +1,761 @@
+// Backward of the FNO corrector (fno_fwd.cu): the gradients of u and of every parameter from
+// dL/dy, the layers' sums before GELU (z), the modes of the layers' inputs and the tiles'
+// magnitudes that the forward recorded.
+//
+//   projection   k_fno_proj_bwd: the 128 hidden values again (one product), their
+//                gradient g1 = dy w2 gelu'(a) (stored for fc1's weight gradient), dL/dz of
+//                the last layer (a second product with the same weights read transposed)
+//                and fc2's gradient;
+//   layer l      modes of dL/dz_l (k_fno_modes), their adjoint mixing, and k_fno_layer with the
+//                transposed weights, times gelu'(z_{l-1}): dL/dz_{l-1};
+//   weights      k_fno_wgrad: dL/dz (or g1) times the layer's input, contracted over all
+//                points on the tensor cores; the Fourier weights from the modes
+//                (k_fno_modes_grad);
+//   the lift     folded into layer 0's adjoint: the lifted state is affine in (u, grid, 1), so
+//                its weight gradient and fc0's are six sums per channel.
+#include "fno_tc.cuh"
+
+namespace inc {
+namespace fno {
+
+int check_fno(const inc_fno_desc* d);  // fno_fwd.cu
+
+// ---- projection -------------------------------------------------------------------------
+struct ProjBwdArgs {
+    const float* x;      // z of the last layer [batch][W][N]
+    const float* xmax;   // [tiles per row][batch]
+    const unsigned char* fc1;  // image
+    const float* wscale;
+    const float* fc1_b;  // [128]
+    const float* fc2_w;  // [128]
+    const float* g_y;    // [batch][N]
+    float* g1;           // [batch][128][N]
+    float* g1max;        // [tiles per row][batch]
+    float* g_x;          // [batch][W][N]
+    float* gxmax;        // [tiles per row][batch]
+    float* sums;         // [blocks][132]: fc2's gradient, then its bias's
+    int batch;
+};
+
+template <int W>
+struct ProjBwdSmem {
+    alignas(128) unsigned char w[3 * 128 * W * 2];
+    alignas(128) unsigned char x[3 * 64 * 128 * 2];
+    alignas(16) float b1[128], w2[128];
+    alignas(16) float red[2][WORKERS / 32];
+    float w2max;
+    uint64_t bar_images, bar;
+    uint32_t tmem;
+};
+
+template <int W, int N>
+__global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
+    extern __shared__ __align__(128) unsigned char fno_smem[];
+    ProjBwdSmem<W>& S = *reinterpret_cast<ProjBwdSmem<W>*>(fno_smem);
+    constexpr int points = N < 128 ? N : 128, nq = N / points, C = W / 2;
+    const int tid = threadIdx.x, half = (tid >> 7) & 1, t = tid & 127;
+    const int tiles = a.batch * nq, step = gridDim.x;
+    if (tid >= WORKERS) tc::tmem_alloc(&S.tmem, 256);
+    if (tid == WORKERS) {
+        tc::mbar_init(&S.bar_images, 1);
+        tc::mbar_init(&S.bar, 1);
+        tc::mbar_init_fence();
+        tc::mbar_expect(&S.bar_images, sizeof(S.w));
+        tc::bulk_load(S.w, a.fc1, sizeof(S.w), &S.bar_images);
+    }
+    for (int i = tid; i < 128; i += THREADS) {
+        S.b1[i] = __ldg(a.fc1_b + i);
+        S.w2[i] = __ldg(a.fc2_w + i);
+    }
+    if (tid < 32) {
+        const float4 e = __ldg(reinterpret_cast<const float4*>(a.fc2_w) + tid);
+        const float m = warp_max(fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))));
+        if (tid == 0) S.w2max = m;
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t d = S.tmem;
+    if (tid >= WORKERS) {  // the issuing warp: three products per tile
+        const bool ok = tc::mbar_wait(&S.bar_images, 0);
+        (void)ok;
+        for (int i = blockIdx.x; i < tiles; i += step) {
+            take_over();
+            if (tid == WORKERS) {  // hidden values: columns 0..127 and 128..255
+                tc::fence_after();
+                issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
+                tc::commit(&S.bar);
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {  // dL/dx += g1[64 h ..] w1, into columns 0.. and 128.., read by then
+                take_over();
+                if (tid == WORKERS) {
+                    tc::fence_after();
+                    const uint32_t x = tc::smem_u32(S.x), w = tc::smem_u32(S.w) + 64 * h * 16;
+                    constexpr uint32_t id = tc::instr_desc(128, W, false, true);
+#pragma unroll 1
+                    for (int k = 0; k < 4; ++k) {
+                        const uint64_t a0 = tc::smem_desc(x + 2 * k * 2048, 2048, 128);
+                        const uint64_t a1 = tc::smem_desc(x + (8 + 2 * k) * 2048, 2048, 128);
+                        const uint64_t a2 = tc::smem_desc(x + (16 + 2 * k) * 2048, 2048, 128);
+                        const uint64_t b0 = tc::smem_desc(w + 16 * k * 16, 128, 384 * 16);
+                        const uint64_t b1 = tc::smem_desc(w + (128 + 16 * k) * 16, 128, 384 * 16);
+                        const uint64_t b2 = tc::smem_desc(w + (256 + 16 * k) * 16, 128, 384 * 16);
+                        tc::mma(d, a0, b0, id, h + k > 0);
+                        tc::mma(d + 128, a1, b0, id, h + k > 0);
+                        tc::mma(d + 128, a0, b1, id, true);
+                        tc::mma(d + 128, a0, b2, id, true);
+                        tc::mma(d + 128, a1, b1, id, true);
+                        tc::mma(d + 128, a2, b0, id, true);
+                    }
+                    tc::commit(&S.bar);
+                }
+                __syncwarp();
+            }
+        }
+        tc::fence_before();
+        __syncthreads();
+        tc::tmem_free(S.tmem, 256);
+        return;
+    }
+    const bool on = points == 128 || t < points;
+    const float ws = __ldg(a.wscale) * (1.f / 65536.f), gbound = 1.13f * S.w2max;  // max gelu' = 1.1290
+    const uint32_t dl = d + ((uint32_t)(t & 96) << 16);
+    uint32_t phase = 0;
+    bool fail = !tc::mbar_wait(&S.bar_images, 0);
+    auto wait = [&] {
+        if (!fail) fail = !tc::mbar_wait(&S.bar, phase);
+        phase ^= 1;
+        tc::fence_after();
+    };
+    float2 v[C / 2];
+    float vmax = 0.f, g_next = 0.f, sum[2] = {0.f, 0.f}, sum_g = 0.f;
+    auto load_tile = [&](int i) {
+        if (i >= tiles) return;
+        const int b = i / nq, p = (i % nq) * points + t;
+        load_channels<C, N>(a.x + ((int64_t)b * W + half * C) * N + p, on, v);
+        vmax = __ldg(a.xmax + (int64_t)(i % nq) * a.batch + b);
+        g_next = on ? __ldg(a.g_y + (int64_t)b * N + p) : 0.f;
+    };
+    load_tile(blockIdx.x);
+    for (int i = blockIdx.x; i < tiles; i += step) {
+        const int b = i / nq, p = (i % nq) * points + t;
+        const float sx = tc::pow2_above(vmax), gy = g_next;
+        store_point<W, C>(S.x, v, 256.f / sx, half * C, t);
+        tc::fence_smem();
+        tc::fence_before();
+        hand_over();
+        load_tile(i + step);
+        const float sg = tc::pow2_above(fabsf(gy) * gbound);  // of this point's g1
+        float m1 = 0.f;
+        if (half == 0) sum_g += gy;
+        wait();
+        const float2 f = make_float2(sx * ws, sx * ws);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // hidden values 64 h + 32 half ..
+            const int j0 = 64 * h + 32 * half;
+            float2 g[16];
+            float e2[32];
+            float* out = a.g1 + ((int64_t)b * 128 + j0) * N + p;
+#pragma unroll
+            for (int c = 0; c < 32; c += 16) {
+                float x0[16], x1[16];
+                tc::tmem_ld16(dl + j0 + c, x0);
+                tc::tmem_ld16(dl + 128 + j0 + c, x1);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; e += 2) {
+                    const int j = c + e;
+                    const float2 bi = *reinterpret_cast<const float2*>(&S.b1[j0 + j]);
+                    const float2 w2 = *reinterpret_cast<const float2*>(&S.w2[j0 + j]);
+                    const float2 z = __ffma2_rn(
+                        __fadd2_rn(make_float2(x0[e], x0[e + 1]), make_float2(x1[e], x1[e + 1])), f, bi);
+                    float2 y, gp;
+                    act::gelu_both2(z, y, gp);
+                    const float2 gg = make_float2(gy, gy);
+                    y = __fmul2_rn(y, gg);
+                    e2[j] = y.x;
+                    e2[j + 1] = y.y;
+                    float2 r = __fmul2_rn(__fmul2_rn(gp, w2), gg);
+                    if (fail) r = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+                    g[j / 2] = r;
+                    m1 = fmaxf(m1, fmaxf(fabsf(r.x), fabsf(r.y)));
+                    if (on) {
+                        out[j * N] = r.x;
+                        out[(j + 1) * N] = r.y;
+                    }
+                }
+            }
+            sum[h] += warp_sums<32>(e2, t & 31);
+            if (h == 1) wait();  // the first half's products have read the tile
+            store_point<64, 32>(S.x, g, 256.f / sg, 32 * half, t);
+            tc::fence_smem();
+            tc::fence_before();
+            hand_over();
+        }
+        wait();
+        const float fs = sg * ws;
+        float m3 = 0.f;
+        float* out = a.g_x + ((int64_t)b * W + half * C) * N + p;
+#pragma unroll
+        for (int c = 0; c < C; c += 16) {
+            float x0[16], x1[16];
+            tc::tmem_ld16(dl + half * C + c, x0);
+            tc::tmem_ld16(dl + 128 + half * C + c, x1);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float r = (x0[e] + x1[e]) * fs;
+                m3 = fmaxf(m3, fabsf(r));
+                if (on) out[(c + e) * N] = fail ? __int_as_float(0x7fffffff) : r;
+            }
+        }
+        tc::fence_before();
+        m1 = warp_max(on ? m1 : 0.f);
+        m3 = warp_max(on ? m3 : 0.f);
+        if ((tid & 31) == 0) {
+            S.red[0][tid >> 5] = m1;
+            S.red[1][tid >> 5] = m3;
+        }
+        worker_sync();
+        if (tid < 2) {
+            const float4 r0 = lds4(S.red[tid]), r1 = lds4(S.red[tid] + 4);
+            (tid == 0 ? a.g1max : a.gxmax)[(int64_t)(i % nq) * a.batch + b] =
+                fmaxf(fmaxf(fmaxf(r0.x, r0.y), fmaxf(r0.z, r0.w)), fmaxf(fmaxf(r1.x, r1.y), fmaxf(r1.z, r1.w)));
+        }
+        worker_sync();
+    }
+    // the CTA's sums, its four warps of either half added in order
+    float* s = reinterpret_cast<float*>(S.x);  // [4][128], then [4]; every product is done
+    const int w = t >> 5, lane = t & 31;
+    s[w * 128 + 32 * half + lane] = sum[0];
+    s[w * 128 + 64 + 32 * half + lane] = sum[1];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum_g += __shfl_xor_sync(0xffffffffu, sum_g, o);
+    if (half == 0 && lane == 0) s[512 + w] = sum_g;
+    worker_sync();
+    float* out = a.sums + (int64_t)blockIdx.x * 132;
+    if (tid < 128) out[tid] = (s[tid] + s[128 + tid]) + (s[256 + tid] + s[384 + tid]);
+    if (tid == 128) out[128] = (s[512] + s[513]) + (s[514] + s[515]);
+    tc::fence_before();
+    __syncthreads();
+}
+
+template <int W, int N>
+int launch_proj_bwd(const ProjBwdArgs& a, int* blocks, cudaStream_t st) {
+    const size_t smem = sizeof(ProjBwdSmem<W>);
+    static_assert(sizeof(ProjBwdSmem<W>) <= 113 * 1024, "two CTAs per SM");
+    cudaFuncSetAttribute(k_fno_proj_bwd<W, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int tiles = a.batch * (N < 128 ? 1 : N / 128), most = 2 * sm_count();
+    *blocks = tiles < most ? tiles : most;
+    k_fno_proj_bwd<W, N><<<*blocks, THREADS, smem, st>>>(a);
+    return check_launch("fno projection backward");
+}
+
+// ---- weight gradients over the points ----------------------------------------------------
+// part[block][o][c] = sum over the block's units of g[b][o][p] x[b][c][p] and rows[block][o] = sum of
+// g: a unit is `seg` points of one trajectory, 64 per chunk.  The rows of g in three
+// stacked pieces are the accumulator lanes, those of x the columns:
+//   MO = 32:  lanes (hi, mid, lo) x columns (hi, mid, lo), one product;
+//   MO = 64:  lanes (hi, mid) x (hi, mid, lo), and lo x hi added to the columns of hi x lo;
+//   MO = 128: hi x (hi, mid, lo), mid x (hi, mid), lo x hi.
+// A unit's sums are read into registers (with its two scales) before the next unit's
+// products start over, so no chain in the tensor cores is longer than a row; g is scaled to
+// 128 instead of 256, so that 512 full-scale terms stay below 2^24 (tc.cuh).
+struct WgradArgs {
+    const float* g;      // [batch][MO][n]
+    const float* gmax;   // [tiles per row][batch]
+    const float* x;      // [batch][W][n], through GELU with in_gelu
+    const float* xmax;   // [tiles per row][batch]
+    float* part;         // [blocks][MO][W]
+    float* rows;         // [blocks][MO]
+    int batch, n, seg, in_gelu;
+};
+template <int MO, int W>
+struct WgradSmem {
+    static constexpr int GP = 3 * MO * 16 + 16, XP = 3 * W * 16 + 16;  // plane pitches
+    struct Buf {
+        alignas(128) unsigned char g[8 * GP];
+        alignas(128) unsigned char x[8 * XP];
+    } buf[2];
+    unsigned char pad[2048];  // (lanes past the pieces read on: what they hold is not used)
+    uint64_t bar[2];
+    uint32_t tmem;
+};
+
+template <int MO, int W>
+__global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradArgs a) {
+    extern __shared__ __align__(128) unsigned char fno_smem[];
+    using Smem = WgradSmem<MO, W>;
+    Smem& S = *reinterpret_cast<Smem*>(fno_smem);
+    constexpr int GP = Smem::GP, XP = Smem::XP, COLS = W == 64 ? 256 : 128;
+    constexpr int IG = MO * 8 / WORKERS, IX = W * 8 / WORKERS;  // row pieces of 8 points per thread and chunk
+    const int tid = threadIdx.x;
+    if (tid >= WORKERS) tc::tmem_alloc(&S.tmem, COLS);
+    if (tid == WORKERS) {
+        tc::mbar_init(&S.bar[0], 1);
+        tc::mbar_init(&S.bar[1], 1);
+        tc::mbar_init_fence();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t d = S.tmem;
+    const int per_row = a.n / a.seg, units = a.batch * per_row, chunks = a.seg / 64;
+    const int mine = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x * chunks : 0;
+    if (tid >= WORKERS) {  // the issuing warp
+        for (int n = 0; n < mine; ++n) {
+            take_over(n & 1);
+            if (tid == WORKERS) {
+                tc::fence_after();
+                const uint32_t g = tc::smem_u32(S.buf[n & 1].g), x = tc::smem_u32(S.buf[n & 1].x);
+                const bool first = n % chunks == 0;
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    const uint64_t b = tc::smem_desc(x + 2 * k * XP, XP, 128);
+                    const uint32_t gk = g + 2 * k * GP;
+                    const bool add = !first || k > 0;
+                    tc::mma(d, tc::smem_desc(gk, GP, 128), b, tc::instr_desc(128, 3 * W), add);
+                    if (MO == 64) {
+                        tc::mma(d + 2 * W, tc::smem_desc(gk + 128 * 16, GP, 128), b, tc::instr_desc(128, W), true);
+                    } else if (MO == 128) {
+                        tc::mma(d + W, tc::smem_desc(gk + 128 * 16, GP, 128), b, tc::instr_desc(128, 2 * W), true);
+                        tc::mma(d + 2 * W, tc::smem_desc(gk + 256 * 16, GP, 128), b, tc::instr_desc(128, W), true);
+                    }
+                }
+                tc::commit(&S.bar[n & 1]);
+            }
+            __syncwarp();
+        }
+        tc::fence_before();
+        __syncthreads();
+        tc::tmem_free(S.tmem, COLS);
+        return;
+    }
+    const int c8 = tid & 7, r0 = tid >> 3;
+    bool fail = false;
+    uint32_t used = 0;
+    const int t = tid & 127, half = tid >> 7, group = t / MO;  // lane, column half, piece of the lane
+    float acc[W / 2], rs[IG];
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < IG; ++i) rs[i] = 0.f;
+    float4 vg[IG][2], vx[IX][2];
+    auto load = [&](int n) {
+        if (n >= mine) return;
+        const int u = blockIdx.x + n / chunks * gridDim.x, b = u / per_row;
+        const int p = (u % per_row) * a.seg + (n % chunks) * 64 + 8 * c8;
+#pragma unroll
+        for (int i = 0; i < IG; ++i) {
+            const float4* s = reinterpret_cast<const float4*>(a.g + ((int64_t)b * MO + r0 + 32 * i) * a.n + p);
+            vg[i][0] = __ldg(s);
+            vg[i][1] = __ldg(s + 1);
+        }
+#pragma unroll
+        for (int i = 0; i < IX; ++i) {
+            const float4* s = reinterpret_cast<const float4*>(a.x + ((int64_t)b * W + r0 + 32 * i) * a.n + p);
+            vx[i][0] = __ldg(s);
+            vx[i][1] = __ldg(s + 1);
+        }
+    };
+    auto put = [&](unsigned char* plane, int rows, int r, const float4(&w)[2], float inv, bool gelu) {
+        float2 e[4] = {make_float2(w[0].x, w[0].y), make_float2(w[0].z, w[0].w), make_float2(w[1].x, w[1].y),
+                       make_float2(w[1].z, w[1].w)};
+        uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (gelu) e[j] = act::gelu2(e[j]);
+            tc::split2(e[j], make_float2(inv, inv), hi[j], mid[j], lo[j]);
+        }
+        unsigned char* s = plane + r * 16;
+        *reinterpret_cast<uint4*>(s) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(s + rows * 16) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+        *reinterpret_cast<uint4*>(s + 2 * rows * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    };
+    float sg = 1.f, sx = 1.f;
+    const int nq = a.n < 128 ? 1 : a.n / 128;
+    load(0);
+#pragma unroll 1
+    for (int n = 0; n < mine; ++n) {
+        const int buf = n & 1;
+        if (n % chunks == 0) {  // the unit's scales: the max over its tiles
+            const int u = blockIdx.x + n / chunks * gridDim.x, b = u / per_row;
+            const int q0 = a.n < 128 ? 0 : (u % per_row) * a.seg / 128, q1 = a.seg < 128 ? q0 + 1 : q0 + a.seg / 128;
+            float mg = 0.f, mx = 0.f;
+            for (int q = q0; q < q1 && q < nq; ++q) {
+                mg = fmaxf(mg, __ldg(a.gmax + (int64_t)q * a.batch + b));
+                mx = fmaxf(mx, __ldg(a.xmax + (int64_t)q * a.batch + b));
+            }
+            sg = tc::pow2_above(mg);
+            sx = tc::pow2_above(mx);
+        }
+        if (n >= 2) {
+            if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
+            used ^= 1u << buf;
+        }
+#pragma unroll
+        for (int i = 0; i < IG; ++i) {
+            rs[i] += ((vg[i][0].x + vg[i][0].y) + (vg[i][0].z + vg[i][0].w)) +
+                     ((vg[i][1].x + vg[i][1].y) + (vg[i][1].z + vg[i][1].w));
+            put(S.buf[buf].g + c8 * GP, MO, r0 + 32 * i, vg[i], 128.f / sg, false);
+        }
+#pragma unroll
+        for (int i = 0; i < IX; ++i) put(S.buf[buf].x + c8 * XP, W, r0 + 32 * i, vx[i], 256.f / sx, a.in_gelu);
+        tc::fence_smem();
+        tc::fence_before();
+        hand_over(buf);
+        load(n + 1);
+        if (n % chunks != chunks - 1) continue;
+        // the unit's sums: every chunk's products done (the last of either buffer)
+        if (chunks > 1) {
+            if (!fail) fail = !tc::mbar_wait(&S.bar[buf ^ 1], (used >> (buf ^ 1)) & 1);
+        }
+        if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
+        tc::fence_after();
+        const float f = fail ? __int_as_float(0x7fffffff) : sg * (1.f / 128.f) * (sx * (1.f / 256.f));
+        const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + half * (W / 2);
+#pragma unroll
+        for (int c = 0; c < W / 2; c += 16) {
+            float q0[16], q1[16], q2[16];
+            tc::tmem_ld16(dl + c, q0);
+            tc::tmem_ld16(dl + W + c, q1);
+            tc::tmem_ld16(dl + 2 * W + c, q2);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                acc[c + i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
+        }
+        tc::fence_before();
+        worker_sync();  // read everywhere before the next unit's products
+    }
+    // the lanes' pieces added up (lo + mid + hi), then the block's slot
+    float* s = reinterpret_cast<float*>(S.buf[0].g);  // [128][W + 1]; every product is done
+    static_assert(sizeof(float) * 128 * (W + 1) <= sizeof(S.buf), "scratch");
+    worker_sync();
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) s[t * (W + 1) + half * (W / 2) + i] = acc[i];
+    worker_sync();
+    float* out = a.part + (int64_t)blockIdx.x * MO * W;
+    for (int i = tid; i < MO * W; i += WORKERS) {
+        const int o = i / W, c = i % W;
+        float r = s[o * (W + 1) + c];
+        if (MO == 32) r += s[(32 + o) * (W + 1) + c] + s[(64 + o) * (W + 1) + c];
+        if (MO == 64) r += s[(64 + o) * (W + 1) + c];
+        out[i] = r;
+    }
+#pragma unroll
+    for (int i = 0; i < IG; ++i) {
+        rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 1);
+        rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 2);
+        rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 4);
+        if (c8 == 0) a.rows[(int64_t)blockIdx.x * MO + r0 + 32 * i] = rs[i];
+    }
+    tc::fence_before();
+    __syncthreads();
+}
+
+// blocks of a weight gradient, and its unit: whole rows when there are plenty
+inline int wgrad_blocks(int batch, int n, int per_sm, int* seg) {
+    const int most = per_sm * sm_count();
+    *seg = batch >= 2 * most || n < 128 ? n : 128;
+    const int64_t units = (int64_t)batch * (n / *seg);
+    return units < most ? (int)units : most;
+}
+
+template <int MO, int W>
+int run_wgrad(WgradArgs a, int* blocks, cudaStream_t st) {
+    const size_t smem = sizeof(WgradSmem<MO, W>);
+    static_assert(sizeof(WgradSmem<MO, W>) <= (MO == 128 ? 227 : 113) * 1024, "shared memory");
+    cudaFuncSetAttribute(k_fno_wgrad<MO, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    *blocks = wgrad_blocks(a.batch, a.n, MO == 128 ? 1 : 2, &a.seg);
+    k_fno_wgrad<MO, W><<<*blocks, THREADS, smem, st>>>(a);
+    return check_launch("fno weight gradient");
+}
+
+// ---- Fourier weight gradients -------------------------------------------------------------
+// dW[c][o][k] = (c_k / n) sum_b conj(X[k][b][c]) G[k][b][o] (c_0 = 1, c_k = 2; torch's convention for
+// complex gradients), all four layers: block = mode, layer, a 32 x 32 tile of (c, o); thread 2 x 2.
+struct ModesGradArgs {
+    const float2* x;  // [4][modes][batch][W]
+    const float2* g;  // [4][modes][batch][W]
+    float2* out[4];   // [W][W][modes]
+    int batch, modes, n;
+};
+template <int W>
+__global__ void __launch_bounds__(256) k_fno_modes_grad(ModesGradArgs a) {
+    constexpr int TB = 32;
+    __shared__ float2 X[TB][32], G[TB][32];
+    const int k = blockIdx.x, l = blockIdx.y, c0 = blockIdx.z / (W / 32) * 32, o0 = blockIdx.z % (W / 32) * 32;
+    const int64_t base = ((int64_t)l * a.modes + k) * a.batch * W;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx, tx + 16; c: ty, ty + 16
+    float2 tot[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) tot[i][j] = make_float2(0.f, 0.f);
+    for (int b0 = 0; b0 < a.batch; b0 += TB) {
+#pragma unroll
+        for (int i = threadIdx.x; i < TB * 32; i += 256) {
+            const int b = i / 32, e = i % 32;
+            const bool in = b0 + b < a.batch;
+            X[b][e] = in ? __ldg(a.x + base + (int64_t)(b0 + b) * W + c0 + e) : make_float2(0.f, 0.f);
+            G[b][e] = in ? __ldg(a.g + base + (int64_t)(b0 + b) * W + o0 + e) : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+        float2 acc[2][2];  // (a chunk's sum first: shorter chains)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (int b = 0; b < TB; ++b)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float2 x = X[b][ty + 16 * i], g = G[b][tx + 16 * j];
+                    acc[i][j].x = fmaf(x.x, g.x, fmaf(x.y, g.y, acc[i][j].x));
+                    acc[i][j].y = fmaf(x.x, g.y, fmaf(-x.y, g.x, acc[i][j].y));
+                }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                tot[i][j].x += acc[i][j].x;
+                tot[i][j].y += acc[i][j].y;
+            }
+        __syncthreads();
+    }
+    const float s = (k == 0 ? 1.f : 2.f) / (float)a.n;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            a.out[l][((int64_t)(c0 + ty + 16 * i) * W + o0 + tx + 16 * j) * a.modes + k] =
+                make_float2(tot[i][j].x * s, tot[i][j].y * s);
+}
+
+// ---- the blocks' partial sums, added in a fixed order ---------------------------------------
+// job j: dst[i] = sum over p < count of src[p * stride + i], i < n.  Block: 32 outputs, 8 slices.
+constexpr int MAX_JOBS = 11;
+struct ReduceArgs {
+    const float* src[MAX_JOBS];
+    float* dst[MAX_JOBS];
+    int stride[MAX_JOBS], count[MAX_JOBS], n[MAX_JOBS], first[MAX_JOBS + 1];
+    int jobs;
+};
+__global__ void __launch_bounds__(256) k_fno_reduce(ReduceArgs a) {
+    __shared__ float s[8][33];
+    int j = 0;
+    while (j + 1 < a.jobs && (int)blockIdx.x >= a.first[j + 1]) ++j;
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int i = (blockIdx.x - a.first[j]) * 32 + lane;
+    float v = 0.f;
+    if (i < a.n[j]) {
+        const float* src = a.src[j] + i;
+#pragma unroll 4
+        for (int p = slice; p < a.count[j]; p += 8) v += __ldg(src + (int64_t)p * a.stride[j]);
+    }
+    s[slice][lane] = v;
+    __syncthreads();
+    if (slice == 0 && i < a.n[j]) {
+#pragma unroll
+        for (int q = 1; q < 8; ++q) v += s[q][lane];
+        a.dst[j][i] = v;
+    }
+}
+
+// Layer 0 and the lift from the six sums per channel: s[0..2][o] = sum dL/dz {u, grid, 1},
+// s[3..5][c] = sum dL/dh {u, grid, 1}, with h[c] = w[c][0] u + w[c][1] grid + b[c].
+template <int W>
+__global__ void __launch_bounds__(256) k_fno_lift_grad(const float* __restrict__ s, const float* __restrict__ w,
+                                                       const float* __restrict__ bias, float* __restrict__ g_w0,
+                                                       float* __restrict__ g_b0, float* __restrict__ g_fc0_w,
+                                                       float* __restrict__ g_fc0_b) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < W * W; i += gridDim.x * 256) {
+        const int o = i / W, c = i % W;
+        g_w0[i] = fmaf(w[2 * c], s[o], fmaf(w[2 * c + 1], s[W + o], bias[c] * s[2 * W + o]));
+        if (c == 0) {
+            g_b0[o] = s[2 * W + o];
+            g_fc0_w[2 * o] = s[3 * W + o];
+            g_fc0_w[2 * o + 1] = s[4 * W + o];
+            g_fc0_b[o] = s[5 * W + o];
+        }
+    }
+}
+
+// scratch of the backward, in floats
+template <int W>
+struct BwdWork {
+    int64_t prep, wt, mixed, gm, mmax, g1, gz, gzmax, g1max, sums, part, rows, six, total;
+    BwdWork(int64_t B, int64_t n, int64_t M) {
+        const int64_t nq = n < 128 ? 1 : n / 128, blocks = 2 * (int64_t)sm_count();
+        int64_t at = 0;
+        auto take = [&](int64_t floats) {
+            const int64_t r = at;
+            at += (floats + 3) / 4 * 4;  // (every array 16-byte aligned)
+            return r;
+        };
+        prep = take((int64_t)sizeof(Prep<W>) / 4);
+        wt = take(2 * 4 * M * W * W);
+        mixed = take(2 * M * B * W);
+        gm = take(2 * 4 * M * B * W);       // modes of dL/dz of every layer
+        mmax = take(4 * B);
+        g1 = take(B * 128 * n);
+        gz = take(2 * B * W * n);           // dL/dz of two layers in turn
+        gzmax = take(2 * nq * B);
+        g1max = take(nq * B);
+        sums = take(blocks * 132);
+        part = take(blocks * (128 * W + 3 * W * W));
+        rows = take(blocks * (128 + 3 * W));
+        six = take(blocks * 6 * W + 6 * W);
+        total = at;
+    }
+};
+
+template <int W>
+int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const float* z, const float* xm,
+                 const float* tmax, const inc_fno_grads* gr, float* work, cudaStream_t st) {
+    const int B = d->rows, n = d->n, M = d->modes, nq = n < 128 ? 1 : n / 128;
+    const int64_t state = (int64_t)B * W * n, modes = (int64_t)M * B * W;
+    const BwdWork<W> o(B, n, M);
+    Prep<W>* prep = reinterpret_cast<Prep<W>*>(work + o.prep);
+    float2* wt = reinterpret_cast<float2*>(work + o.wt);
+    float2* mixed = reinterpret_cast<float2*>(work + o.mixed);
+    float2* gm = reinterpret_cast<float2*>(work + o.gm);
+    float* gz = work + o.gz;
+    float* gzmax = work + o.gzmax;
+    const int64_t most = 2 * (int64_t)sm_count();
+    PrepArgs pa{};
+    for (int l = 0; l < 4; ++l) {
+        pa.modes_w[l] = reinterpret_cast<const float2*>(d->modes_w[l]);
+        pa.w[l] = d->w[l];
+    }
+    pa.fc1 = d->fc1_w;
+    pa.wt = wt;
+    pa.zero = work + o.mmax;
+    pa.batch = B;
+    pa.n = n;
+    pa.modes = M;
+    int rc = run_prep<W, true>(pa, prep, st);
+    if (rc) return rc;
+    ReduceArgs ra{};
+    auto job = [&](const float* src, float* dst, int stride, int count, int len) {
+        const int j = ra.jobs++;
+        ra.src[j] = src;
+        ra.dst[j] = dst;
+        ra.stride[j] = stride;
+        ra.count[j] = count;
+        ra.n[j] = len;
+        ra.first[j + 1] = ra.first[j] + (len + 31) / 32;
+    };
+    int blocks = 0;
+    {  // the projection: dL/dz of layer 3 into gz[1] (layer l's in gz[l & 1])
+        const ProjBwdArgs p{z + 3 * state, tmax + 3 * nq * B, prep->fc1, prep->scale + 4, d->fc1_b, d->fc2_w, g_y,
+                            work + o.g1, work + o.g1max, gz + state, gzmax + nq * B, work + o.sums, B};
+        switch (n) {
+            case 64: rc = launch_proj_bwd<W, 64>(p, &blocks, st); break;
+            case 128: rc = launch_proj_bwd<W, 128>(p, &blocks, st); break;
+            case 256: rc = launch_proj_bwd<W, 256>(p, &blocks, st); break;
+            default: rc = launch_proj_bwd<W, 512>(p, &blocks, st); break;
+        }
+        if (rc) return rc;
+        job(work + o.sums, gr->fc2_w, 132, blocks, 128);
+        job(work + o.sums + 128, gr->fc2_b, 132, blocks, 1);
+        float* part = work + o.part;
+        float* rows = work + o.rows;
+        rc = run_wgrad<128, W>(WgradArgs{work + o.g1, work + o.g1max, z + 3 * state, tmax + 3 * nq * B, part, rows, B, n, 0,
+                                         0}, &blocks, st);
+        if (rc) return rc;
+        job(part, gr->fc1_w, 128 * W, blocks, 128 * W);
+        job(rows, gr->fc1_b, 128, blocks, 128);
+    }
+    for (int l = 3; l >= 0; --l) {
+        const float* g = gz + (l & 1) * state;
+        const float* gmx = gzmax + (l & 1) * nq * B;
+        rc = run_modes<W>(ModesArgs{g, gmx, prep->transform, gm + l * modes, B * W, B, M, 0}, n, st);
+        if (rc) return rc;
+        rc = run_mix<W>(gm + l * modes, wt + (int64_t)l * M * W * W, mixed, work + o.mmax + l * B, B, n, M, st);
+        if (rc) return rc;
+        if (l > 0) {
+            float* part = work + o.part + most * (128 * W + (l - 1) * W * W);
+            float* rows = work + o.rows + most * (128 + (l - 1) * W);
+            rc = run_wgrad<W, W>(WgradArgs{g, gmx, z + (l - 1) * state, tmax + (int64_t)(l - 1) * nq * B, part, rows, B, n,
+                                           0, 1}, &blocks, st);
+            if (rc) return rc;
+            job(part, gr->w[l], W * W, blocks, W * W);
+            job(rows, gr->b[l], W, blocks, W);
+        }
+        LayerArgs a{};
+        a.x = g;
+        a.xmax = gmx;
+        a.w = prep->w[l];
+        a.inverse = prep->inverse[0];
+        a.wscale = prep->scale + l;
+        a.mixed = mixed;
+        a.mixed_max = work + o.mmax + l * B;
+        a.batch = B;
+        a.modes = M;
+        if (l > 0) {
+            a.zprev = z + (l - 1) * state;
+            a.out = gz + ((l - 1) & 1) * state;
+            a.tmax = gzmax + ((l - 1) & 1) * nq * B;
+            rc = run_layer<W, false, BWD>(a, n, st);
+        } else {
+            a.u = u;
+            a.grid = d->grid;
+            a.grid_stride = d->grid_stride;
+            a.fc0_w = d->fc0_w;
+            a.fc0_b = d->fc0_b;
+            a.g_u = gr->u;
+            a.sums = work + o.six + 6 * W;
+            rc = run_layer<W, false, BWD0>(a, n, st);
+        }
+        if (rc) return rc;
+    }
+    job(work + o.six + 6 * W, work + o.six, 6 * W, tile_grid(B, nq), 6 * W);
+    k_fno_reduce<<<ra.first[ra.jobs], 256, 0, st>>>(ra);
+    k_fno_lift_grad<W><<<W * W / 256, 256, 0, st>>>(work + o.six, d->fc0_w, d->fc0_b, gr->w[0], gr->b[0], gr->fc0_w,
+                                                   gr->fc0_b);
+    ModesGradArgs mg{};
+    mg.x = reinterpret_cast<const float2*>(xm);
+    mg.g = gm;
+    for (int l = 0; l < 4; ++l) mg.out[l] = reinterpret_cast<float2*>(gr->modes_w[l]);
+    mg.batch = B;
+    mg.modes = M;
+    mg.n = n;
+    k_fno_modes_grad<W><<<dim3(M, 4, (W / 32) * (W / 32)), 256, 0, st>>>(mg);
+    return check_launch("fno gradients");
+}
+
+}  // namespace fno
+}  // namespace inc
+
+using namespace inc;
+
+extern "C" int64_t inc_fno_backward_work_size(const inc_fno_desc* d) {
+    if (!d || d->rows <= 0 || !fno::supported(d->width, d->n, d->modes)) return -1;
+    return d->width == 64 ? fno::BwdWork<64>(d->rows, d->n, d->modes).total
+                          : fno::BwdWork<32>(d->rows, d->n, d->modes).total;
+}
+
+extern "C" int inc_fno_backward(const inc_fno_desc* d, const float* u, const float* g_y, const float* z,
+                                const float* x_modes, const float* tmax, const inc_fno_grads* g, float* work,
+                                void* stream) {
+    const int rc = fno::check_fno(d);
+    if (rc) return rc;
+    bool ok = u && g_y && z && x_modes && tmax && g && work && (reinterpret_cast<uintptr_t>(work) & 15u) == 0 &&
+              (reinterpret_cast<uintptr_t>(z) & 15u) == 0 && (reinterpret_cast<uintptr_t>(d->fc2_w) & 15u) == 0 &&
+              g->fc0_w && g->fc0_b && g->fc1_w && g->fc1_b && g->fc2_w && g->fc2_b;
+    for (int l = 0; ok && l < 4; ++l)
+        ok = g->modes_w[l] && g->w[l] && g->b[l] && (reinterpret_cast<uintptr_t>(g->modes_w[l]) & 7u) == 0;
+    if (!ok) {
+        set_error("fno_backward: bad arguments");
+        return INC_E_INVALID;
+    }
+    cudaStream_t st = as_stream(stream);
+    return d->width == 64 ? fno::run_backward<64>(d, u, g_y, z, x_modes, tmax, g, work, st)
+                          : fno::run_backward<32>(d, u, g_y, z, x_modes, tmax, g, work, st);
+}

@@ -55,6 +55,17 @@ INC_DEV void tmem_ld16(uint32_t addr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+INC_DEV void tmem_ld8(uint32_t addr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+INC_DEV void tmem_ld(uint32_t addr, float (&v)[16]) { tmem_ld16(addr, v); }
+INC_DEV void tmem_ld(uint32_t addr, float (&v)[8]) { tmem_ld8(addr, v); }
 INC_DEV void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- mbarrier --------------------------------------------------------------------
@@ -76,6 +87,18 @@ INC_DEV bool mbar_wait(uint64_t* b, uint32_t parity) {
         if (ok) return true;
     }
     return false;
+}
+
+// Bulk copy of a contiguous global array (16-byte aligned, bytes a multiple of 16) into this
+// CTA's shared memory; `b` expects its bytes (mbar_expect) and completes when they are there.
+INC_DEV void mbar_expect(uint64_t* b, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+INC_DEV void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(b))
+                 : "memory");
 }
 
 // ---- matrix instructions -----------------------------------------------------------
@@ -123,12 +146,12 @@ INC_DEV uint32_t cvt_bf16x2(float a, float b) {
 // x * inv (a power of two, |x * inv| <= 256) of two values -> their pieces, packed.
 // The products inside the fused operations are exact.
 INC_DEV void split2(float2 x, float2 inv, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const float2 M = make_float2(12582912.f, 12582912.f);  // 1.5 * 2^23: rounds to integers
+    const float2 M = make_float2(12582912.f, 12582912.f), m1 = make_float2(-1.f, -1.f);  // 1.5 * 2^23: to integers
     const float2 h = __fadd2_rn(__ffma2_rn(x, inv, M), make_float2(-M.x, -M.y));
-    const float2 r = __ffma2_rn(x, inv, make_float2(-h.x, -h.y));
+    const float2 r = __ffma2_rn(h, m1, __fmul2_rn(x, inv));
     hi = __byte_perm(__float_as_uint(h.x), __float_as_uint(h.y), 0x7632);  // integers <= 256: exact
     mid = cvt_bf16x2(r.x, r.y);
-    const float2 q = __fadd2_rn(r, make_float2(-__uint_as_float(mid << 16), -__uint_as_float(mid & 0xffff0000u)));
+    const float2 q = __ffma2_rn(make_float2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), m1, r);
     lo = cvt_bf16x2(q.x, q.y);
 }
 // eight values -> 16 bytes of each piece

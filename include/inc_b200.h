@@ -395,6 +395,56 @@ int inc_bias_gelu(const float* h, const float* bias, float* y, int32_t rows, int
 int inc_bias_gelu_bwd(const float* g_y, const float* h, const float* bias, float* g_h,
                       float* row_sums, int32_t rows, int32_t n, int32_t channels, void* stream);
 
+/* ---- corrector: the whole FNO ----------------------------------------------- */
+/* FNO1D.forward (models/models_1d/fno.py:39-105): y = fc2(gelu(fc1(layers(fc0([u, grid])))))
+ * with four layers h = gelu(conv(h) + w(h)) (no gelu after the last).  All parameters
+ * FP32 in torch's layouts: fc0_w [width][2], modes_w[l] complex [width in][width out][modes],
+ * w[l] [width][width], fc1_w [128][width], fc2_w [128].  width 32 or 64, n 64, 128, 256 or
+ * 512, 1 <= modes <= 16; others return INC_E_UNSUPPORTED.                        */
+typedef struct inc_fno_desc {
+    int32_t rows, n, width, modes;
+    int64_t grid_stride;        /* elements between the grid's rows (0: one row for all) */
+    const float* grid;          /* [rows][n] coordinates                                */
+    const float* fc0_w;
+    const float* fc0_b;
+    const float* modes_w[4];
+    const float* w[4];
+    const float* b[4];
+    const float* fc1_w;
+    const float* fc1_b;
+    const float* fc2_w;
+    const float* fc2_b;
+} inc_fno_desc;
+/* Floats of scratch (16-byte aligned) for a forward: train = 1 when z is given. */
+int64_t inc_fno_work_size(const inc_fno_desc* d, int32_t train);
+/* y [rows][n] = FNO(u [rows][n]).  For a backward, z [4][rows][width][n] receives the
+ * layers' sums before GELU, x_modes [4][modes][rows][width] complex the modes of the
+ * layers' inputs and tmax [4][max(1, n / 128)][rows] the tiles' magnitudes; all NULL
+ * for an evaluation.                                                             */
+int inc_fno_forward(const inc_fno_desc* d, const float* u, float* y, float* z, float* x_modes,
+                    float* tmax, float* work, void* stream);
+
+/* Its backward: the gradients of every parameter (torch's layouts; complex ones in
+ * torch's convention) and, when u is not NULL, of u, from g_y [rows][n] and what the
+ * forward recorded.  work: inc_fno_backward_work_size floats; z, work and fc2_w
+ * 16-byte aligned.                                                              */
+typedef struct inc_fno_grads {
+    float* u;
+    float* fc0_w;
+    float* fc0_b;
+    float* modes_w[4];
+    float* w[4];
+    float* b[4];
+    float* fc1_w;
+    float* fc1_b;
+    float* fc2_w;
+    float* fc2_b;
+} inc_fno_grads;
+int64_t inc_fno_backward_work_size(const inc_fno_desc* d);
+int inc_fno_backward(const inc_fno_desc* d, const float* u, const float* g_y, const float* z,
+                     const float* x_modes, const float* tmax, const inc_fno_grads* g, float* work,
+                     void* stream);
+
 /* ---- measurement utility ------------------------------------------------ */
 /* FP32 FMA throughput probe used by bench.py for the roofline denominator:
  * `blocks` x 256 threads, each 128 * iters FMAs (2 flops each) in 8

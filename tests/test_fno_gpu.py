@@ -1,0 +1,107 @@
+"""The whole FNO corrector on the GPU (inc_fno_forward / inc_fno_backward): outputs and every
+gradient against its FP64 copy on torch's FFTs, at the edges of its ranges (one row, odd
+batches, rows of half a tile to four tiles, the widths and mode counts it takes), rows of
+very different magnitude, and the calls that keep the general path."""
+import pytest
+import torch
+
+from inc_b200.correctors import FNO1D, fp64_copy
+
+pytestmark = pytest.mark.gpu
+TOL, GTOL = 1e-5, 1e-4  # max abs error over max abs FP64 value, as for the layers' own tests
+
+
+def _rel(a, ref):
+    a, ref = (torch.view_as_real(t) if t.is_complex() else t for t in (a.detach().cpu(), ref.detach().cpu()))
+    return (a.double() - ref).abs().max().item() / max(ref.abs().max().item(), 1e-30)
+
+
+def _net(width, modes, L=16):
+    torch.manual_seed(width + modes)
+    return FNO1D(L=L, modes=modes, width=width)
+
+
+def _fused(y):
+    return "FNOFn" in type(y.grad_fn).__name__
+
+
+@pytest.mark.parametrize("B,n,width,modes", [
+    (1, 64, 32, 1), (1, 512, 64, 16), (3, 64, 64, 16), (5, 128, 32, 5), (7, 256, 64, 12), (2, 512, 32, 16),
+    (65, 128, 64, 16), (149, 64, 64, 7), (150, 256, 32, 16), (301, 128, 64, 3)])
+def test_fno_matches_fp64(cuda, B, n, width, modes):
+    net = _net(width, modes)
+    g = torch.Generator().manual_seed(B + n)
+    u = torch.randn(B, n, generator=g, dtype=torch.float64)
+    L = 20.0 + torch.rand(B, generator=g, dtype=torch.float64)
+    gy = torch.randn(B, n, generator=g, dtype=torch.float64)
+    ref = fp64_copy(net)
+    ur = u.clone().requires_grad_(True)
+    yr = ref(ur, L.float().double())
+    yr.backward(gy)
+    net = net.to(cuda)
+    uc = u.float().to(cuda).requires_grad_(True)
+    y = net(uc, L.float().to(cuda))
+    assert _fused(y)
+    y.backward(gy.float().to(cuda))
+    with torch.no_grad():
+        assert _rel(net(uc, L.float().to(cuda)), yr) < TOL  # evaluation
+    assert _rel(y, yr) < TOL
+    assert _rel(uc.grad, ur.grad) < GTOL
+    for (name, p), (_, pr) in zip(net.named_parameters(), ref.named_parameters()):
+        assert _rel(p.grad, pr.grad) < GTOL, name
+
+
+def test_fno_rows_of_different_magnitude_and_non_finite(cuda):
+    """Each trajectory's tiles have their own scales: small and large states beside each other
+    and beside a non-finite one, each as accurate as alone."""
+    net = _net(64, 16)
+    u = torch.randn(6, 128, generator=torch.Generator().manual_seed(0), dtype=torch.float64)
+    u *= torch.tensor([0.0, 1e-6, 1.0, 1.0, 30.0, 1e3], dtype=torch.float64)[:, None]
+    ref = fp64_copy(net)
+    with torch.no_grad():
+        yr = ref(u)
+        u[2, 40] = float("nan")
+        y = net.to(cuda)(u.float().to(cuda)).cpu()
+    assert torch.isnan(y[2]).any()
+    for r in (0, 1, 3, 4, 5):
+        assert _rel(y[r], yr[r]) < TOL, r
+
+
+def test_fno_general_path_is_kept_and_agrees(cuda):
+    """Hooked layers, a domain size that needs a gradient, and shapes outside the fused kernels
+    run layer by layer, with the same results."""
+    net = _net(64, 16).to(cuda)
+    u = torch.randn(4, 128, generator=torch.Generator().manual_seed(1)).to(cuda).requires_grad_(True)
+    y = net(u)
+    assert _fused(y)
+    seen = []
+    h = net.conv1.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+    yh = net(u)
+    h.remove()
+    assert not _fused(yh) and seen == [(4, 64, 128)]
+    assert _rel(yh, y.double()) < TOL
+    L = torch.full((4,), 16.0, device=cuda, requires_grad=True)
+    yl = net(u, L)
+    yl.sum().backward()
+    assert not _fused(yl) and L.grad is not None and _rel(yl, y.double()) < TOL
+    for width, modes, n in ((16, 8, 128), (64, 20, 128), (64, 16, 32)):
+        out = _net(width, modes).to(cuda)(torch.randn(2, n, device=cuda))
+        assert out.shape == (2, n) and not _fused(out)
+
+
+def test_fno_partial_gradients_and_permuted_input(cuda):
+    """Only what asks for a gradient gets one; a permuted (non-contiguous) state is taken."""
+    net = _net(32, 8).to(cuda)
+    u = torch.randn(128, 3, generator=torch.Generator().manual_seed(2)).to(cuda).t()
+    assert not u.is_contiguous()
+    net(u).square().mean().backward()
+    full = [p.grad.clone() for p in net.parameters()]
+    net.zero_grad()
+    for p in net.parameters():
+        p.requires_grad_(False)
+    net.w2.weight.requires_grad_(True)
+    uc = u.contiguous().requires_grad_(True)
+    net(uc).square().mean().backward()
+    assert uc.grad is not None
+    for (name, p), g in zip(net.named_parameters(), full):
+        assert (p.grad is None) if name != "w2.weight" else torch.equal(p.grad, g), name
