@@ -45,22 +45,33 @@ class BurgersRolloutFn(torch.autograd.Function):
         return g_u0, g_s, None, None, None, None
 
 
+# Largest tape (bytes) a checkpointed KS rollout takes in place of its checkpoints.  The tape's
+# backward has 9 row-pair transforms a step against 17 for replay and adjoint: forward and
+# backward of 512 x 512, 64 steps 574 -> 424 us (268 MB), 1024 x 256, 40 steps 352 -> 276 us,
+# 37 x 64, 40 steps 167 -> 122 us; no measured shape was slower.  Longer rollouts of large
+# batches keep the checkpoints, whose memory does not grow as fast (1 / (4 ckpt_every) of it).
+KS_TAPE_BYTES_MAX = 1 << 30
+
+
 class KSRolloutFn(torch.autograd.Function):
     """ckpt_every > 0: checkpoints every ckpt_every steps, segments replayed in the
-    backward; ckpt_every == 0: a tape of every step's states (no replay, more memory)."""
+    backward, or a tape of every step's states (no replay, more memory) where that is at most
+    KS_TAPE_BYTES_MAX; ckpt_every == 0: the tape."""
 
     @staticmethod
     def forward(ctx, u0, s, plan, steps, ckpt_every, want_grad):
         B, N = u0.shape
         frames = torch.empty(B, steps, N, device=u0.device, dtype=u0.dtype)
-        if want_grad and ckpt_every == 0:
+        tape = want_grad and (ckpt_every == 0 or (ckpt_every > 0 and steps > 0
+                                                      and plan.tape_size(steps) <= KS_TAPE_BYTES_MAX))
+        if tape:
             saved = torch.empty(plan.tape_size(steps), dtype=torch.uint8, device=u0.device)
             plan.rollout_tape(u0, s, steps, frames, None, saved)
         else:
             k = ckpt_every if ckpt_every > 0 else 8
             saved = torch.empty(B, _nseg(steps, k), N, device=u0.device, dtype=u0.dtype) if want_grad else None
             plan.rollout(u0, s, steps, frames, None, k, saved)
-        ctx.plan, ctx.steps, ctx.k, ctx.has_s = plan, steps, ckpt_every, s is not None
+        ctx.plan, ctx.steps, ctx.k, ctx.has_s = plan, steps, (0 if tape else ckpt_every), s is not None
         ctx.shape = (B, N)
         if want_grad:
             ctx.save_for_backward(saved, s if s is not None else u0.new_empty(0))
@@ -105,7 +116,8 @@ def ks_rollout(solver: KSSolverTorch, u0, steps, domain_size, s=None, ckpt_every
 
     Differentiable w.r.t. u0 and s.  The backward replays ckpt_every-step segments from
     checkpoints; ckpt_every=0 records every step's states in a tape instead (32 bytes per
-    row pair, cell and step) and the backward reads them, with no replay."""
+    row pair, cell and step) and the backward reads them, with no replay.  A tape of at most
+    KS_TAPE_BYTES_MAX is taken for any ckpt_every: the same gradients to rounding, faster."""
     _check_state(u0, solver.resolution)
     u0 = u0.contiguous()
     s = _contig(s)

@@ -397,3 +397,28 @@ def test_errors(cuda):
     solver = _solver(64, 0.1)
     with pytest.raises(ValueError):
         solver.step(torch.zeros(2, 64, device=cuda), torch.tensor([64.0, -1.0], device=cuda))
+
+
+@pytest.mark.parametrize("B,N,steps,k", [(1, 16, 1, 1), (37, 64, 9, 4), (6, 256, 13, 8), (3, 512, 5, 8)])
+def test_rollout_gradients_tape_in_place_of_checkpoints(cuda, monkeypatch, B, N, steps, k):
+    """A small rollout takes the tape whatever ckpt_every says; above the bound it keeps its
+    checkpoints: frames alike, gradients equal to rounding, with and without s."""
+    from inc_b200 import rollout as ro
+    rng = np.random.default_rng(B + N)
+    L = 0.22 * N
+    ds = torch.full((B,), L, device=cuda)
+    u0 = np.cos(2 * np.pi * np.arange(N) / N)[None] * rng.uniform(0.5, 1.5, (B, 1))
+    for with_s in (True, False):
+        got = []
+        for bound in (ro.KS_TAPE_BYTES_MAX, 0):
+            monkeypatch.setattr(ro, "KS_TAPE_BYTES_MAX", bound)
+            solver = _solver(N, 0.1, "ETRK2", [L] * B)
+            u = torch.tensor(u0, dtype=torch.float32, device=cuda, requires_grad=True)
+            s = torch.full((B, N), 0.02, device=cuda, requires_grad=True) if with_s else None
+            fr = ro.ks_rollout(solver, u, steps, ds, s=s, ckpt_every=k)
+            assert fr.grad_fn.k == (0 if bound else k)
+            (fr * torch.linspace(-1, 1, N, device=cuda)).sum().backward()
+            got.append([fr.detach(), u.grad] + ([s.grad] if with_s else []))
+            monkeypatch.undo()
+        for a, b in zip(*got):
+            assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
