@@ -78,10 +78,9 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // the issuing warp: three products per tile
         const bool ok = tc::mbar_wait(&S.bar_images, 0);
-        (void)ok;
         for (int i = blockIdx.x; i < tiles; i += step) {
             take_over();
-            if (tid == WORKERS) {  // hidden values: columns 0..127 and 128..255
+            if (tid == WORKERS && ok) {  // hidden values: columns 0..127 and 128..255
                 tc::fence_after();
                 issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 tc::commit(&S.bar);
@@ -90,7 +89,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {  // dL/dx += g1[64 h ..] w1, into columns 0.. and 128.., read by then
                 take_over();
-                if (tid == WORKERS) {
+                if (tid == WORKERS && ok) {
                     tc::fence_after();
                     const uint32_t x = tc::smem_u32(S.x), w = tc::smem_u32(S.w) + 64 * h * 16;
                     constexpr uint32_t id = tc::instr_desc(128, W, false, true);
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
     const float ws = __ldg(a.wscale) * (1.f / 65536.f), gbound = 1.13f * S.w2max;  // max gelu' = 1.1290
     const uint32_t dl = d + ((uint32_t)(t & 96) << 16);
     uint32_t phase = 0;
-    bool fail = !tc::mbar_wait(&S.bar_images, 0);
+    bool fail = false;
     auto wait = [&] {
         if (!fail) fail = !tc::mbar_wait(&S.bar, phase);
         phase ^= 1;
@@ -272,6 +271,7 @@ struct WgradArgs {
     float* rows;         // [blocks][MO]
     int batch, n, seg, in_gelu;
 };
+constexpr int WG_WORKERS = 512;
 template <int MO, int W>
 struct WgradSmem {
     static constexpr int GP = 3 * MO * 16 + 16, XP = 3 * W * 16 + 16;  // plane pitches
@@ -285,15 +285,17 @@ struct WgradSmem {
 };
 
 template <int MO, int W>
-__global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradArgs a) {
+__global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];
     using Smem = WgradSmem<MO, W>;
     Smem& S = *reinterpret_cast<Smem*>(fno_smem);
     constexpr int GP = Smem::GP, XP = Smem::XP, COLS = W == 64 ? 256 : 128;
-    constexpr int IG = MO * 8 / WORKERS, IX = W * 8 / WORKERS;  // row pieces of 8 points per thread and chunk
+    // pieces of 8 points of a row of g (the first MO rows) or x, per thread and chunk; the
+    // last round may be half a block
+    constexpr int ITEMS = (MO + W) * 8, IT = (ITEMS + WG_WORKERS - 1) / WG_WORKERS;
     const int tid = threadIdx.x;
-    if (tid >= WORKERS) tc::tmem_alloc(&S.tmem, COLS);
-    if (tid == WORKERS) {
+    if (tid >= WG_WORKERS) tc::tmem_alloc(&S.tmem, COLS);
+    if (tid == WG_WORKERS) {
         tc::mbar_init(&S.bar[0], 1);
         tc::mbar_init(&S.bar[1], 1);
         tc::mbar_init_fence();
@@ -304,10 +306,10 @@ __global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradA
     const uint32_t d = S.tmem;
     const int per_row = a.n / a.seg, units = a.batch * per_row, chunks = a.seg / 64;
     const int mine = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x * chunks : 0;
-    if (tid >= WORKERS) {  // the issuing warp
+    if (tid >= WG_WORKERS) {  // the issuing warp
         for (int n = 0; n < mine; ++n) {
-            take_over(n & 1);
-            if (tid == WORKERS) {
+            take_over<WG_WORKERS>(n & 1);
+            if (tid == WG_WORKERS) {
                 tc::fence_after();
                 const uint32_t g = tc::smem_u32(S.buf[n & 1].g), x = tc::smem_u32(S.buf[n & 1].x);
                 const bool first = n % chunks == 0;
@@ -336,50 +338,35 @@ __global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradA
     const int c8 = tid & 7, r0 = tid >> 3;
     bool fail = false;
     uint32_t used = 0;
-    const int t = tid & 127, half = tid >> 7, group = t / MO;  // lane, column half, piece of the lane
-    float acc[W / 2], rs[IG];
+    // lane, quarter of the columns, piece of the lane
+    constexpr int CQ = W / 4;
+    const int t = tid & 127, quarter = tid >> 7, group = t / MO;
+    float acc[CQ], rs[IT];
 #pragma unroll
-    for (int i = 0; i < W / 2; ++i) acc[i] = 0.f;
+    for (int i = 0; i < CQ; ++i) acc[i] = 0.f;
 #pragma unroll
-    for (int i = 0; i < IG; ++i) rs[i] = 0.f;
-    float4 vg[IG][2], vx[IX][2];
-    auto load = [&](int n) {
+    for (int i = 0; i < IT; ++i) rs[i] = 0.f;
+    // chunks are loaded two ahead (one where a thread's share is large: registers)
+    constexpr int DEPTH = IT <= 2 ? 2 : 1;
+    float4 v[DEPTH][IT][2];
+    auto load = [&](int n, float4(&w)[IT][2]) {
         if (n >= mine) return;
         const int u = blockIdx.x + n / chunks * gridDim.x, b = u / per_row;
         const int p = (u % per_row) * a.seg + (n % chunks) * 64 + 8 * c8;
 #pragma unroll
-        for (int i = 0; i < IG; ++i) {
-            const float4* s = reinterpret_cast<const float4*>(a.g + ((int64_t)b * MO + r0 + 32 * i) * a.n + p);
-            vg[i][0] = __ldg(s);
-            vg[i][1] = __ldg(s + 1);
+        for (int i = 0; i < IT; ++i) {
+            const int r = r0 + 64 * i;
+            if (r < MO + W) {
+                const float4* s = reinterpret_cast<const float4*>(
+                    r < MO ? a.g + ((int64_t)b * MO + r) * a.n + p : a.x + ((int64_t)b * W + r - MO) * a.n + p);
+                w[i][0] = ldg_na4(s);
+                w[i][1] = ldg_na4(s + 1);
+            }
         }
-#pragma unroll
-        for (int i = 0; i < IX; ++i) {
-            const float4* s = reinterpret_cast<const float4*>(a.x + ((int64_t)b * W + r0 + 32 * i) * a.n + p);
-            vx[i][0] = __ldg(s);
-            vx[i][1] = __ldg(s + 1);
-        }
-    };
-    auto put = [&](unsigned char* plane, int rows, int r, const float4(&w)[2], float inv, bool gelu) {
-        float2 e[4] = {make_float2(w[0].x, w[0].y), make_float2(w[0].z, w[0].w), make_float2(w[1].x, w[1].y),
-                       make_float2(w[1].z, w[1].w)};
-        uint32_t hi[4], mid[4], lo[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (gelu) e[j] = act::gelu2(e[j]);
-            tc::split2(e[j], make_float2(inv, inv), hi[j], mid[j], lo[j]);
-        }
-        unsigned char* s = plane + r * 16;
-        *reinterpret_cast<uint4*>(s) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(s + rows * 16) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-        *reinterpret_cast<uint4*>(s + 2 * rows * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     };
     float sg = 1.f, sx = 1.f;
     const int nq = a.n < 128 ? 1 : a.n / 128;
-    load(0);
-#pragma unroll 1
-    for (int n = 0; n < mine; ++n) {
-        const int buf = n & 1;
+    auto chunk = [&](int n, int buf, float4(&w)[IT][2]) {
         if (n % chunks == 0) {  // the unit's scales: the max over its tiles
             const int u = blockIdx.x + n / chunks * gridDim.x, b = u / per_row;
             const int q0 = a.n < 128 ? 0 : (u % per_row) * a.seg / 128, q1 = a.seg < 128 ? q0 + 1 : q0 + a.seg / 128;
@@ -396,18 +383,34 @@ __global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradA
             used ^= 1u << buf;
         }
 #pragma unroll
-        for (int i = 0; i < IG; ++i) {
-            rs[i] += ((vg[i][0].x + vg[i][0].y) + (vg[i][0].z + vg[i][0].w)) +
-                     ((vg[i][1].x + vg[i][1].y) + (vg[i][1].z + vg[i][1].w));
-            put(S.buf[buf].g + c8 * GP, MO, r0 + 32 * i, vg[i], 128.f / sg, false);
-        }
+        for (int i = 0; i < IT; ++i) {
+            const int r = r0 + 64 * i;  // (a warp's rows are all of g or all of x)
+            if (r < MO + W) {
+                const bool is_g = r < MO;
+                float2 e[4] = {make_float2(w[i][0].x, w[i][0].y), make_float2(w[i][0].z, w[i][0].w),
+                               make_float2(w[i][1].x, w[i][1].y), make_float2(w[i][1].z, w[i][1].w)};
+                if (is_g) {
+                    rs[i] += ((e[0].x + e[0].y) + (e[1].x + e[1].y)) + ((e[2].x + e[2].y) + (e[3].x + e[3].y));
+                } else if (a.in_gelu) {
 #pragma unroll
-        for (int i = 0; i < IX; ++i) put(S.buf[buf].x + c8 * XP, W, r0 + 32 * i, vx[i], 256.f / sx, a.in_gelu);
+                    for (int j = 0; j < 4; ++j) e[j] = act::gelu2(e[j]);
+                }
+                const float inv = is_g ? 128.f / sg : 256.f / sx;
+                uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) tc::split2(e[j], make_float2(inv, inv), hi[j], mid[j], lo[j]);
+                unsigned char* s = is_g ? S.buf[buf].g + c8 * GP + r * 16 : S.buf[buf].x + c8 * XP + (r - MO) * 16;
+                const int piece = (is_g ? MO : W) * 16;
+                *reinterpret_cast<uint4*>(s) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(s + piece) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+                *reinterpret_cast<uint4*>(s + 2 * piece) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        }
         tc::fence_smem();
         tc::fence_before();
-        hand_over(buf);
-        load(n + 1);
-        if (n % chunks != chunks - 1) continue;
+        hand_over<WG_WORKERS>(buf);
+        load(n + DEPTH, w);
+        if (n % chunks != chunks - 1) return;
         // the unit's sums: every chunk's products done (the last of either buffer)
         if (chunks > 1) {
             if (!fail) fail = !tc::mbar_wait(&S.bar[buf ^ 1], (used >> (buf ^ 1)) & 1);
@@ -415,30 +418,34 @@ __global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradA
         if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
         tc::fence_after();
         const float f = fail ? __int_as_float(0x7fffffff) : sg * (1.f / 128.f) * (sx * (1.f / 256.f));
-        const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + half * (W / 2);
+        const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + quarter * CQ;
+        float q0[CQ], q1[CQ], q2[CQ];
+        tc::tmem_ld(dl, q0);
+        tc::tmem_ld(dl + W, q1);
+        tc::tmem_ld(dl + 2 * W, q2);
+        tc::tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < W / 2; c += 16) {
-            float q0[16], q1[16], q2[16];
-            tc::tmem_ld16(dl + c, q0);
-            tc::tmem_ld16(dl + W + c, q1);
-            tc::tmem_ld16(dl + 2 * W + c, q2);
-            tc::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                acc[c + i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
-        }
+        for (int i = 0; i < CQ; ++i)
+            acc[i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
         tc::fence_before();
-        worker_sync();  // read everywhere before the next unit's products
+        worker_sync<WG_WORKERS>();  // read everywhere before the next unit's products
+    };
+    load(0, v[0]);
+    if (DEPTH == 2) load(1, v[DEPTH - 1]);
+#pragma unroll 1
+    for (int n = 0; n < mine; n += 2) {
+        chunk(n, 0, v[0]);
+        if (n + 1 < mine) chunk(n + 1, 1, v[DEPTH - 1]);
     }
-    // the lanes' pieces added up (lo + mid + hi), then the block's slot
+    // the lanes' pieces added up (hi, then mid and lo), then the block's slot
     float* s = reinterpret_cast<float*>(S.buf[0].g);  // [128][W + 1]; every product is done
     static_assert(sizeof(float) * 128 * (W + 1) <= sizeof(S.buf), "scratch");
-    worker_sync();
+    worker_sync<WG_WORKERS>();
 #pragma unroll
-    for (int i = 0; i < W / 2; ++i) s[t * (W + 1) + half * (W / 2) + i] = acc[i];
-    worker_sync();
+    for (int i = 0; i < CQ; ++i) s[t * (W + 1) + quarter * CQ + i] = acc[i];
+    worker_sync<WG_WORKERS>();
     float* out = a.part + (int64_t)blockIdx.x * MO * W;
-    for (int i = tid; i < MO * W; i += WORKERS) {
+    for (int i = tid; i < MO * W; i += WG_WORKERS) {
         const int o = i / W, c = i % W;
         float r = s[o * (W + 1) + c];
         if (MO == 32) r += s[(32 + o) * (W + 1) + c] + s[(64 + o) * (W + 1) + c];
@@ -446,37 +453,40 @@ __global__ void __launch_bounds__(THREADS, MO == 128 ? 1 : 2) k_fno_wgrad(WgradA
         out[i] = r;
     }
 #pragma unroll
-    for (int i = 0; i < IG; ++i) {
+    for (int i = 0; i < IT; ++i) {
         rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 1);
         rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 2);
         rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 4);
-        if (c8 == 0) a.rows[(int64_t)blockIdx.x * MO + r0 + 32 * i] = rs[i];
+        if (c8 == 0 && r0 + 64 * i < MO) a.rows[(int64_t)blockIdx.x * MO + r0 + 64 * i] = rs[i];
     }
     tc::fence_before();
     __syncthreads();
 }
 
-// blocks of a weight gradient, and its unit: whole rows when there are plenty
-inline int wgrad_blocks(int batch, int n, int per_sm, int* seg) {
-    const int most = per_sm * sm_count();
-    *seg = batch >= 2 * most || n < 128 ? n : 128;
-    const int64_t units = (int64_t)batch * (n / *seg);
-    return units < most ? (int)units : most;
+// a unit: 128 points while that leaves a block few units, else as many as a row has (fewer
+// reads of the accumulators)
+inline int wgrad_seg(int batch, int n) {
+    if (n <= 128) return n;
+    return (int64_t)batch * (n / 128) <= 16 * (int64_t)sm_count() ? 128 : n;
 }
 
 template <int MO, int W>
 int run_wgrad(WgradArgs a, int* blocks, cudaStream_t st) {
     const size_t smem = sizeof(WgradSmem<MO, W>);
-    static_assert(sizeof(WgradSmem<MO, W>) <= (MO == 128 ? 227 : 113) * 1024, "shared memory");
+    static_assert(sizeof(WgradSmem<MO, W>) <= 227 * 1024, "shared memory");
     cudaFuncSetAttribute(k_fno_wgrad<MO, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    *blocks = wgrad_blocks(a.batch, a.n, MO == 128 ? 1 : 2, &a.seg);
-    k_fno_wgrad<MO, W><<<*blocks, THREADS, smem, st>>>(a);
+    a.seg = wgrad_seg(a.batch, a.n);
+    const int64_t units = (int64_t)a.batch * (a.n / a.seg);
+    *blocks = units < sm_count() ? (int)units : sm_count();
+    k_fno_wgrad<MO, W><<<*blocks, WG_WORKERS + 32, smem, st>>>(a);
     return check_launch("fno weight gradient");
 }
 
 // ---- Fourier weight gradients -------------------------------------------------------------
 // dW[c][o][k] = (c_k / n) sum_b conj(X[k][b][c]) G[k][b][o] (c_0 = 1, c_k = 2; torch's convention for
-// complex gradients), all four layers: block = mode, layer, a 32 x 32 tile of (c, o); thread 2 x 2.
+// complex gradients), all four layers: block = mode, layer, 32 of the o; thread: 4 c x 2 o, the
+// factors Re X and Im X in separate packed accumulators (two packed operations per complex
+// product), the next 16 trajectories loaded while these are multiplied.
 struct ModesGradArgs {
     const float2* x;  // [4][modes][batch][W]
     const float2* g;  // [4][modes][batch][W]
@@ -484,61 +494,76 @@ struct ModesGradArgs {
     int batch, modes, n;
 };
 template <int W>
-__global__ void __launch_bounds__(256) k_fno_modes_grad(ModesGradArgs a) {
-    constexpr int TB = 32;
-    __shared__ float2 X[TB][32], G[TB][32];
-    const int k = blockIdx.x, l = blockIdx.y, c0 = blockIdx.z / (W / 32) * 32, o0 = blockIdx.z % (W / 32) * 32;
+__global__ void __launch_bounds__(W * 4) k_fno_modes_grad(ModesGradArgs a) {
+    constexpr int TB = 16, T = W * 4, LX = TB * W / T, LG = TB * 32 / T;
+    __shared__ float2 X[TB][W], G[TB][32];
+    const int k = blockIdx.x, l = blockIdx.y, o0 = blockIdx.z * 32;
     const int64_t base = ((int64_t)l * a.modes + k) * a.batch * W;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx, tx + 16; c: ty, ty + 16
-    float2 tot[2][2];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx, tx + 16; c: ty + i W / 4
+    float2 rx[LX], rg[LG];
+    auto load = [&](int b0) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) tot[i][j] = make_float2(0.f, 0.f);
-    for (int b0 = 0; b0 < a.batch; b0 += TB) {
-#pragma unroll
-        for (int i = threadIdx.x; i < TB * 32; i += 256) {
-            const int b = i / 32, e = i % 32;
-            const bool in = b0 + b < a.batch;
-            X[b][e] = in ? __ldg(a.x + base + (int64_t)(b0 + b) * W + c0 + e) : make_float2(0.f, 0.f);
-            G[b][e] = in ? __ldg(a.g + base + (int64_t)(b0 + b) * W + o0 + e) : make_float2(0.f, 0.f);
+        for (int i = 0; i < LX; ++i) {
+            const int e = threadIdx.x + i * T, b = b0 + e / W;
+            rx[i] = b < a.batch ? __ldg(a.x + base + (int64_t)b * W + e % W) : make_float2(0.f, 0.f);
         }
+#pragma unroll
+        for (int i = 0; i < LG; ++i) {
+            const int e = threadIdx.x + i * T, b = b0 + e / 32;
+            rg[i] = b < a.batch ? __ldg(a.g + base + (int64_t)b * W + o0 + e % 32) : make_float2(0.f, 0.f);
+        }
+    };
+    float2 tre[4][2], tim[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) tre[i][j] = tim[i][j] = make_float2(0.f, 0.f);
+    load(0);
+    for (int b0 = 0; b0 < a.batch; b0 += TB) {
         __syncthreads();
-        float2 acc[2][2];  // (a chunk's sum first: shorter chains)
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < LX; ++i) (&X[0][0])[threadIdx.x + i * T] = rx[i];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 8
-        for (int b = 0; b < TB; ++b)
+        for (int i = 0; i < LG; ++i) (&G[0][0])[threadIdx.x + i * T] = rg[i];
+        __syncthreads();
+        if (b0 + TB < a.batch) load(b0 + TB);
+        float2 re[4][2], im[4][2];  // (a chunk's sum first: shorter chains)
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < TB; ++b) {
+            const float2 g[2] = {G[b][tx], G[b][tx + 16]};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 x = X[b][ty + i * (W / 4)];
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const float2 x = X[b][ty + 16 * i], g = G[b][tx + 16 * j];
-                    acc[i][j].x = fmaf(x.x, g.x, fmaf(x.y, g.y, acc[i][j].x));
-                    acc[i][j].y = fmaf(x.x, g.y, fmaf(-x.y, g.x, acc[i][j].y));
+                    re[i][j] = __ffma2_rn(make_float2(x.x, x.x), g[j], re[i][j]);
+                    im[i][j] = __ffma2_rn(make_float2(x.y, x.y), g[j], im[i][j]);
                 }
+            }
+        }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                tot[i][j].x += acc[i][j].x;
-                tot[i][j].y += acc[i][j].y;
+                tre[i][j] = __fadd2_rn(tre[i][j], re[i][j]);
+                tim[i][j] = __fadd2_rn(tim[i][j], im[i][j]);
             }
-        __syncthreads();
     }
     const float s = (k == 0 ? 1.f : 2.f) / (float)a.n;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-            a.out[l][((int64_t)(c0 + ty + 16 * i) * W + o0 + tx + 16 * j) * a.modes + k] =
-                make_float2(tot[i][j].x * s, tot[i][j].y * s);
+        for (int j = 0; j < 2; ++j)  // conj(x) g = (x.x g.x + x.y g.y, x.x g.y - x.y g.x)
+            a.out[l][((int64_t)(ty + i * (W / 4)) * W + o0 + tx + 16 * j) * a.modes + k] =
+                make_float2((tre[i][j].x + tim[i][j].y) * s, (tre[i][j].y - tim[i][j].x) * s);
 }
 
 // ---- the blocks' partial sums, added in a fixed order ---------------------------------------
-// job j: dst[i] = sum over p < count of src[p * stride + i], i < n.  Block: 32 outputs, 8 slices.
+// job j: dst[i] = sum over p < count of src[p * stride + i], i < n.  Block: 32 outputs, 32 slices.
 constexpr int MAX_JOBS = 11;
 struct ReduceArgs {
     const float* src[MAX_JOBS];
@@ -546,8 +571,8 @@ struct ReduceArgs {
     int stride[MAX_JOBS], count[MAX_JOBS], n[MAX_JOBS], first[MAX_JOBS + 1];
     int jobs;
 };
-__global__ void __launch_bounds__(256) k_fno_reduce(ReduceArgs a) {
-    __shared__ float s[8][33];
+__global__ void __launch_bounds__(1024) k_fno_reduce(ReduceArgs a) {
+    __shared__ float s[32][33];
     int j = 0;
     while (j + 1 < a.jobs && (int)blockIdx.x >= a.first[j + 1]) ++j;
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
@@ -555,15 +580,16 @@ __global__ void __launch_bounds__(256) k_fno_reduce(ReduceArgs a) {
     float v = 0.f;
     if (i < a.n[j]) {
         const float* src = a.src[j] + i;
-#pragma unroll 4
-        for (int p = slice; p < a.count[j]; p += 8) v += __ldg(src + (int64_t)p * a.stride[j]);
+#pragma unroll 5
+        for (int p = slice; p < a.count[j]; p += 32) v += __ldg(src + (int64_t)p * a.stride[j]);
     }
     s[slice][lane] = v;
     __syncthreads();
-    if (slice == 0 && i < a.n[j]) {
+    if (threadIdx.x < 32 && i < a.n[j]) {
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int q = 1; q < 8; ++q) v += s[q][lane];
-        a.dst[j][i] = v;
+        for (int q = 0; q < 32; ++q) t[q & 3] += s[q][lane];
+        a.dst[j][i] = (t[0] + t[1]) + (t[2] + t[3]);
     }
 }
 
@@ -716,7 +742,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
         if (rc) return rc;
     }
     job(work + o.six + 6 * W, work + o.six, 6 * W, tile_grid(B, nq), 6 * W);
-    k_fno_reduce<<<ra.first[ra.jobs], 256, 0, st>>>(ra);
+    k_fno_reduce<<<ra.first[ra.jobs], 1024, 0, st>>>(ra);
     k_fno_lift_grad<W><<<W * W / 256, 256, 0, st>>>(work + o.six, d->fc0_w, d->fc0_b, gr->w[0], gr->b[0], gr->fc0_w,
                                                    gr->fc0_b);
     ModesGradArgs mg{};
@@ -726,7 +752,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
     mg.batch = B;
     mg.modes = M;
     mg.n = n;
-    k_fno_modes_grad<W><<<dim3(M, 4, (W / 32) * (W / 32)), 256, 0, st>>>(mg);
+    k_fno_modes_grad<W><<<dim3(M, 4, W / 32), W * 4, 0, st>>>(mg);
     return check_launch("fno gradients");
 }
 

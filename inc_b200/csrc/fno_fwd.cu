@@ -65,10 +65,9 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // the issuing warp
         const bool ok = tc::mbar_wait(&S.bar_images, 0);
-        (void)ok;
         for (int i = blockIdx.x; i < tiles; i += step) {
             take_over();
-            if (tid == WORKERS) {
+            if (tid == WORKERS && ok) {
                 tc::fence_after();
                 issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 tc::commit(&S.bar);
@@ -84,7 +83,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
     const float ws = __ldg(a.wscale) * (1.f / 65536.f), b2 = __ldg(a.fc2_b);
     const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + 64 * half;
     uint32_t phase = 0;
-    bool fail = !tc::mbar_wait(&S.bar_images, 0);
+    bool fail = false;
     float2 v[C / 2];
     float vmax = 0.f;
     auto load_tile = [&](int i) {

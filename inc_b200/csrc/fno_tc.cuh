@@ -32,6 +32,17 @@ constexpr int KM = 16;             // modes of the tables (a network with fewer 
 constexpr int WORKERS = 256;       // 128 points x 2 channel halves
 constexpr int THREADS = WORKERS + 32;
 
+// Loads of states: read once, so they leave the L1 (a few KB beside the tiles) alone
+INC_DEV float ldg_na(const float* p) {
+    float v;
+    asm("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+INC_DEV float4 ldg_na4(const float4* p) {
+    float4 v;
+    asm("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 INC_DEV float4 lds4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 // Barriers: the workers' own; and the hand-overs to the issuing warp, on which the workers
@@ -219,8 +230,8 @@ template <int C, int N>
 INC_DEV void load_channels(const float* __restrict__ base, bool live, float2 (&v)[C / 2]) {
 #pragma unroll
     for (int c = 0; c < C; c += 2) {
-        v[c / 2].x = live ? __ldg(base + c * N) : 0.f;
-        v[c / 2].y = live ? __ldg(base + (c + 1) * N) : 0.f;
+        v[c / 2].x = live ? ldg_na(base + c * N) : 0.f;
+        v[c / 2].y = live ? ldg_na(base + (c + 1) * N) : 0.f;
     }
 }
 
@@ -306,12 +317,12 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     tc::fence_after();
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // ---- the issuing warp
-        const bool ok = tc::mbar_wait(&S.bar_images, 0);  // (the workers turn their outputs to NaN)
-        (void)ok;
+        // (images that did not arrive: nothing is issued, and the workers' waits run out)
+        const bool ok = tc::mbar_wait(&S.bar_images, 0);
         int buf = 0;
         for (int b = b0; b < a.batch; b += step) {
             take_over();
-            if (tid == WORKERS) {
+            if (tid == WORKERS && ok) {
                 tc::fence_after();
                 issue_product<W, W>(d + 2 * W * buf, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 issue_product<W, 32>(d + 2 * W * buf, tc::smem_u32(S.gt), 8192, tc::smem_u32(S.m), true);
@@ -338,7 +349,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     }
     const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + c0;
     uint32_t phase = 0;
-    bool fail = !tc::mbar_wait(&S.bar_images, 0);  // a wait that ran out: the outputs turn to NaN
+    bool fail = false;  // a wait for the tensor cores ran out: the outputs turn to NaN
     float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // a tile on its way in: values (LIFT: u and grid at the point), mixed modes, magnitudes
     float2 v[C / 2];
@@ -437,6 +448,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
         phase ^= 1;
         const float fx = fail ? __int_as_float(0x7fffffff) : f_next;
         const float u0 = s0, u1 = s1;  // (BWD0: this tile's)
+        float2 zp[MODE == BWD ? C / 2 : 1];
         if (b + step < a.batch) {  // the tile's products are done: its buffers take the next one
             f_next = stage_tile();
             tc::fence_smem();
@@ -446,34 +458,29 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
                 load_ends(b + step);
                 point_sums(v, 0);
             }
-            load_tile(b + 2 * step);
         }
+        if constexpr (MODE == BWD) load_channels<C, N>(a.zprev + ((int64_t)b * W + c0) * N + p, on, zp);
+        load_tile(b + 2 * step);
         tc::fence_after();
         float m = 0.f, gu = 0.f;
         float* out = MODE == BWD0 ? nullptr : a.out + ((int64_t)b * W + c0) * N + p;
-        const float* zr = MODE == BWD ? a.zprev + ((int64_t)b * W + c0) * N + p : nullptr;
         float2 h[MODE == BWD0 ? C / 2 : 1];
+        constexpr int CH = MODE == BWD ? 8 : 16;  // columns at a time (BWD holds zprev beside them)
 #pragma unroll
-        for (int i0 = 0; i0 < C; i0 += 16) {
-            float2 zp[8];
-            if constexpr (MODE == BWD) load_channels<16, N>(zr + i0 * N, on, zp);
-            float x0[16], x1[16];
-            tc::tmem_ld16(dl + 2 * W * buf + i0, x0);
-            tc::tmem_ld16(dl + 2 * W * buf + W + i0, x1);
+        for (int i0 = 0; i0 < C; i0 += CH) {
+            float x0[CH], x1[CH];
+            tc::tmem_ld(dl + 2 * W * buf + i0, x0);
+            tc::tmem_ld(dl + 2 * W * buf + W + i0, x1);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-                const float4 bi = lds4(&S.bias[c0 + i0 + i]);
+            for (int i = 0; i < CH; i += 4) {
+                const float4 bi = kBwd ? make_float4(0.f, 0.f, 0.f, 0.f) : lds4(&S.bias[c0 + i0 + i]);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const int e = i + 2 * j, ch = i0 + e;
                     float2 z = __ffma2_rn(__fadd2_rn(make_float2(x0[e], x0[e + 1]), make_float2(x1[e], x1[e + 1])),
                                           make_float2(fx, fx), j == 0 ? make_float2(bi.x, bi.y) : make_float2(bi.z, bi.w));
-                    if constexpr (MODE == BWD) {
-                        float2 y, gp;
-                        act::gelu_both2(zp[e / 2], y, gp);
-                        z = __fmul2_rn(z, gp);
-                    }
+                    if constexpr (MODE == BWD) z = __fmul2_rn(z, act::gelu_grad2(zp[ch / 2]));
                     if constexpr (MODE == FWD) {
                         m = fmaxf(m, fmaxf(z.x, z.y));  // |gelu(z)| <= max(z, 0.17)
                         if (a.store_gelu) z = act::gelu2(z);
@@ -600,12 +607,11 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
     const uint32_t d = S.tmem;
     if (tid >= MODES_WORKERS) {  // the issuing warp
         const bool ok = tc::mbar_wait(&S.bar_images, 0);
-        (void)ok;
         int n = 0;
         for (int i = blockIdx.x; i < tiles; i += gridDim.x)
             for (int ch = 0; ch < CHUNKS; ++ch, ++n) {
                 take_over<MODES_WORKERS>(n & 1);
-                if (tid == MODES_WORKERS) {
+                if (tid == MODES_WORKERS && ok) {
                     tc::fence_after();
                     const uint32_t x = tc::smem_u32(S.a[n & 1]), f = tc::smem_u32(S.ft) + ch * 8 * F_PLANE;
 #pragma unroll 1
@@ -625,7 +631,7 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
         tc::tmem_free(S.tmem, 128);
         return;
     }
-    bool fail = !tc::mbar_wait(&S.bar_images, 0);
+    bool fail = false;
     const int c8 = tid & 7, r0 = tid >> 3;  // this thread's points of a chunk; rows r0 and r0 + 64
     // chunks are loaded two ahead, so that a load has about two chunks' time to arrive
     float4 v[2][2][2];
@@ -638,8 +644,8 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
             w[h][0] = w[h][1] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (n < mine && row < a.rows) {
                 const float4* s = reinterpret_cast<const float4*>(a.x + (int64_t)row * N + ch * 64 + 8 * c8);
-                w[h][0] = __ldg(s);
-                w[h][1] = __ldg(s + 1);
+                w[h][0] = ldg_na4(s);
+                w[h][1] = ldg_na4(s + 1);
             }
         }
     };
@@ -742,18 +748,21 @@ int run_modes(const ModesArgs& a, int n, cudaStream_t st) {
 // ---- mode mixing ---------------------------------------------------------------------
 // out[b][k][r] = (1 / n) sum_j in[k][b][j] S[k][j][r]; S[k][j][r] = W[j][r][k] (forward) or
 // conj(W[r][j][k]) (adjoint), laid out by the preparation.  omax[b] = max |out[b]| (zeroed by
-// the preparation; a max does not depend on the order).  Block: one mode, MIX_B
-// trajectories; thread: four outputs of MIX_R trajectories, so that the weights read from
-// shared memory are used four times (with one trajectory per thread the mixing of 512 x
-// 64 x 16 modes was bound by them: 24 us).
-constexpr int MIX_R = 4;
+// the preparation; a max does not depend on the order).  Block: one mode, MIX_B = 32
+// trajectories; a thread has four outputs of MIX_R trajectories over half of the inputs
+// (the halves are joined by shuffles), real and imaginary factors in separate packed
+// accumulators (two packed operations per complex product).  The first form (all inputs
+// per thread, scalar operations, 64 trajectories) took 11.5 us at 256 x 64 x 16 modes: too few
+// blocks, each a long chain.
 template <int W>
-constexpr int mix_b() { return 256 / (W / 4) * MIX_R; }
+constexpr int mix_r() { return W == 64 ? 4 : 2; }
+constexpr int MIX_B = 32;
 template <int W>
 __global__ void __launch_bounds__(256) k_fno_mix(const float2* __restrict__ in, const float2* __restrict__ wt,
                                                  float2* __restrict__ out, float* __restrict__ omax, int batch,
                                                  int modes, float scale) {
-    constexpr int MIX_B = mix_b<W>(), TPT = W / 4, SUB = 256 / TPT;
+    constexpr int MIX_R = mix_r<W>(), TPT = W / 4, SUB = 128 / TPT;
+    static_assert(SUB * MIX_R == MIX_B, "trajectories per block");
     extern __shared__ __align__(128) unsigned char fno_smem[];
     float4* S = reinterpret_cast<float4*>(fno_smem);               // [W][W / 2] pairs of complex
     float4* X = S + W * W / 2;                                     // [MIX_B][W / 2]
@@ -766,14 +775,16 @@ __global__ void __launch_bounds__(256) k_fno_mix(const float2* __restrict__ in, 
     for (int i = threadIdx.x; i < MIX_B * W / 2; i += 256)
         X[i] = 2 * i < nb * W ? __ldg(xin + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    const int r0 = threadIdx.x % TPT, b = threadIdx.x / TPT;  // trajectories b, b + SUB, ...
-    float2 acc[MIX_R][4];
+    // lanes: outputs, then the half of the inputs, then trajectories
+    const int r0 = threadIdx.x % TPT, jh = threadIdx.x / TPT % 2, b = threadIdx.x / (2 * TPT);
+    float2 re[MIX_R][4], im[MIX_R][4];
 #pragma unroll
     for (int i = 0; i < MIX_R; ++i)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) acc[i][r] = make_float2(0.f, 0.f);
+        for (int r = 0; r < 4; ++r) re[i][r] = im[i][r] = make_float2(0.f, 0.f);
 #pragma unroll 4
-    for (int j = 0; j < W; ++j) {
+    for (int jj = 0; jj < W / 2; ++jj) {
+        const int j = jh * (W / 2) + jj;
         const float4 w0 = S[j * (W / 2) + 2 * r0], w1 = S[j * (W / 2) + 2 * r0 + 1];
         const float2 w[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y),
                              make_float2(w1.z, w1.w)};
@@ -782,27 +793,31 @@ __global__ void __launch_bounds__(256) k_fno_mix(const float2* __restrict__ in, 
             const float2 x = reinterpret_cast<const float2*>(X)[(b + i * SUB) * W + j];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                acc[i][r].x = fmaf(x.x, w[r].x, fmaf(-x.y, w[r].y, acc[i][r].x));
-                acc[i][r].y = fmaf(x.x, w[r].y, fmaf(x.y, w[r].x, acc[i][r].y));
+                re[i][r] = __ffma2_rn(make_float2(x.x, x.x), w[r], re[i][r]);
+                im[i][r] = __ffma2_rn(make_float2(x.y, x.y), w[r], im[i][r]);
             }
         }
     }
 #pragma unroll
     for (int i = 0; i < MIX_R; ++i) {
         float m = 0.f;
+        float2 o[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            acc[i][r].x *= scale;
-            acc[i][r].y *= scale;
-            m = fmaxf(m, fmaxf(fabsf(acc[i][r].x), fabsf(acc[i][r].y)));
+            o[r] = make_float2(re[i][r].x - im[i][r].y, re[i][r].y + im[i][r].x);
+            o[r].x += __shfl_xor_sync(0xffffffffu, o[r].x, TPT);
+            o[r].y += __shfl_xor_sync(0xffffffffu, o[r].y, TPT);
+            o[r].x *= scale;
+            o[r].y *= scale;
+            m = fmaxf(m, fmaxf(fabsf(o[r].x), fabsf(o[r].y)));
         }
 #pragma unroll
-        for (int o = TPT / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        for (int s = TPT / 2; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
         const int bb = b + i * SUB;
-        if (bb < nb) {
-            float4* o = reinterpret_cast<float4*>(out + ((int64_t)(b0 + bb) * modes + k) * W + 4 * r0);
-            o[0] = make_float4(acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y);
-            o[1] = make_float4(acc[i][2].x, acc[i][2].y, acc[i][3].x, acc[i][3].y);
+        if (bb < nb && jh == 0) {
+            float4* dst = reinterpret_cast<float4*>(out + ((int64_t)(b0 + bb) * modes + k) * W + 4 * r0);
+            dst[0] = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+            dst[1] = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
             if (r0 == 0) atomicMax(reinterpret_cast<unsigned int*>(omax) + b0 + bb, __float_as_uint(m));
         }
     }
@@ -811,10 +826,10 @@ __global__ void __launch_bounds__(256) k_fno_mix(const float2* __restrict__ in, 
 template <int W>
 int run_mix(const float2* in, const float2* wt, float2* out, float* omax, int batch, int n, int modes,
             cudaStream_t st) {
-    const size_t smem = (W * W + mix_b<W>() * W) * sizeof(float2);
+    const size_t smem = (W * W + MIX_B * W) * sizeof(float2);
     cudaFuncSetAttribute(k_fno_mix<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fno_mix<W><<<dim3(modes, (batch + mix_b<W>() - 1) / mix_b<W>()), 256, smem, st>>>(in, wt, out, omax, batch, modes,
-                                                                                     1.f / (float)n);
+    k_fno_mix<W><<<dim3(modes, (batch + MIX_B - 1) / MIX_B), 256, smem, st>>>(in, wt, out, omax, batch, modes,
+                                                                           1.f / (float)n);
     return check_launch("fno mix");
 }
 

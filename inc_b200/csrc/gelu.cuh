@@ -42,6 +42,16 @@ INC_DEV float2 gelu2(float2 z) {
     return make_float2(fmaxf(z.x, 0.f) - fabsf(w.x), fmaxf(z.y, 0.f) - fabsf(w.y));
 }
 
+// the derivative of gelu at two values: Phi(z) + z phi(z), phi(z) = exp(-z^2 / 2) / sqrt(2 pi)
+INC_DEV float2 gelu_grad2(float2 z) {
+    const float2 q = gauss_tail2(z);
+    constexpr float k = -0.72134752044448170f, d = 0.39894228040143268f;  // -log2(e) / 2, 1 / sqrt(2 pi)
+    const float2 zk = __fmul2_rn(__fmul2_rn(z, z), make_float2(k, k));
+    const float2 zd = __fmul2_rn(z, make_float2(d, d));
+    return make_float2(fmaf(zd.x, ex2_approx(zk.x), z.x > 0.f ? 1.f - q.x : q.x),
+                       fmaf(zd.y, ex2_approx(zk.y), z.y > 0.f ? 1.f - q.y : q.y));
+}
+
 // gelu and its derivative of two values
 INC_DEV void gelu_both2(float2 z, float2& g, float2& gp) {
     const float2 q = gauss_tail2(z), w = __fmul2_rn(z, q);
