@@ -117,6 +117,9 @@ SIGNATURES = {
                                                _vp, _vp, C.c_int32, _vp, _vp, _vp]),
     "inc_burgers_cnn_rollout_bwd_acts": (C.c_int, [C.POINTER(BurgersDesc), _vp, _vp, _vp, _vp, C.c_double,
                                                    C.c_int32, C.c_int32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "inc_burgers_cnn_rollout_bwd_states_work_size": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32]),
+    "inc_burgers_cnn_rollout_bwd_states": (C.c_int, [C.POINTER(BurgersDesc), _vp, _vp, _vp, _vp, C.c_double, C.c_int32,
+                                                     _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
 }
 INC_NOALLOC_CKPT_FLOATS = 2 * 1024 * 1024
 INC_CNN_WEIGHT_FLOATS = 10657

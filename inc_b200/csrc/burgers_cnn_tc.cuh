@@ -135,6 +135,21 @@ INC_DEV void read_layer16(uint32_t d, int c0, float f, const float* bias, float2
     }
 }
 
+// the same without a bias
+INC_DEV void read_sums16(uint32_t d, int c0, float f, float2 (&z)[8]) {
+    float v0[16], v1[16], v2[16];
+    tc::tmem_ld16(d + c0, v0);
+    tc::tmem_ld16(d + 32 + c0, v1);
+    tc::tmem_ld16(d + 64 + c0, v2);
+    tc::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int e = 2 * i;
+        z[i] = __fmul2_rn(__fadd2_rn(f2(v0[e], v0[e + 1]), __fadd2_rn(f2(v1[e], v1[e + 1]), f2(v2[e], v2[e + 1]))),
+                          f2s(f));
+    }
+}
+
 // max |v| over this thread's channels and its row (a barrier of the CTA inside; fails
 // is or-ed over the CTA)
 template <int N>

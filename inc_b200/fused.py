@@ -110,13 +110,14 @@ class BurgersCNNRolloutFn(torch.autograd.Function):
         w = _pack_params(params, u0.device)
         frames = torch.empty(B, steps, N, device=u0.device, dtype=torch.float32)
         corr = torch.empty_like(frames)
-        nseg = (steps + ckpt_every - 1) // ckpt_every
-        ckpts = torch.empty(B, nseg, N, device=u0.device, dtype=torch.float32)
-        # the hidden layers' pre-activations of every step, kept for the backward when they
-        # fit ACTS_BYTES_MAX (else the backward recomputes them)
+        # the hidden layers' pre-activations and the state of every step, kept for the backward
+        # when they fit ACTS_BYTES_MAX (else the backward replays segments and recomputes them)
         acts = None
         if B * steps * 2 * 32 * N * 4 <= ACTS_BYTES_MAX:
             acts = torch.empty(B, steps, 2, 32, N, device=u0.device, dtype=torch.float32)
+            ckpt_every = 1
+        nseg = (steps + ckpt_every - 1) // ckpt_every
+        ckpts = torch.empty(B, nseg, N, device=u0.device, dtype=torch.float32)
         launch.cnn_rollout(w, u0, steps, frames, corr, None, ckpt_every, ckpts, acts=acts)
         ctx.save_for_backward(ckpts, corr, w, acts)
         ctx.launch, ctx.steps, ctx.ckpt_every, ctx.shape = launch, steps, ckpt_every, (B, N)
@@ -129,11 +130,13 @@ class BurgersCNNRolloutFn(torch.autograd.Function):
         dev = ckpts.device
         g_u0 = torch.empty(B, N, device=dev, dtype=torch.float32)
         g_w = torch.empty(nat.INC_CNN_WEIGHT_FLOATS, device=dev, dtype=torch.float32)
-        work = torch.empty(B, nat.INC_CNN_WEIGHT_FLOATS, device=dev, dtype=torch.float32)
         gf = None if g_frames is None else g_frames.contiguous()
         gc = None if g_corr is None else g_corr.contiguous()
-        ctx.launch.cnn_rollout_bwd(w, ckpts, corr, ctx.steps, ctx.ckpt_every, gf, gc, None, g_u0, g_w, work,
-                                   acts=acts)
+        if acts is not None:
+            ctx.launch.cnn_rollout_bwd_states(w, ckpts, corr, ctx.steps, gf, gc, None, g_u0, g_w, acts)
+        else:
+            work = torch.empty(B, nat.INC_CNN_WEIGHT_FLOATS, device=dev, dtype=torch.float32)
+            ctx.launch.cnn_rollout_bwd(w, ckpts, corr, ctx.steps, ctx.ckpt_every, gf, gc, None, g_u0, g_w, work)
         return (g_u0, None, None, None) + unpack_cnn_grads(g_w)
 
 

@@ -178,6 +178,20 @@ class _BurgersLaunch:
                 rc = lib.inc_burgers_cnn_rollout_bwd_acts(*args, acts.data_ptr(), nat.stream_of(self.dev))
         nat.check(rc, "inc_burgers_cnn_rollout_bwd")
 
+    def cnn_rollout_bwd_states(self, weights, states, corrections, steps, g_frames, g_corrections, g_final, g_u0,
+                               g_weights, acts):
+        """The backward from the forward's record of every step (``states``: cnn_rollout's ckpts
+        with ckpt_every = 1, and ``acts``)."""
+        lib = nat.lib()
+        size = lib.inc_burgers_cnn_rollout_bwd_states_work_size(self.desc.rows, self.desc.n, steps)
+        with nat.on_device(self.dev):
+            work = torch.empty(size, device=self.dev, dtype=torch.float32)
+            rc = lib.inc_burgers_cnn_rollout_bwd_states(
+                C.byref(self.desc), weights.data_ptr(), states.data_ptr(), corrections.data_ptr(),
+                nat.ptr(self.t_rows), self.t0, steps, nat.ptr(g_frames), nat.ptr(g_corrections), nat.ptr(g_final),
+                g_u0.data_ptr(), g_weights.data_ptr(), acts.data_ptr(), work.data_ptr(), nat.stream_of(self.dev))
+        nat.check(rc, "inc_burgers_cnn_rollout_bwd_states")
+
     def rollout_bwd(self, ckpts, s, steps, ckpt_every, g_frames, g_final, g_u0, g_s):
         with nat.on_device(self.dev):
             rc = nat.lib().inc_burgers_rollout_bwd(C.byref(self.desc), ckpts.data_ptr(), nat.ptr(s),

@@ -355,6 +355,18 @@ int inc_energy_spectrum(const float* u, float* out, int32_t rows, int32_t n, voi
 int inc_ks_fft_rows(const float* v, float* out, int32_t rows, int32_t n, int32_t mode,
                     void* stream);
 
+/* The same backward from a record of every step: states [rows][steps][n], the state each
+ * step starts from (what inc_burgers_cnn_rollout_acts writes to ckpts with ckpt_every = 1),
+ * and acts.  Nothing is replayed or recomputed, and the hidden layers' adjoints and
+ * weight gradients run on the tensor cores.  work: ..._work_size floats (-1 for
+ * unsupported sizes).                                                            */
+int64_t inc_burgers_cnn_rollout_bwd_states_work_size(int32_t rows, int32_t n, int32_t steps);
+int inc_burgers_cnn_rollout_bwd_states(const inc_burgers_desc* d, const float* weights, const float* states,
+                                       const float* corrections, const float* t_rows, double t0,
+                                       int32_t steps, const float* g_frames, const float* g_corrections,
+                                       const float* g_final, float* g_u0, float* g_weights,
+                                       const float* acts, float* work, void* stream);
+
 /* ---- corrector: FNO spectral convolution ----------------------------------- */
 /* y[b][o] = irfft(sum_c rfft(x[b][c])[k] * (w_re + i w_im)[c][o][k] for
  * k < modes, zero above), n points, plus bias[o] and addend[b][o][n] where
