@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
     float(*part)[KW][N] = S.o.part;
     const int t = threadIdx.x, rl = t / N, g = t % N;
     const int tile = N < 128 ? rl : t / 128;
-    const bool leader = N < 128 ? g == 0 : t % 128 == 0;
+    const bool issuer = N < 128 ? g < 32 : t % 128 < 32;  // the warp that issues its tile's products
     const int row = blockIdx.x * R + rl;
     const bool valid = row < a.rows;
     if (t < 32) tc::tmem_alloc(&S.tmem, Cfg::COLS);
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
             tc::fence_smem();
             tc::fence_before();
             __syncthreads();
-            if (leader) {
+            if (issuer && tc::elect()) {
                 tc::fence_after();
                 issue_layer<N>(S.tmem + 96 * tile, S.act, S.w[l], tile);
                 tc::commit(&S.bar[tile]);

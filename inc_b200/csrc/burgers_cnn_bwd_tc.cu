@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
     const int t = threadIdx.x, rl = t / N, g = t % N, w = t >> 5, lane = t & 31;
     const int pr = (32 * w) / N, px = (32 * w) % N;  // this warp's 32 cells: row, first cell
     const int tile = N < 128 ? rl : t / 128;
-    const bool leader = N < 128 ? g == 0 : t % 128 == 0;
+    const bool issuer = N < 128 ? g < 32 : t % 128 < 32;  // the warp that issues its tile's products
     const int row = blockIdx.x * R + rl;
     const bool valid = row < a.rows;
     const int src = valid ? row : 0;  // a row past the batch runs row 0 with zero adjoints
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         tc::fence_smem();
         tc::fence_before();
         __syncthreads();
-        if (leader) {
+        if (issuer && tc::elect()) {
             tc::fence_after();
             issue_layer<N>(S.tmem + 96 * tile, S.act, S.w[l], tile);
             tc::commit(&S.bar[tile]);
@@ -456,19 +456,19 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
             const int k0 = gi / places * GROUP, len = min(GROUP, a.steps - k0);
             for (int j = 0; j < len; ++j, ++n) {
                 wg_take_over(n & 1);
-                if (tid == WG) {
+                if (tc::elect()) {
                     tc::fence_after();
-                    const uint32_t x = tc::smem_u32(S.buf[n & 1].dz), y = tc::smem_u32(S.buf[n & 1].a);
+                    const uint64_t x = tc::smem_desc(tc::smem_u32(S.buf[n & 1].dz) + 32, 128, PL);
+                    const uint64_t y = tc::smem_desc(tc::smem_u32(S.buf[n & 1].a), 128, PL);
                     constexpr uint32_t id = tc::instr_desc(128, 96, true, true);
-#pragma unroll 1
+#pragma unroll
                     for (int tap = 0; tap < KW; ++tap)
 #pragma unroll
                         for (int r = 0; r < R; ++r)
-#pragma unroll 4
+#pragma unroll
                             for (int q = 0; q < U; q += 16)
-                                tc::mma(d + 96 * tap, tc::smem_desc(x + (r * (U + 4) + 2 + q) * 16, 128, PL),
-                                        tc::smem_desc(y + (r * (U + 4) + tap + q) * 16, 128, PL), id,
-                                        j > 0 || r > 0 || q > 0);
+                                tc::mma(d + 96 * tap, tc::desc_at(x, (r * (U + 4) + q) * 16),
+                                        tc::desc_at(y, (r * (U + 4) + tap + q) * 16), id, j > 0 || r > 0 || q > 0);
                     tc::commit(&S.bar[n & 1]);
                 }
                 __syncwarp();

@@ -95,7 +95,7 @@ INC_DEV void store_cell(unsigned char* act, const float (&v)[C], float inv, int 
 }
 
 // One layer's products for one tile: 5 taps x 2 channel halves, accumulators at
-// columns d .. d + 95 of the tile's 128 lanes; one thread issues.
+// columns d .. d + 95 of the tile's 128 lanes; one thread issues (tc::elect).
 template <int N>
 INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned char* w, int tile) {
     constexpr int PL = TcCfg<N>::PLANE;
@@ -103,15 +103,16 @@ INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned ch
     const int slot0 = N < 128 ? tile * (N + 4) - tile * 64 : tile * 128;
     const uint32_t a0 = tc::smem_u32(act) + slot0 * 16, b0 = tc::smem_u32(w);
     constexpr uint32_t i96 = tc::instr_desc(128, 96), i64 = tc::instr_desc(128, 64), i32 = tc::instr_desc(128, 32);
-#pragma unroll 1
+    const uint64_t ad = tc::smem_desc(a0, PL, 128), bd = tc::smem_desc(b0, W_PLANE, 128);
+#pragma unroll
     for (int k = 0; k < KW; ++k) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint64_t b = tc::smem_desc(b0 + k * W_TAP + 2 * h * W_PLANE, W_PLANE, 128);
-            const uint32_t a = a0 + k * 16 + 2 * h * PL;
-            tc::mma(d, tc::smem_desc(a, PL, 128), b, i96, k + h > 0);
-            tc::mma(d + 32, tc::smem_desc(a + 4 * PL, PL, 128), b, i64, true);
-            tc::mma(d + 64, tc::smem_desc(a + 8 * PL, PL, 128), b, i32, true);
+            const uint64_t b = tc::desc_at(bd, k * W_TAP + 2 * h * W_PLANE);
+            const uint64_t a = tc::desc_at(ad, k * 16 + 2 * h * PL);
+            tc::mma(d, a, b, i96, k + h > 0);
+            tc::mma(d + 32, tc::desc_at(a, 4 * PL), b, i64, true);
+            tc::mma(d + 64, tc::desc_at(a, 8 * PL), b, i32, true);
         }
     }
 }

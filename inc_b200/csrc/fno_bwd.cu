@@ -77,10 +77,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
     tc::fence_after();
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // the issuing warp: three products per tile
-        const bool ok = tc::mbar_wait(&S.bar_images, 0);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
         for (int i = blockIdx.x; i < tiles; i += step) {
             take_over();
-            if (tid == WORKERS && ok) {  // hidden values: columns 0..127 and 128..255
+            if (ok && tc::elect()) {  // hidden values: columns 0..127 and 128..255
                 tc::fence_after();
                 issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 tc::commit(&S.bar);
@@ -89,18 +89,16 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {  // dL/dx += g1[64 h ..] w1, into columns 0.. and 128.., read by then
                 take_over();
-                if (tid == WORKERS && ok) {
+                if (ok && tc::elect()) {
                     tc::fence_after();
-                    const uint32_t x = tc::smem_u32(S.x), w = tc::smem_u32(S.w) + 64 * h * 16;
+                    const uint64_t x = tc::smem_desc(tc::smem_u32(S.x), 2048, 128);
+                    const uint64_t w = tc::smem_desc(tc::smem_u32(S.w) + 64 * h * 16, 128, 384 * 16);
                     constexpr uint32_t id = tc::instr_desc(128, W, false, true);
-#pragma unroll 1
+#pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const uint64_t a0 = tc::smem_desc(x + 2 * k * 2048, 2048, 128);
-                        const uint64_t a1 = tc::smem_desc(x + (8 + 2 * k) * 2048, 2048, 128);
-                        const uint64_t a2 = tc::smem_desc(x + (16 + 2 * k) * 2048, 2048, 128);
-                        const uint64_t b0 = tc::smem_desc(w + 16 * k * 16, 128, 384 * 16);
-                        const uint64_t b1 = tc::smem_desc(w + (128 + 16 * k) * 16, 128, 384 * 16);
-                        const uint64_t b2 = tc::smem_desc(w + (256 + 16 * k) * 16, 128, 384 * 16);
+                        const uint64_t a0 = tc::desc_at(x, 2 * k * 2048), a1 = tc::desc_at(a0, 8 * 2048);
+                        const uint64_t a2 = tc::desc_at(a0, 16 * 2048), b0 = tc::desc_at(w, 16 * k * 16);
+                        const uint64_t b1 = tc::desc_at(b0, 128 * 16), b2 = tc::desc_at(b0, 256 * 16);
                         tc::mma(d, a0, b0, id, h + k > 0);
                         tc::mma(d + 128, a1, b0, id, h + k > 0);
                         tc::mma(d + 128, a0, b1, id, true);
@@ -309,21 +307,21 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
     if (tid >= WG_WORKERS) {  // the issuing warp
         for (int n = 0; n < mine; ++n) {
             take_over<WG_WORKERS>(n & 1);
-            if (tid == WG_WORKERS) {
+            if (tc::elect()) {
                 tc::fence_after();
-                const uint32_t g = tc::smem_u32(S.buf[n & 1].g), x = tc::smem_u32(S.buf[n & 1].x);
+                const uint64_t g = tc::smem_desc(tc::smem_u32(S.buf[n & 1].g), GP, 128);
+                const uint64_t x = tc::smem_desc(tc::smem_u32(S.buf[n & 1].x), XP, 128);
                 const bool first = n % chunks == 0;
-#pragma unroll 1
+#pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const uint64_t b = tc::smem_desc(x + 2 * k * XP, XP, 128);
-                    const uint32_t gk = g + 2 * k * GP;
+                    const uint64_t b = tc::desc_at(x, 2 * k * XP), gk = tc::desc_at(g, 2 * k * GP);
                     const bool add = !first || k > 0;
-                    tc::mma(d, tc::smem_desc(gk, GP, 128), b, tc::instr_desc(128, 3 * W), add);
+                    tc::mma(d, gk, b, tc::instr_desc(128, 3 * W), add);
                     if (MO == 64) {
-                        tc::mma(d + 2 * W, tc::smem_desc(gk + 128 * 16, GP, 128), b, tc::instr_desc(128, W), true);
+                        tc::mma(d + 2 * W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, W), true);
                     } else if (MO == 128) {
-                        tc::mma(d + W, tc::smem_desc(gk + 128 * 16, GP, 128), b, tc::instr_desc(128, 2 * W), true);
-                        tc::mma(d + 2 * W, tc::smem_desc(gk + 256 * 16, GP, 128), b, tc::instr_desc(128, W), true);
+                        tc::mma(d + W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, 2 * W), true);
+                        tc::mma(d + 2 * W, tc::desc_at(gk, 256 * 16), b, tc::instr_desc(128, W), true);
                     }
                 }
                 tc::commit(&S.bar[n & 1]);

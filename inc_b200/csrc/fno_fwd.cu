@@ -64,10 +64,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
     tc::fence_after();
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // the issuing warp
-        const bool ok = tc::mbar_wait(&S.bar_images, 0);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
         for (int i = blockIdx.x; i < tiles; i += step) {
             take_over();
-            if (tid == WORKERS && ok) {
+            if (ok && tc::elect()) {
                 tc::fence_after();
                 issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 tc::commit(&S.bar);

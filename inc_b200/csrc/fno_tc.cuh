@@ -184,20 +184,17 @@ INC_DEV float point_max(const float2 (&v)[C / 2]) {
 }
 // D[128 x N] at columns d .. d + N - 1 (hi.hi) and d + N .. d + 2N - 1 (the rest) = (or +=,
 // with `add`) A [128 x K] B[N x K]^T.  A: pieces of a point tile (planes of 2048 bytes,
-// pieces a_piece apart); B: stacked pieces [3 N][K].  One thread.
+// pieces a_piece apart); B: stacked pieces [3 N][K].  One thread (tc::elect).
 template <int N, int K>
 INC_DEV void issue_product(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b, bool add) {
     constexpr uint32_t plane_b = 3 * N * 16;
     constexpr uint32_t i2 = tc::instr_desc(128, 2 * N), i1 = tc::instr_desc(128, N);
-#pragma unroll 1
+    const uint64_t ad = tc::smem_desc(a, 2048, 128), bd = tc::smem_desc(b, plane_b, 128);
+#pragma unroll
     for (int k = 0; k < K / 16; ++k) {
-        const uint64_t a0 = tc::smem_desc(a + 2 * k * 2048, 2048, 128);
-        const uint64_t a1 = tc::smem_desc(a + a_piece + 2 * k * 2048, 2048, 128);
-        const uint64_t a2 = tc::smem_desc(a + 2 * a_piece + 2 * k * 2048, 2048, 128);
-        const uint32_t bb = b + 2 * k * plane_b;
-        const uint64_t b0 = tc::smem_desc(bb, plane_b, 128);
-        const uint64_t b1 = tc::smem_desc(bb + N * 16, plane_b, 128);
-        const uint64_t b2 = tc::smem_desc(bb + 2 * N * 16, plane_b, 128);
+        const uint64_t a0 = tc::desc_at(ad, 2 * k * 2048), b0 = tc::desc_at(bd, 2 * k * plane_b);
+        const uint64_t a1 = tc::desc_at(a0, a_piece), a2 = tc::desc_at(a0, 2 * a_piece);
+        const uint64_t b1 = tc::desc_at(b0, N * 16), b2 = tc::desc_at(b0, 2 * N * 16);
         tc::mma(d, a0, b0, i2, add || k > 0);  // hi.hi | hi.mid
         tc::mma(d + N, a1, b0, i1, true);      // mid.hi
         tc::mma(d + N, a0, b2, i1, true);      // hi.lo
@@ -318,11 +315,11 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     const uint32_t d = S.tmem;
     if (tid >= WORKERS) {  // ---- the issuing warp
         // (images that did not arrive: nothing is issued, and the workers' waits run out)
-        const bool ok = tc::mbar_wait(&S.bar_images, 0);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
         int buf = 0;
         for (int b = b0; b < a.batch; b += step) {
             take_over();
-            if (tid == WORKERS && ok) {
+            if (ok && tc::elect()) {
                 tc::fence_after();
                 issue_product<W, W>(d + 2 * W * buf, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
                 issue_product<W, 32>(d + 2 * W * buf, tc::smem_u32(S.gt), 8192, tc::smem_u32(S.m), true);
@@ -606,21 +603,21 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
     tc::fence_after();
     const uint32_t d = S.tmem;
     if (tid >= MODES_WORKERS) {  // the issuing warp
-        const bool ok = tc::mbar_wait(&S.bar_images, 0);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
         int n = 0;
         for (int i = blockIdx.x; i < tiles; i += gridDim.x)
             for (int ch = 0; ch < CHUNKS; ++ch, ++n) {
                 take_over<MODES_WORKERS>(n & 1);
-                if (tid == MODES_WORKERS && ok) {
+                if (ok && tc::elect()) {
                     tc::fence_after();
-                    const uint32_t x = tc::smem_u32(S.a[n & 1]), f = tc::smem_u32(S.ft) + ch * 8 * F_PLANE;
-#pragma unroll 1
+                    const uint64_t x = tc::smem_desc(tc::smem_u32(S.a[n & 1]), A_PITCH, 128);
+                    const uint64_t f = tc::smem_desc(tc::smem_u32(S.ft) + ch * 8 * F_PLANE, F_PLANE, 128);
+#pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const uint64_t bd = tc::smem_desc(f + 2 * k * F_PLANE, F_PLANE, 128);
-                        const uint32_t ak = x + 2 * k * A_PITCH;
-                        tc::mma(d, tc::smem_desc(ak, A_PITCH, 128), bd, tc::instr_desc(128, 96), ch + k > 0);
-                        tc::mma(d + 32, tc::smem_desc(ak + 8 * A_PITCH, A_PITCH, 128), bd, tc::instr_desc(128, 64), true);
-                        tc::mma(d + 64, tc::smem_desc(ak + 16 * A_PITCH, A_PITCH, 128), bd, tc::instr_desc(128, 32), true);
+                        const uint64_t ak = tc::desc_at(x, 2 * k * A_PITCH), bd = tc::desc_at(f, 2 * k * F_PLANE);
+                        tc::mma(d, ak, bd, tc::instr_desc(128, 96), ch + k > 0);
+                        tc::mma(d + 32, tc::desc_at(ak, 8 * A_PITCH), bd, tc::instr_desc(128, 64), true);
+                        tc::mma(d + 64, tc::desc_at(ak, 16 * A_PITCH), bd, tc::instr_desc(128, 32), true);
                     }
                     tc::commit(&S.bar[n & 1]);
                 }
