@@ -257,9 +257,13 @@ int launch_proj_bwd(const ProjBwdArgs& a, int* blocks, cudaStream_t st) {
 //   MO = 32:  lanes (hi, mid, lo) x columns (hi, mid, lo), one product;
 //   MO = 64:  lanes (hi, mid) x (hi, mid, lo), and lo x hi added to the columns of hi x lo;
 //   MO = 128: hi x (hi, mid, lo), mid x (hi, mid), lo x hi.
-// A unit's sums are read into registers (with its two scales) before the next unit's
-// products start over, so no chain in the tensor cores is longer than a row; g is scaled to
-// 128 instead of 256, so that 512 full-scale terms stay below 2^24 (tc.cuh).
+// A unit's sums are read into registers (with its two scales) while the next unit's products
+// run into the other half of the columns, so no chain in the tensor cores is longer than a
+// row; g is scaled to 128 instead of 256, so that 512 full-scale terms stay below 2^24 (tc.cuh).
+// 16 warps split; the last of them also issues (8 or 12 instructions per chunk).  A 17th warp
+// for that cost every thread 32 registers (128 -> 96), and reading the sums before the next
+// unit started left the tensor cores idle: 33 -> 30 us (64 x 64) and 37 -> 35 us (128 x 64) at
+// 256 rows of 512 points.
 struct WgradArgs {
     const float* g;      // [batch][MO][n]
     const float* gmax;   // [tiles per row][batch]
@@ -283,17 +287,17 @@ struct WgradSmem {
 };
 
 template <int MO, int W>
-__global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
+__global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];
     using Smem = WgradSmem<MO, W>;
     Smem& S = *reinterpret_cast<Smem*>(fno_smem);
-    constexpr int GP = Smem::GP, XP = Smem::XP, COLS = W == 64 ? 256 : 128;
+    constexpr int GP = Smem::GP, XP = Smem::XP, COLS = W == 64 ? 256 : 128;  // (of one unit's sums)
     // pieces of 8 points of a row of g (the first MO rows) or x, per thread and chunk; the
     // last round may be half a block
     constexpr int ITEMS = (MO + W) * 8, IT = (ITEMS + WG_WORKERS - 1) / WG_WORKERS;
     const int tid = threadIdx.x;
-    if (tid >= WG_WORKERS) tc::tmem_alloc(&S.tmem, COLS);
-    if (tid == WG_WORKERS) {
+    if (tid < 32) tc::tmem_alloc(&S.tmem, 2 * COLS);
+    if (tid == 0) {
         tc::mbar_init(&S.bar[0], 1);
         tc::mbar_init(&S.bar[1], 1);
         tc::mbar_init_fence();
@@ -304,35 +308,25 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
     const uint32_t d = S.tmem;
     const int per_row = a.n / a.seg, units = a.batch * per_row, chunks = a.seg / 64;
     const int mine = blockIdx.x < units ? (units - blockIdx.x + gridDim.x - 1) / gridDim.x * chunks : 0;
-    if (tid >= WG_WORKERS) {  // the issuing warp
-        for (int n = 0; n < mine; ++n) {
-            take_over<WG_WORKERS>(n & 1);
-            if (tc::elect()) {
-                tc::fence_after();
-                const uint64_t g = tc::smem_desc(tc::smem_u32(S.buf[n & 1].g), GP, 128);
-                const uint64_t x = tc::smem_desc(tc::smem_u32(S.buf[n & 1].x), XP, 128);
-                const bool first = n % chunks == 0;
+    auto issue = [&](int n) {  // chunk n's products (one thread)
+        const uint64_t g = tc::smem_desc(tc::smem_u32(S.buf[n & 1].g), GP, 128);
+        const uint64_t x = tc::smem_desc(tc::smem_u32(S.buf[n & 1].x), XP, 128);
+        const uint32_t du = d + (n / chunks & 1) * COLS;
+        const bool first = n % chunks == 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint64_t b = tc::desc_at(x, 2 * k * XP), gk = tc::desc_at(g, 2 * k * GP);
-                    const bool add = !first || k > 0;
-                    tc::mma(d, gk, b, tc::instr_desc(128, 3 * W), add);
-                    if (MO == 64) {
-                        tc::mma(d + 2 * W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, W), true);
-                    } else if (MO == 128) {
-                        tc::mma(d + W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, 2 * W), true);
-                        tc::mma(d + 2 * W, tc::desc_at(gk, 256 * 16), b, tc::instr_desc(128, W), true);
-                    }
-                }
-                tc::commit(&S.bar[n & 1]);
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t b = tc::desc_at(x, 2 * k * XP), gk = tc::desc_at(g, 2 * k * GP);
+            const bool add = !first || k > 0;
+            tc::mma(du, gk, b, tc::instr_desc(128, 3 * W), add);
+            if (MO == 64) {
+                tc::mma(du + 2 * W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, W), true);
+            } else if (MO == 128) {
+                tc::mma(du + W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, 2 * W), true);
+                tc::mma(du + 2 * W, tc::desc_at(gk, 256 * 16), b, tc::instr_desc(128, W), true);
             }
-            __syncwarp();
         }
-        tc::fence_before();
-        __syncthreads();
-        tc::tmem_free(S.tmem, COLS);
-        return;
-    }
+        tc::commit(&S.bar[n & 1]);
+    };
     const int c8 = tid & 7, r0 = tid >> 3;
     bool fail = false;
     uint32_t used = 0;
@@ -364,7 +358,23 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
     };
     float sg = 1.f, sx = 1.f;
     const int nq = a.n < 128 ? 1 : a.n / 128;
+    // the sums of the unit that ended with chunk n (in buffer `buf`)
+    auto drain = [&](int n, int buf, float f) {
+        if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
+        tc::fence_after();
+        if (fail) f = __int_as_float(0x7fffffff);
+        const uint32_t dl = d + (n / chunks & 1) * COLS + ((uint32_t)(t & 96) << 16) + quarter * CQ;
+        float q0[CQ], q1[CQ], q2[CQ];
+        tc::tmem_ld(dl, q0);
+        tc::tmem_ld(dl + W, q1);
+        tc::tmem_ld(dl + 2 * W, q2);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < CQ; ++i)
+            acc[i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
+    };
     auto chunk = [&](int n, int buf, float4(&w)[IT][2]) {
+        const float f_prev = sg * (1.f / 128.f) * (sx * (1.f / 256.f));
         if (n % chunks == 0) {  // the unit's scales: the max over its tiles
             const int u = blockIdx.x + n / chunks * gridDim.x, b = u / per_row;
             const int q0 = a.n < 128 ? 0 : (u % per_row) * a.seg / 128, q1 = a.seg < 128 ? q0 + 1 : q0 + a.seg / 128;
@@ -404,29 +414,21 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
                 *reinterpret_cast<uint4*>(s + 2 * piece) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
+        load(n + DEPTH, w);
         tc::fence_smem();
         tc::fence_before();
-        hand_over<WG_WORKERS>(buf);
-        load(n + DEPTH, w);
-        if (n % chunks != chunks - 1) return;
-        // the unit's sums: every chunk's products done (the last of either buffer)
-        if (chunks > 1) {
-            if (!fail) fail = !tc::mbar_wait(&S.bar[buf ^ 1], (used >> (buf ^ 1)) & 1);
+        if (tid < WG_WORKERS - 32) {
+            hand_over<WG_WORKERS - 32>(buf);
+        } else {
+            take_over<WG_WORKERS - 32>(buf);
+            if (tc::elect()) {
+                tc::fence_after();
+                issue(n);
+            }
+            __syncwarp();
         }
-        if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
-        tc::fence_after();
-        const float f = fail ? __int_as_float(0x7fffffff) : sg * (1.f / 128.f) * (sx * (1.f / 256.f));
-        const uint32_t dl = d + ((uint32_t)(t & 96) << 16) + quarter * CQ;
-        float q0[CQ], q1[CQ], q2[CQ];
-        tc::tmem_ld(dl, q0);
-        tc::tmem_ld(dl + W, q1);
-        tc::tmem_ld(dl + 2 * W, q2);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < CQ; ++i)
-            acc[i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
-        tc::fence_before();
-        worker_sync<WG_WORKERS>();  // read everywhere before the next unit's products
+        // the unit before this one, while this one's products run into the other columns
+        if (n > 0 && n % chunks == 0) drain(n - 1, buf ^ 1, f_prev);
     };
     load(0, v[0]);
     if (DEPTH == 2) load(1, v[DEPTH - 1]);
@@ -435,6 +437,8 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
         chunk(n, 0, v[0]);
         if (n + 1 < mine) chunk(n + 1, 1, v[DEPTH - 1]);
     }
+    if (mine > 0) drain(mine - 1, (mine - 1) & 1, sg * (1.f / 128.f) * (sx * (1.f / 256.f)));
+    tc::fence_before();
     // the lanes' pieces added up (hi, then mid and lo), then the block's slot
     float* s = reinterpret_cast<float*>(S.buf[0].g);  // [128][W + 1]; every product is done
     static_assert(sizeof(float) * 128 * (W + 1) <= sizeof(S.buf), "scratch");
@@ -457,8 +461,7 @@ __global__ void __launch_bounds__(WG_WORKERS + 32, 1) k_fno_wgrad(WgradArgs a) {
         rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], 4);
         if (c8 == 0 && r0 + 64 * i < MO) a.rows[(int64_t)blockIdx.x * MO + r0 + 64 * i] = rs[i];
     }
-    tc::fence_before();
-    __syncthreads();
+    if (tid < 32) tc::tmem_free(d, 2 * COLS);
 }
 
 // a unit: 128 points while that leaves a block few units, else as many as a row has (fewer
@@ -476,7 +479,7 @@ int run_wgrad(WgradArgs a, int* blocks, cudaStream_t st) {
     a.seg = wgrad_seg(a.batch, a.n);
     const int64_t units = (int64_t)a.batch * (a.n / a.seg);
     *blocks = units < sm_count() ? (int)units : sm_count();
-    k_fno_wgrad<MO, W><<<*blocks, WG_WORKERS + 32, smem, st>>>(a);
+    k_fno_wgrad<MO, W><<<*blocks, WG_WORKERS, smem, st>>>(a);
     return check_launch("fno weight gradient");
 }
 
