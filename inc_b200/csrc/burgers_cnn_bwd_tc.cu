@@ -381,8 +381,14 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
 // co), columns (tap, piece of a, ci); the useful six of the nine piece pairs are added in
 // registers.  dz is scaled to 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
 // Even blocks take layer 2 (a = gelu(z1), z1 from the recorded state), odd ones layer 3.
-// 16 warps prepare the two operand tiles (two buffers), a 17th issues.  Bound by the
-// products: 80 of M = 128, N = 96 per unit, 56 cycles each.
+// The bias gradient is one more block of columns (a = 1).  16 warps prepare the two operand
+// tiles (two buffers), a 17th issues.  Bound by the preparation (about 5,500 clocks a unit: two
+// loads' latency, the split, GELU and the stores) and the reading of a group's sums, which
+// the products of the group wait for; the products take 80 x 56 clocks.  709 us for 256 rows x
+// 256 cells x 32 steps in its first form; 629 with an elected issuer (tc::elect); 440 with
+// the sums read without branches and the bias gradient out of the registers; 432 with the
+// next unit's lines fetched to the L2.  Not faster: 8 warps with the next values held in
+// registers (432), 16 with them (478, spills), the sums kept in memory (707).
 constexpr int WG = 512;
 constexpr int GROUP = 4;
 struct CnnWgradArgs {
@@ -404,7 +410,7 @@ template <int N>
 struct CnnWgradSmem {
     struct Buf {
         alignas(128) unsigned char dz[3 * 4 * WgCfg<N>::PLANE];
-        alignas(128) unsigned char a[3 * 4 * WgCfg<N>::PLANE];
+        alignas(128) unsigned char a[(3 * 4 + 2) * WgCfg<N>::PLANE];  // two planes of ones follow the pieces
     } buf[2];  // (dz's lanes past 96 read on into a: not used)
     alignas(16) float w1[KW][C], b1[C];
     uint64_t bar[2];
@@ -429,6 +435,10 @@ INC_DEV void store_half(unsigned char* tile, int plane, const float2 (&v)[8], fl
     }
 }
 
+// accumulator columns of a tap's 96; the middle tap's are followed by 16 times dz summed (a = 1)
+__host__ __device__ constexpr int tap_col(int k) { return 96 * k + (k > KW / 2 ? 16 : 0); }
+constexpr int ONES = tap_col(KW / 2) + 96;
+
 template <int N>
 __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
     using Cfg = WgCfg<N>;
@@ -445,6 +455,12 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
     }
     for (int i = tid; i < KW * C; i += WG + 32) S.w1[i / C][i % C] = __ldg(a.w + OFF_W1 + (i % C) * KW + i / C);
     if (tid < C) S.b1[tid] = __ldg(a.w + OFF_B1 + tid);
+    for (int i = tid; i < 2 * PL / 16; i += WG + 32)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            *reinterpret_cast<uint4*>(S.buf[q].a + 12 * PL + i * 16) =
+                make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+    tc::fence_smem();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -460,15 +476,16 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
                     tc::fence_after();
                     const uint64_t x = tc::smem_desc(tc::smem_u32(S.buf[n & 1].dz) + 32, 128, PL);
                     const uint64_t y = tc::smem_desc(tc::smem_u32(S.buf[n & 1].a), 128, PL);
-                    constexpr uint32_t id = tc::instr_desc(128, 96, true, true);
+                    constexpr uint32_t i96 = tc::instr_desc(128, 96, true, true), i112 = tc::instr_desc(128, 112, true, true);
 #pragma unroll
                     for (int tap = 0; tap < KW; ++tap)
 #pragma unroll
                         for (int r = 0; r < R; ++r)
 #pragma unroll
                             for (int q = 0; q < U; q += 16)
-                                tc::mma(d + 96 * tap, tc::desc_at(x, (r * (U + 4) + q) * 16),
-                                        tc::desc_at(y, (r * (U + 4) + tap + q) * 16), id, j > 0 || r > 0 || q > 0);
+                                tc::mma(d + tap_col(tap), tc::desc_at(x, (r * (U + 4) + q) * 16),
+                                        tc::desc_at(y, (r * (U + 4) + tap + q) * 16), tap == KW / 2 ? i112 : i96,
+                                        j > 0 || r > 0 || q > 0);
                     tc::commit(&S.bar[n & 1]);
                 }
                 __syncwarp();
@@ -483,16 +500,14 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
     const int slot = rl * (U + 4) + x + 2;
     const int halo = H > 1 ? 0 : (x < 2 ? U : (x >= U - 2 ? -U : 0));  // the copy a row's ends own
     const int lane_q = (tid >> 5) & 3, colq = tid >> 7;  // accumulator lanes' piece; 8 of the 32 input channels
-    float acc[KW][8], gb[16];
+    float acc[KW][8], gb = 0.f;
 #pragma unroll
     for (int k = 0; k < KW; ++k)
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[k][i] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) gb[i] = 0.f;
     bool fail = false;
     uint32_t used = 0;
-    float f_done = 0.f;  // scales of the group whose sums are still in tensor memory (0: none)
+    float f_done = 0.f, fb_done = 0.f;  // scales of the group whose sums are still in tensor memory (0: none)
     // the layer's input (half of the channels) at cell xa of a row and step
     auto input = [&](int row, int k, int xa, float2(&v)[8]) {
         if (layer == 1) {
@@ -514,24 +529,42 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
             }
         }
     };
+    // the lines of unit (gi, j), or of the next group's first, on their way to the L2: a 128-byte
+    // line per thread (the first half dz's, the second the input's)
+    auto prefetch = [&](int gi, int j) {
+        if (j == min(GROUP, a.steps - gi / places * GROUP)) {
+            gi += blocks;
+            j = 0;
+        }
+        if (gi >= groups || (tid >= 256 && layer == 0)) return;
+        constexpr int LINES = U / 32;  // of a row's cells in a channel
+        const int e = tid & 255, line = e % LINES, ch = e / LINES % C, r = e / (LINES * C);
+        const int place = gi % places, row = place / H * R + r, k = gi / places * GROUP + j;
+        if (row >= a.rows) return;
+        const float* p = tid < 256 ? acts_tile(const_cast<float*>(a.dz), row, a.steps, k, layer, ch, N)
+                                   : acts_tile(const_cast<float*>(a.acts), row, a.steps, k, 0, ch, N);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + place % H * U + line * 32));
+    };
     auto drain = [&](int last) {  // the finished group's sums; `last`: the buffer of its last unit
         if (!fail) fail = !tc::mbar_wait(&S.bar[last], (used >> last) & 1);
         tc::fence_after();
+        // (every lane reads the same columns: loads under a branch cost a few hundred clocks each)
         const float f = fail ? __int_as_float(0x7fffffff) : f_done;
+        const float f1 = lane_q < 2 ? f : 0.f, f2 = lane_q < 1 ? f : 0.f;
         const uint32_t dl = d + ((uint32_t)(tid & 96) << 16) + 8 * colq;
-        if (lane_q < 3) {
+        float ones[8];
+        tc::tmem_ld8(d + ((uint32_t)(tid & 96) << 16) + ONES, ones);
 #pragma unroll
-            for (int k = 0; k < KW; ++k) {
-                float q0[8], q1[8], q2[8];
-                tc::tmem_ld8(dl + 96 * k, q0);
-                if (lane_q < 2) tc::tmem_ld8(dl + 96 * k + 32, q1);
-                if (lane_q < 1) tc::tmem_ld8(dl + 96 * k + 64, q2);
-                tc::tmem_ld_wait();
+        for (int k = 0; k < KW; ++k) {
+            float q0[8], q1[8], q2[8];
+            tc::tmem_ld8(dl + tap_col(k), q0);
+            tc::tmem_ld8(dl + tap_col(k) + 32, q1);
+            tc::tmem_ld8(dl + tap_col(k) + 64, q2);
+            tc::tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    acc[k][i] += (lane_q == 0 ? q0[i] + (q1[i] + q2[i]) : (lane_q == 1 ? q0[i] + q1[i] : q0[i])) * f;
-            }
+            for (int i = 0; i < 8; ++i) acc[k][i] += fmaf(q0[i], f, fmaf(q1[i], f1, q2[i] * f2));
         }
+        gb += ones[0] * (fail ? f : fb_done);
         tc::fence_before();
         wg_sync();  // read everywhere before the next group's products
     };
@@ -557,6 +590,7 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
                 if (!fail) fail = !tc::mbar_wait(&S.bar[buf], (used >> buf) & 1);
                 used ^= 1u << buf;
             }
+            prefetch(gi, j + 1);
             float2 v[8];
             {
                 const float* p = acts_tile(const_cast<float*>(a.dz), valid ? row : 0, a.steps, k, layer, 16 * half, N) + x0;
@@ -564,8 +598,6 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
                 for (int i = 0; i < 8; ++i) {
                     v[i].x = valid ? __ldg(p + 2 * i * N) : 0.f;
                     v[i].y = valid ? __ldg(p + (2 * i + 1) * N) : 0.f;
-                    gb[2 * i] += v[i].x;
-                    gb[2 * i + 1] += v[i].y;
                 }
             }
             store_half(S.buf[buf].dz, PL, v, 64.f / sd, slot, half);
@@ -587,7 +619,8 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
             if (j == 0 && f_done != 0.f) drain(buf ^ 1);
             wg_hand_over(buf);
         }
-        f_done = sd * (1.f / 64.f) * (sa * (1.f / 256.f));
+        fb_done = sd * (1.f / 64.f);
+        f_done = fb_done * (sa * (1.f / 256.f));
     }
     if (f_done != 0.f) drain((n - 1) & 1);
     // the pieces of a lane's co added up, in the packed order [ci][co][k]
@@ -599,14 +632,8 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) s[(lane_q * 32 + (tid & 31)) * 161 + (8 * colq + i) * KW + k] = acc[k][i];
     }
-    // bias gradients: sums over the block's cells, 16 warps x 16 channels
-    float* sb = s + 3 * 32 * 161;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) gb[i] += __shfl_xor_sync(0xffffffffu, gb[i], o);
-        if ((tid & 31) == 0) sb[(tid >> 5) * 16 + i] = gb[i];
-    }
+    float* sb = s + 3 * 32 * 161;  // bias gradients, [3][32]
+    if (lane_q < 3 && colq == 0) sb[lane_q * 32 + (tid & 31)] = gb;
     wg_sync();
     float* out = a.part + ((int64_t)layer * blocks + me) * HID;
     for (int i = tid; i < C * C * KW; i += WG) {
@@ -614,12 +641,7 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
         const float* p = s + co * 161 + ci * KW + k;
         out[i] = p[0] + (p[32 * 161] + p[64 * 161]);
     }
-    if (tid < C) {
-        float r = 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) r += sb[(tid / 16 * 8 + q) * 16 + tid % 16];
-        out[C * C * KW + tid] = r;
-    }
+    if (tid < C) out[C * C * KW + tid] = sb[tid] + (sb[32 + tid] + sb[64 + tid]);
     tc::fence_before();
     __syncthreads();
 }
