@@ -267,11 +267,11 @@ int launch_proj_bwd(const ProjBwdArgs& a, int* blocks, cudaStream_t st) {
 struct WgradArgs {
     const float* g;      // [batch][MO][n]
     const float* gmax;   // [tiles per row][batch]
-    const float* x;      // [batch][W][n], through GELU with in_gelu
+    const float* x;      // [batch][W][n], through GELU for the layers (MO = W)
     const float* xmax;   // [tiles per row][batch]
     float* part;         // [blocks][MO][W]
     float* rows;         // [blocks][MO]
-    int batch, n, seg, in_gelu;
+    int batch, n, seg;
 };
 constexpr int WG_WORKERS = 512;
 template <int MO, int W>
@@ -328,6 +328,7 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         tc::commit(&S.bar[n & 1]);
     };
     const int c8 = tid & 7, r0 = tid >> 3;
+    constexpr bool full = (MO + W) % 64 == 0;
     bool fail = false;
     uint32_t used = 0;
     // lane, quarter of the columns, piece of the lane
@@ -348,9 +349,9 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
 #pragma unroll
         for (int i = 0; i < IT; ++i) {
             const int r = r0 + 64 * i;
-            if (r < MO + W) {
+            if (full || r < MO + W) {
                 const float4* s = reinterpret_cast<const float4*>(
-                    r < MO ? a.g + ((int64_t)b * MO + r) * a.n + p : a.x + ((int64_t)b * W + r - MO) * a.n + p);
+                    (MO % 64 == 0 ? 64 * i < MO : r < MO) ? a.g + ((int64_t)b * MO + r) * a.n + p : a.x + ((int64_t)b * W + r - MO) * a.n + p);
                 w[i][0] = ldg_na4(s);
                 w[i][1] = ldg_na4(s + 1);
             }
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         tc::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < CQ; ++i)
-            acc[i] += (group == 0 ? q0[i] + (q1[i] + q2[i]) : (group == 1 ? q0[i] + q1[i] : q0[i])) * f;
+            acc[i] += (q0[i] + ((group < 2 ? q1[i] : 0.f) + (group < 1 ? q2[i] : 0.f))) * f;
     };
     auto chunk = [&](int n, int buf, float4(&w)[IT][2]) {
         const float f_prev = sg * (1.f / 128.f) * (sx * (1.f / 256.f));
@@ -392,14 +393,14 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         }
 #pragma unroll
         for (int i = 0; i < IT; ++i) {
-            const int r = r0 + 64 * i;  // (a warp's rows are all of g or all of x)
-            if (r < MO + W) {
-                const bool is_g = r < MO;
+            const int r = r0 + 64 * i;  // (a warp's rows are all of g or all of x: known here where MO is 64 or 128)
+            if (full || r < MO + W) {
+                const bool is_g = MO % 64 == 0 ? 64 * i < MO : r < MO;
                 float2 e[4] = {make_float2(w[i][0].x, w[i][0].y), make_float2(w[i][0].z, w[i][0].w),
                                make_float2(w[i][1].x, w[i][1].y), make_float2(w[i][1].z, w[i][1].w)};
                 if (is_g) {
                     rs[i] += ((e[0].x + e[0].y) + (e[1].x + e[1].y)) + ((e[2].x + e[2].y) + (e[3].x + e[3].y));
-                } else if (a.in_gelu) {
+                } else if (MO == W) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) e[j] = act::gelu2(e[j]);
                 }
@@ -693,8 +694,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
         job(work + o.sums + 128, gr->fc2_b, 132, blocks, 1);
         float* part = work + o.part;
         float* rows = work + o.rows;
-        rc = run_wgrad<128, W>(WgradArgs{work + o.g1, work + o.g1max, z + 3 * state, tmax + 3 * nq * B, part, rows, B, n, 0,
-                                         0}, &blocks, st);
+        rc = run_wgrad<128, W>(WgradArgs{work + o.g1, work + o.g1max, z + 3 * state, tmax + 3 * nq * B, part, rows, B, n, 0}, &blocks, st);
         if (rc) return rc;
         job(part, gr->fc1_w, 128 * W, blocks, 128 * W);
         job(rows, gr->fc1_b, 128, blocks, 128);
@@ -702,7 +702,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
     for (int l = 3; l >= 0; --l) {
         const float* g = gz + (l & 1) * state;
         const float* gmx = gzmax + (l & 1) * nq * B;
-        rc = run_modes<W>(ModesArgs{g, gmx, prep->transform, gm + l * modes, B * W, B, M, 0}, n, st);
+        rc = run_modes<W, false>(ModesArgs{g, gmx, prep->transform, gm + l * modes, B * W, B, M}, n, st);
         if (rc) return rc;
         rc = run_mix<W>(gm + l * modes, wt + (int64_t)l * M * W * W, mixed, work + o.mmax + l * B, B, n, M, st);
         if (rc) return rc;
@@ -710,7 +710,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
             float* part = work + o.part + most * (128 * W + (l - 1) * W * W);
             float* rows = work + o.rows + most * (128 + (l - 1) * W);
             rc = run_wgrad<W, W>(WgradArgs{g, gmx, z + (l - 1) * state, tmax + (int64_t)(l - 1) * nq * B, part, rows, B, n,
-                                           0, 1}, &blocks, st);
+                                           0}, &blocks, st);
             if (rc) return rc;
             job(part, gr->w[l], W * W, blocks, W * W);
             job(rows, gr->b[l], W, blocks, W);
@@ -729,7 +729,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
             a.zprev = z + (l - 1) * state;
             a.out = gz + ((l - 1) & 1) * state;
             a.tmax = gzmax + ((l - 1) & 1) * nq * B;
-            rc = run_layer<W, false, BWD>(a, n, st);
+            rc = run_layer<W, false, BWD, true>(a, n, st);
         } else {
             a.u = u;
             a.grid = d->grid;
@@ -738,7 +738,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
             a.fc0_b = d->fc0_b;
             a.g_u = gr->u;
             a.sums = work + o.six + 6 * W;
-            rc = run_layer<W, false, BWD0>(a, n, st);
+            rc = run_layer<W, false, BWD0, true>(a, n, st);
         }
         if (rc) return rc;
     }

@@ -154,6 +154,12 @@ int64_t work_floats(int64_t B, int64_t n, int64_t M, bool train) {
            (train ? 0 : 2 * B * W * n + 4 * nq * B);
 }
 
+template <int W, bool TRAIN>
+int forward_layer(const LayerArgs& a, int l, int n, cudaStream_t st) {
+    return l == 0 ? run_layer<W, true, FWD, TRAIN>(a, n, st)
+                  : (l < 3 ? run_layer<W, false, FWD, TRAIN>(a, n, st) : run_layer<W, false, LAST, TRAIN>(a, n, st));
+}
+
 template <int W>
 int run_forward(const inc_fno_desc* d, const float* u, float* y, float* z, float* xm, float* tmax, float* work,
                 cudaStream_t st) {
@@ -192,8 +198,8 @@ int run_forward(const inc_fno_desc* d, const float* u, float* y, float* z, float
         const float* x = l == 0 ? u : (z ? z + (l - 1) * state : h + ((l - 1) & 1) * state);
         float2* im = xm ? reinterpret_cast<float2*>(xm) + l * modes : part;  // the input's modes
         if (l > 0) {
-            const ModesArgs ma{x, tmax + (int64_t)(l - 1) * nq * B, prep->transform, im, B * W, B, M, z != nullptr};
-            rc = run_modes<W>(ma, n, st);
+            const ModesArgs ma{x, tmax + (int64_t)(l - 1) * nq * B, prep->transform, im, B * W, B, M};
+            rc = z ? run_modes<W, true>(ma, n, st) : run_modes<W, false>(ma, n, st);
             if (rc) break;
         }
         rc = run_mix<W>(im, wt + (int64_t)l * M * W * W, mixed, mmax + l * B, B, n, M, st);
@@ -213,12 +219,9 @@ int run_forward(const inc_fno_desc* d, const float* u, float* y, float* z, float
         a.fc0_b = d->fc0_b;
         a.batch = B;
         a.modes = M;
-        a.in_gelu = z != nullptr;
-        a.store_gelu = z == nullptr;
         a.x = x;
         a.out = z ? z + l * state : h + (l & 1) * state;
-        rc = l == 0 ? run_layer<W, true, FWD>(a, n, st)
-                    : (l < 3 ? run_layer<W, false, FWD>(a, n, st) : run_layer<W, false, LAST>(a, n, st));
+        rc = z ? forward_layer<W, true>(a, l, n, st) : forward_layer<W, false>(a, l, n, st);
     }
     if (rc) return rc;
     const ProjArgs p{z ? z + 3 * state : h + state, tmax + 3 * nq * B, prep->fc1, prep->scale + 4, d->fc1_b, d->fc2_w,

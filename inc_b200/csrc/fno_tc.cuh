@@ -235,12 +235,14 @@ INC_DEV void load_channels(const float* __restrict__ base, bool live, float2 (&v
 // One FNO layer on the point tiles (forward and input adjoint):
 //   z[o][p] = sum_c w[o][c] x[c][p] + sum_k (table)[p][k] mixed[k][o] + bias[o].
 // MODE:
-//   FWD     z stored, or gelu(z) with store_gelu;
+//   FWD     z stored, or gelu(z) in an evaluation;
 //   LAST    z stored (the last layer: no GELU follows);
 //   BWD     z gelu'(zprev) stored (x = dL/dz of this layer, w transposed, zprev the layer
 //           below's z);
 //   BWD0    the first layer's adjoint: nothing stored but g_u and the sums below.
-// LIFT: x[c] is the lift of (u, grid); else it is read, through GELU with in_gelu.
+// LIFT: x[c] is the lift of (u, grid); else it is read, in training's forward through GELU
+// (its record holds the sums before it).  TRAIN is a parameter of the template: a test of it
+// among the elements keeps their arithmetic from overlapping.
 // The two products share one scale (the larger of theirs), so they accumulate together.
 enum { FWD, LAST, BWD, BWD0 };
 
@@ -263,7 +265,7 @@ struct LayerArgs {
     float* g_u;             // BWD0: [batch][N]
     float* sums;            // BWD0: [blocks][6][W]
     int64_t grid_stride;
-    int batch, modes, in_gelu, store_gelu;
+    int batch, modes;
 };
 
 template <int W>
@@ -281,11 +283,11 @@ struct LayerSmem {
     uint32_t tmem;
 };
 
-template <int W, int N, bool LIFT, int MODE>
+template <int W, int N, bool LIFT, int MODE, bool TRAIN>
 __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];
     LayerSmem<W>& S = *reinterpret_cast<LayerSmem<W>*>(fno_smem);
-    constexpr bool kBwd = MODE >= BWD;
+    constexpr bool kBwd = MODE >= BWD, kInGelu = TRAIN && !LIFT && !kBwd, kStoreGelu = !TRAIN && MODE == FWD;
     constexpr int points = N < 128 ? N : 128, nq = N / points, C = W / 2;
     constexpr int COLS = 4 * W;  // two tiles' accumulators
     const int tid = threadIdx.x, half = (tid >> 7) & 1, t = tid & 127, c0 = half * C;
@@ -390,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
                 v[c / 2 + 1] = __ffma2_rn(make_float2(w0.z, w0.w), u2,
                                           __ffma2_rn(make_float2(w1.z, w1.w), x2, make_float2(bb.z, bb.w)));
             }
-        } else if (a.in_gelu) {
+        } else if constexpr (kInGelu) {
 #pragma unroll
             for (int i = 0; i < C / 2; ++i) v[i] = act::gelu2(v[i]);
         }
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
                     if constexpr (MODE == BWD) z = __fmul2_rn(z, act::gelu_grad2(zp[ch / 2]));
                     if constexpr (MODE == FWD) {
                         m = fmaxf(m, fmaxf(z.x, z.y));  // |gelu(z)| <= max(z, 0.17)
-                        if (a.store_gelu) z = act::gelu2(z);
+                        if constexpr (kStoreGelu) z = act::gelu2(z);
                     } else {
                         m = fmaxf(m, fmaxf(fabsf(z.x), fabsf(z.y)));
                     }
@@ -541,21 +543,21 @@ inline int tile_grid(int batch, int nq) {
     return want < most ? want : (most > 0 ? most : nq);
 }
 
-template <int W, int N, bool LIFT, int MODE>
+template <int W, int N, bool LIFT, int MODE, bool TRAIN>
 int launch_layer(const LayerArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(LayerSmem<W>);
     static_assert(sizeof(LayerSmem<W>) <= 113 * 1024, "two CTAs per SM");
-    cudaFuncSetAttribute(k_fno_layer<W, N, LIFT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fno_layer<W, N, LIFT, MODE><<<tile_grid(a.batch, N < 128 ? 1 : N / 128), THREADS, smem, st>>>(a);
+    cudaFuncSetAttribute(k_fno_layer<W, N, LIFT, MODE, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_fno_layer<W, N, LIFT, MODE, TRAIN><<<tile_grid(a.batch, N < 128 ? 1 : N / 128), THREADS, smem, st>>>(a);
     return check_launch("fno layer");
 }
-template <int W, bool LIFT, int MODE>
+template <int W, bool LIFT, int MODE, bool TRAIN>
 int run_layer(const LayerArgs& a, int n, cudaStream_t st) {
     switch (n) {
-        case 64: return launch_layer<W, 64, LIFT, MODE>(a, st);
-        case 128: return launch_layer<W, 128, LIFT, MODE>(a, st);
-        case 256: return launch_layer<W, 256, LIFT, MODE>(a, st);
-        default: return launch_layer<W, 512, LIFT, MODE>(a, st);
+        case 64: return launch_layer<W, 64, LIFT, MODE, TRAIN>(a, st);
+        case 128: return launch_layer<W, 128, LIFT, MODE, TRAIN>(a, st);
+        case 256: return launch_layer<W, 256, LIFT, MODE, TRAIN>(a, st);
+        default: return launch_layer<W, 512, LIFT, MODE, TRAIN>(a, st);
     }
 }
 
@@ -570,11 +572,11 @@ int run_layer(const LayerArgs& a, int n, cudaStream_t st) {
 constexpr int MODES_WORKERS = 512;
 constexpr int A_PITCH = 2048 + 16;
 struct ModesArgs {
-    const float* x;      // [rows][N], through GELU with in_gelu
+    const float* x;      // [rows][N], with GELU through it
     const float* xmax;   // [tiles per row][batch]
     const unsigned char* table;
     float2* part;        // [modes][batch][W] = [modes][rows]
-    int rows, batch, modes, in_gelu;
+    int rows, batch, modes;
 };
 struct ModesSmem {
     alignas(128) unsigned char ft[64 * F_PLANE];
@@ -583,7 +585,7 @@ struct ModesSmem {
     uint32_t tmem;
 };
 
-template <int W, int N>
+template <int W, int N, bool GELU>
 __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];
     ModesSmem& S = *reinterpret_cast<ModesSmem*>(fno_smem);
@@ -673,7 +675,7 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
             uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                if (a.in_gelu) e[j] = act::gelu2(e[j]);
+                if constexpr (GELU) e[j] = act::gelu2(e[j]);
                 tc::split2(e[j], make_float2(inv[h], inv[h]), hi[j], mid[j], lo[j]);
             }
             unsigned char* s = S.a[buf] + c8 * A_PITCH + (r0 + 64 * h) * 16;
@@ -724,21 +726,21 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
     __syncthreads();
 }
 
-template <int W, int N>
+template <int W, int N, bool GELU>
 int launch_modes(const ModesArgs& a, cudaStream_t st) {
-    cudaFuncSetAttribute(k_fno_modes<W, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ModesSmem));
+    cudaFuncSetAttribute(k_fno_modes<W, N, GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ModesSmem));
     static_assert(sizeof(ModesSmem) <= 227 * 1024, "shared memory");
     const int tiles = (a.rows + 127) / 128, sms = sm_count();
-    k_fno_modes<W, N><<<tiles < sms ? tiles : sms, MODES_WORKERS + 32, sizeof(ModesSmem), st>>>(a);
+    k_fno_modes<W, N, GELU><<<tiles < sms ? tiles : sms, MODES_WORKERS + 32, sizeof(ModesSmem), st>>>(a);
     return check_launch("fno modes");
 }
-template <int W>
+template <int W, bool GELU>
 int run_modes(const ModesArgs& a, int n, cudaStream_t st) {
     switch (n) {
-        case 64: return launch_modes<W, 64>(a, st);
-        case 128: return launch_modes<W, 128>(a, st);
-        case 256: return launch_modes<W, 256>(a, st);
-        default: return launch_modes<W, 512>(a, st);
+        case 64: return launch_modes<W, 64, GELU>(a, st);
+        case 128: return launch_modes<W, 128, GELU>(a, st);
+        case 256: return launch_modes<W, 256, GELU>(a, st);
+        default: return launch_modes<W, 512, GELU>(a, st);
     }
 }
 
