@@ -248,6 +248,7 @@ def _channel_linear(lin: nn.Linear, x):
 
 
 FNO_N = (64, 128, 256, 512)
+FNO_ROWS = 32 * 65535
 _FNO_LAYERS = ("conv0", "conv1", "conv2", "conv3"), ("w0", "w1", "w2", "w3")
 
 
@@ -282,8 +283,8 @@ class FNOFn(torch.autograd.Function):
             xm = u.new_empty(4, M, B, W, 2)
             tmax = u.new_empty(4, max(1, n // 128), B)
         lib = nat.lib()
-        work = u.new_empty(lib.inc_fno_work_size(C.byref(d), int(record)))
         with nat.on_device(u.device):
+            work = u.new_empty(lib.inc_fno_work_size(C.byref(d), int(record)))
             rc = lib.inc_fno_forward(C.byref(d), u.data_ptr(), y.data_ptr(), nat.ptr(z), nat.ptr(xm), nat.ptr(tmax),
                                      work.data_ptr(), nat.stream_of(u.device))
         nat.check(rc, "inc_fno_forward")
@@ -294,7 +295,7 @@ class FNOFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         u, grid, z, xm, tmax, *params = ctx.saved_tensors
-        gy = gy.contiguous()
+        gy = gy.resolve_neg().contiguous()
         d = FNOFn._desc(u, grid, params)
         need = ctx.needs_input_grad
         gu = torch.empty_like(u) if need[0] else None
@@ -306,8 +307,8 @@ class FNOFn(torch.autograd.Function):
             g.modes_w[i], g.w[i], g.b[i] = (grads[j].data_ptr() for j in (2 + i, 6 + 2 * i, 7 + 2 * i))
         g.fc1_w, g.fc1_b, g.fc2_w, g.fc2_b = (t.data_ptr() for t in grads[14:])
         lib = nat.lib()
-        work = u.new_empty(lib.inc_fno_backward_work_size(C.byref(d)))
         with nat.on_device(u.device):
+            work = u.new_empty(lib.inc_fno_backward_work_size(C.byref(d)))
             rc = lib.inc_fno_backward(C.byref(d), u.data_ptr(), gy.data_ptr(), z.data_ptr(), xm.data_ptr(),
                                       tmax.data_ptr(), C.byref(g), work.data_ptr(), nat.stream_of(u.device))
         nat.check(rc, "inc_fno_backward")
@@ -354,11 +355,13 @@ class FNO1D(nn.Module):
         return out + [self.fc1.weight, self.fc1.bias, self.fc2.weight, self.fc2.bias]
 
     def _fused(self, x, L) -> bool:
-        """True when FNOFn computes this call: FP32 CUDA states of 64..512 cells, width 32 or
-        64 and at most 16 modes, the plain layers (nothing hooked, replaced or reshaped), no
+        """True when FNOFn computes this call: FP32 CUDA states of 64..512 cells (as many rows as
+        one launch's blocks of 32 reach), width 32 or 64 and at most 16 modes, the plain
+        layers (nothing hooked, replaced or reshaped, no pending conjugation or sign), no
         autocast, no gradient to L."""
         if not (isinstance(x, torch.Tensor) and x.is_cuda and x.dtype == torch.float32 and x.dim() == 2
-                and x.shape[0] > 0 and x.shape[1] in FNO_N and self.width in (32, 64) and 1 <= self.modes1 <= 16):
+                and 0 < x.shape[0] <= FNO_ROWS and x.shape[1] in FNO_N and not x.is_neg()
+                and self.width in (32, 64) and 1 <= self.modes1 <= 16):
             return False
         if torch.is_autocast_enabled("cuda") or (isinstance(L, torch.Tensor) and (L.requires_grad or not L.is_cuda)):
             return False
@@ -374,7 +377,7 @@ class FNO1D(nn.Module):
         shapes = [(W, 2), (W,)] + [(W, W, M)] * 4 + [(W, W, 1), (W,)] * 4 + [(128, W), (128,), (1, 128), (1,)]
         for i, (p, shape) in enumerate(zip(self._layer_params(), shapes)):
             if (not isinstance(p, torch.Tensor) or tuple(p.shape) != shape or p.device != x.device
-                    or p.dtype != (torch.complex64 if 2 <= i < 6 else torch.float32)):
+                    or p.dtype != (torch.complex64 if 2 <= i < 6 else torch.float32) or p.is_conj() or p.is_neg()):
                 return False
         return True
 

@@ -68,8 +68,9 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
         S.w2[i] = __ldg(a.fc2_w + i);
     }
     if (tid < 32) {
-        const float4 e = __ldg(reinterpret_cast<const float4*>(a.fc2_w) + tid);
-        const float m = warp_max(fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))));
+        float m = 0.f;
+        for (int i = tid; i < 128; i += 32) m = fmaxf(m, fabsf(__ldg(a.fc2_w + i)));
+        m = warp_max(m);
         if (tid == 0) S.w2max = m;
     }
     tc::fence_before();
@@ -774,7 +775,7 @@ extern "C" int inc_fno_backward(const inc_fno_desc* d, const float* u, const flo
     const int rc = fno::check_fno(d);
     if (rc) return rc;
     bool ok = u && g_y && z && x_modes && tmax && g && work && (reinterpret_cast<uintptr_t>(work) & 15u) == 0 &&
-              (reinterpret_cast<uintptr_t>(z) & 15u) == 0 && (reinterpret_cast<uintptr_t>(d->fc2_w) & 15u) == 0 &&
+              (reinterpret_cast<uintptr_t>(z) & 15u) == 0 &&
               g->fc0_w && g->fc0_b && g->fc1_w && g->fc1_b && g->fc2_w && g->fc2_b;
     for (int l = 0; ok && l < 4; ++l)
         ok = g->modes_w[l] && g->w[l] && g->b[l] && (reinterpret_cast<uintptr_t>(g->modes_w[l]) & 7u) == 0;

@@ -183,8 +183,8 @@ class _BurgersLaunch:
         """The backward from the forward's record of every step (``states``: cnn_rollout's ckpts
         with ckpt_every = 1, and ``acts``)."""
         lib = nat.lib()
-        size = lib.inc_burgers_cnn_rollout_bwd_states_work_size(self.desc.rows, self.desc.n, steps)
         with nat.on_device(self.dev):
+            size = lib.inc_burgers_cnn_rollout_bwd_states_work_size(self.desc.rows, self.desc.n, steps)
             work = torch.empty(size, device=self.dev, dtype=torch.float32)
             rc = lib.inc_burgers_cnn_rollout_bwd_states(
                 C.byref(self.desc), weights.data_ptr(), states.data_ptr(), corrections.data_ptr(),

@@ -358,8 +358,8 @@ int inc_ks_fft_rows(const float* v, float* out, int32_t rows, int32_t n, int32_t
 /* The same backward from a record of every step: states [rows][steps][n], the state each
  * step starts from (what inc_burgers_cnn_rollout_acts writes to ckpts with ckpt_every = 1),
  * and acts.  Nothing is replayed or recomputed, and the hidden layers' adjoints and
- * weight gradients run on the tensor cores.  work: ..._work_size floats (-1 for
- * unsupported sizes).                                                            */
+ * weight gradients run on the tensor cores.  work: ..._work_size floats for the
+ * current device (-1 for unsupported sizes).                                     */
 int64_t inc_burgers_cnn_rollout_bwd_states_work_size(int32_t rows, int32_t n, int32_t steps);
 int inc_burgers_cnn_rollout_bwd_states(const inc_burgers_desc* d, const float* weights, const float* states,
                                        const float* corrections, const float* t_rows, double t0,
@@ -438,8 +438,8 @@ int inc_fno_forward(const inc_fno_desc* d, const float* u, float* y, float* z, f
 
 /* Its backward: the gradients of every parameter (torch's layouts; complex ones in
  * torch's convention) and, when u is not NULL, of u, from g_y [rows][n] and what the
- * forward recorded.  work: inc_fno_backward_work_size floats; z, work and fc2_w
- * 16-byte aligned.                                                              */
+ * forward recorded.  work: inc_fno_backward_work_size floats (for the current
+ * device); z and work 16-byte aligned.                                          */
 typedef struct inc_fno_grads {
     float* u;
     float* fc0_w;

@@ -105,3 +105,34 @@ def test_fno_partial_gradients_and_permuted_input(cuda):
     assert uc.grad is not None
     for (name, p), g in zip(net.named_parameters(), full):
         assert (p.grad is None) if name != "w2.weight" else torch.equal(p.grad, g), name
+
+
+@pytest.mark.parametrize("offset", [1, 3])
+def test_fno_parameters_at_odd_offsets(cuda, offset):
+    """Parameters that are views into one buffer, 4-byte aligned only: the same bits."""
+    torch.manual_seed(offset)
+    net = FNO1D(L=16.0, modes=8, width=32).to(cuda)
+    u = torch.randn(5, 64, device=cuda)
+
+    def grads():
+        net.zero_grad()
+        y = net(u)
+        y.square().sum().backward()
+        return [y.detach()] + [p.grad.clone() for p in net.parameters()]
+
+    want = grads()
+    with torch.no_grad():
+        for p in net.parameters():
+            if not p.is_complex():
+                buf = torch.empty(p.numel() + offset, device=cuda)
+                buf[offset:].copy_(p.reshape(-1))
+                p.data = buf[offset:].view(p.shape)
+    assert net._fused(u, 16.0) and net.fc2.weight.data_ptr() % 16 != 0
+    for a, b in zip(grads(), want):
+        assert torch.equal(a, b)
+
+
+def test_fno_pending_conjugation_is_not_read_raw(cuda):
+    net = FNO1D(L=16.0, modes=8, width=32).to(cuda)
+    net.conv1.weights1 = torch.nn.Parameter(net.conv1.weights1.detach().conj())
+    assert net.conv1.weights1.is_conj() and not net._fused(torch.randn(2, 64, device=cuda), 16.0)
