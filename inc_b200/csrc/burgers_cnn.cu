@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
     float(*part)[KW][N] = S.o.part;
     const int t = threadIdx.x, rl = t / N, g = t % N;
     const int tile = N < 128 ? rl : t / 128;
-    const bool issuer = N < 128 ? g < 32 : t % 128 < 32;  // the warp that issues its tile's products
+    const bool issuer = t / 32 == T / 32 - (N < 128 ? 2 : 4);  // the warp that issues, one of the last tile's
     const int row = blockIdx.x * R + rl;
     const bool valid = row < a.rows;
     if (t < 32) tc::tmem_alloc(&S.tmem, Cfg::COLS);
@@ -128,10 +128,13 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
             tc::fence_smem();
             tc::fence_before();
             __syncthreads();
-            if (issuer && tc::elect()) {
+            if (issuer && tc::elect()) {  // tile by tile: the first's sums are read while the last's products run
                 tc::fence_after();
-                issue_layer<N>(S.tmem + 96 * tile, S.act, S.w[l], tile);
-                tc::commit(&S.bar[tile]);
+#pragma unroll
+                for (int q = 0; q < Cfg::TILES; ++q) {
+                    issue_layer<N>(S.tmem + 96 * q, S.act, S.w[l], q);
+                    tc::commit(&S.bar[q]);
+                }
             }
             fail = !tc::mbar_wait(&S.bar[tile], phase);
             phase ^= 1;
