@@ -283,8 +283,14 @@ struct LayerSmem {
     uint32_t tmem;
 };
 
+// Who issues: in the forward a ninth warp; in the adjoint the last of the eight, which leaves a
+// thread 128 registers in place of 96 and with them room to load zprev a tile ahead (256 x 64 x
+// 512: 33.2 -> 29.6 us, the first layer's 30.1 -> 24.8; the forward with the lift 18.0 -> 20.3 that
+// way, the others equal).
+constexpr int layer_threads(int mode) { return mode >= BWD ? WORKERS : THREADS; }
+
 template <int W, int N, bool LIFT, int MODE, bool TRAIN>
-__global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
+__global__ void __launch_bounds__(layer_threads(MODE), 2) k_fno_layer(LayerArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];
     LayerSmem<W>& S = *reinterpret_cast<LayerSmem<W>*>(fno_smem);
     constexpr bool kBwd = MODE >= BWD, kInGelu = TRAIN && !LIFT && !kBwd, kStoreGelu = !TRAIN && MODE == FWD;
@@ -294,8 +300,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     const int q = blockIdx.x % nq, p = q * points + t;
     const int step = gridDim.x / nq;  // CTAs per row position
     const int b0 = blockIdx.x / nq;
-    if (tid >= WORKERS) tc::tmem_alloc(&S.tmem, COLS);
-    if (tid == WORKERS) {
+    if (tid < 32) tc::tmem_alloc(&S.tmem, COLS);
+    if (tid == 0) {
         tc::mbar_init(&S.bar_images, 1);
         tc::mbar_init(&S.bar_layer, 1);
         tc::mbar_init_fence();
@@ -303,7 +309,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
         tc::bulk_load(S.w, a.w, sizeof(S.w), &S.bar_images);
         tc::bulk_load(S.gt, a.inverse + (int64_t)q * G_BYTES, G_BYTES, &S.bar_images);
     }
-    for (int i = tid; i < W; i += THREADS) {
+    for (int i = tid; i < W; i += layer_threads(MODE)) {
         S.bias[i] = kBwd ? 0.f : __ldg(a.bias + i);
         if (LIFT || MODE == BWD0) {
             S.lift[0][i] = __ldg(a.fc0_w + 2 * i);
@@ -315,26 +321,40 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     __syncthreads();
     tc::fence_after();
     const uint32_t d = S.tmem;
-    if (tid >= WORKERS) {  // ---- the issuing warp
+    auto products = [&](int buf) {  // one thread
+        tc::fence_after();
+        issue_product<W, W>(d + 2 * W * buf, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
+        issue_product<W, 32>(d + 2 * W * buf, tc::smem_u32(S.gt), 8192, tc::smem_u32(S.m), true);
+        tc::commit(&S.bar_layer);
+    };
+    if (!kBwd && tid >= WORKERS) {  // ---- the issuing warp
         // (images that did not arrive: nothing is issued, and the workers' waits run out)
         const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
         int buf = 0;
         for (int b = b0; b < a.batch; b += step) {
             take_over();
-            if (ok && tc::elect()) {
-                tc::fence_after();
-                issue_product<W, W>(d + 2 * W * buf, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
-                issue_product<W, 32>(d + 2 * W * buf, tc::smem_u32(S.gt), 8192, tc::smem_u32(S.m), true);
-                tc::commit(&S.bar_layer);
-            }
+            if (ok && tc::elect()) products(buf);
             __syncwarp();
             buf ^= 1;
         }
         tc::fence_before();
         __syncthreads();
-        tc::tmem_free(S.tmem, COLS);
         return;
     }
+    bool ok = true, waited = false;
+    auto issue = [&](int buf) {  // the staged tile is ready
+        if constexpr (!kBwd) {
+            hand_over();
+        } else if (tid < WORKERS - 32) {
+            hand_over<WORKERS - 32>();
+        } else {
+            if (!waited) ok = __all_sync(0xffffffffu, tc::mbar_wait(&S.bar_images, 0));
+            waited = true;
+            take_over<WORKERS - 32>();
+            if (ok && tc::elect()) products(buf);
+            __syncwarp();
+        }
+    };
     // ---- the workers
     const bool on = points == 128 || t < points;  // (rows of 64 cells use half of a tile)
     const float ws = __ldg(a.wscale);
@@ -435,7 +455,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     load_tile(b0);
     float f_next = stage_tile();
     tc::fence_smem();
-    hand_over();
+    issue(0);
     if constexpr (MODE == BWD0) {
         load_ends(b0);
         point_sums(v, 0);
@@ -443,22 +463,22 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     load_tile(b0 + step);
     int buf = 0;
     for (int b = b0; b < a.batch; b += step) {
+        float2 zp[MODE == BWD ? C / 2 : 1];
+        if constexpr (MODE == BWD) load_channels<C, N>(a.zprev + ((int64_t)b * W + c0) * N + p, on, zp);
         if (!fail) fail = !tc::mbar_wait(&S.bar_layer, phase);
         phase ^= 1;
         const float fx = fail ? __int_as_float(0x7fffffff) : f_next;
         const float u0 = s0, u1 = s1;  // (BWD0: this tile's)
-        float2 zp[MODE == BWD ? C / 2 : 1];
         if (b + step < a.batch) {  // the tile's products are done: its buffers take the next one
             f_next = stage_tile();
             tc::fence_smem();
             tc::fence_before();
-            hand_over();
+            issue(buf ^ 1);
             if constexpr (MODE == BWD0) {
                 load_ends(b + step);
                 point_sums(v, 0);
             }
         }
-        if constexpr (MODE == BWD) load_channels<C, N>(a.zprev + ((int64_t)b * W + c0) * N + p, on, zp);
         load_tile(b + 2 * step);
         tc::fence_after();
         float m = 0.f, gu = 0.f;
@@ -535,6 +555,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_layer(LayerArgs a) {
     }
     tc::fence_before();
     __syncthreads();
+    if (tid < 32) tc::tmem_free(d, COLS);
 }
 
 // CTAs of a tile kernel: at most two per SM, a multiple of the row positions
@@ -548,7 +569,7 @@ int launch_layer(const LayerArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(LayerSmem<W>);
     static_assert(sizeof(LayerSmem<W>) <= 113 * 1024, "two CTAs per SM");
     cudaFuncSetAttribute(k_fno_layer<W, N, LIFT, MODE, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_fno_layer<W, N, LIFT, MODE, TRAIN><<<tile_grid(a.batch, N < 128 ? 1 : N / 128), THREADS, smem, st>>>(a);
+    k_fno_layer<W, N, LIFT, MODE, TRAIN><<<tile_grid(a.batch, N < 128 ? 1 : N / 128), layer_threads(MODE), smem, st>>>(a);
     return check_launch("fno layer");
 }
 template <int W, bool LIFT, int MODE, bool TRAIN>
