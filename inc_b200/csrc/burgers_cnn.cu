@@ -14,13 +14,15 @@
 // tensor cores (burgers_cnn_tc.cuh), with three-piece operands whose rounding is below
 // that of an FP32 multiply-add chain (tc.cuh).  A thread turns its cell's 32
 // activations into pieces with one power-of-two scale per row (the row's max |a|, one
-// warp reduction and one barrier), a thread per 128 cells issues the products, and each
+// warp reduction and one barrier), one thread issues the products tile by tile, and each
 // thread reads its cell's 32 sums back from tensor memory.
 //
-// What bounds a step: the FP32 and integer work around the products (96 GELUs, the
-// splits and the first and last layers, about 2,900 instructions per cell) with the
-// products themselves (2 x 1,490 cycles per 128 cells) beside it; two CTAs per SM
-// overlap the two.
+// What bounds a step: a chain.  With two rows of 256 cells on an SM a step takes about
+// 27,000 clocks: 2 x 5,500 from issuing a layer's products to their end (1,490 per tile,
+// four tiles in turn), 2 x 2,200 in the split and its stores, 2 x 2,500 in reading and
+// GELU, 2,500 in the first layer and 4,000 in the solver's step.  256 x 256 x 32 steps:
+// 426 us, against 1,154 with all four layers on the FP32 pipes.  Issuing a layer's
+// products in two channel halves, the first beside the second's split, measured 429.
 #include "burgers_cnn_tc.cuh"
 
 namespace inc {

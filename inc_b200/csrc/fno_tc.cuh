@@ -14,9 +14,15 @@
 // tensor-memory lane.  The split's scale is the tile's max, recorded by the launch that
 // wrote the state.  A CTA keeps one position of the row and walks over the trajectories;
 // its table and weights, prepared as shared-memory images by one launch per call, arrive
-// by bulk copies and stay.  8 warps do the arithmetic and a ninth only issues products,
-// so nobody waits behind the tensor cores' queue; the products of the next tile run
-// while this one's results are read, and two CTAs share an SM.
+// by bulk copies and stay.  8 warps do the arithmetic (in the forward a ninth only issues
+// products, see layer_threads); the products of the next tile run while this one's results
+// are read, and two CTAs share an SM.
+//
+// What bounds a layer: the loads' latency at the start of a launch (4,000 to 12,000 clocks
+// until the first tile and the images are there), then the splits and GELUs beside the
+// loads.  512 x 64 x 512: 43.5 us for 134 MB read and written (20.8 us at the copy rate); a
+// batched FP32 matmul, a spectral convolution and a GELU pass took about 150.  Programmatic launch
+// overlap, an L2 prefetch of later tiles and 16 warps a CTA measured no faster.
 //
 // The modes of a state are a launch of their own (k_fno_modes) with the points as the
 // contraction: taking them in the layer's epilogue instead (a second split and product per
@@ -588,8 +594,9 @@ int run_layer(const LayerArgs& a, int n, cudaStream_t st) {
 // contraction, 64 per chunk, and the table's 96 stacked rows the columns.  A thread
 // splits 8 consecutive points of a row at a time (float4 loads, 256 contiguous bytes per
 // 8 lanes); the planes' pitch of 2064 bytes makes their 16-byte stores conflict-free.
-// 16 warps split (and apply GELU), a 17th issues.  Bound by reading the state (67 MB at 512 x
-// 64 x 512: 10.4 us at the copy rate) and the split.
+// 16 warps split (and apply GELU), a 17th issues.  Bound by reading the state and the split:
+// 12.4 us at 256 x 64 x 512 (33.5 MB, 5.2 us at the copy rate; 128 tiles leave 20 SMs idle),
+// 13.9 with GELU, 21.7 at 512 x 64 x 512 (256 tiles on 148 SMs: a second round on 108).
 constexpr int MODES_WORKERS = 512;
 constexpr int A_PITCH = 2048 + 16;
 struct ModesArgs {

@@ -5,11 +5,15 @@
 u = solver.step(u); results[:, k] = u``) for a ``PeriodicCNN1D`` corrector in
 one launch of ``inc_burgers_cnn_rollout``: the four convolutions run from
 shared memory before every step, so no per-step corrector launches remain.
-With gradients on (rows of 64, 128, 256 or 512 cells), the rollout is one autograd node
-whose backward is ``inc_burgers_cnn_rollout_bwd``: segment replay from
-checkpoints, the network's activations recomputed in shared memory, the
-solver's adjoint and the network's backward in one kernel, weight gradients
-summed over rows in a fixed order.  ``simulate_rollout`` dispatches here by
+With gradients on (rows of 64, 128, 256 or 512 cells), the rollout is one autograd node.
+While the hidden layers' pre-activations of every step fit ``ACTS_BYTES_MAX``, the
+forward records them and every state, and the backward is
+``inc_burgers_cnn_rollout_bwd_states``: the solver's and the network's adjoint in
+reverse, then the weight gradients over all cells and steps, on the tensor cores,
+with no replay.  Longer records are not kept, and the backward is
+``inc_burgers_cnn_rollout_bwd``: segment replay from checkpoints, the activations
+recomputed in shared memory, everything in one kernel.  Weight gradients are summed in
+a fixed order either way.  ``simulate_rollout`` dispatches here by
 itself when the model and solver qualify (``cnn_supported`` /
 ``cnn_train_supported``); otherwise it keeps the per-step loop.
 """
@@ -65,7 +69,9 @@ def pack_cnn_weights(model, device=None) -> torch.Tensor:
 CNN_TRAIN_N = CNN_N
 MAX_CKPT_EVERY = 32
 # Largest record of the hidden layers' pre-activations the training path keeps (bytes):
-# 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps.
+# 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps; the backward
+# takes as much again while it runs.  That training step is 1.85 ms with the record, 3.76 with
+# the replay (4.47 when the replay's forward ran on the FP32 pipes).
 ACTS_BYTES_MAX = 4 << 30
 
 
@@ -152,8 +158,9 @@ def burgers_cnn_rollout(model, solver, u0, steps, corrections=True, ckpt_every=8
     as ``simulate_rollout(model, solver, u0, steps, "INC")`` computes them.
 
     With gradients enabled (and u0 or the model's parameters requiring them) the
-    result is differentiable through the fused backward, which replays
-    ckpt_every-step segments (n = 64, 128, 256 or 512).  Advances ``solver.t`` by steps * dt and
+    result is differentiable through the fused backward (n = 64, 128, 256 or 512), which
+    replays ckpt_every-step segments where the record of every step is not kept
+    (``ACTS_BYTES_MAX``).  Advances ``solver.t`` by steps * dt and
     leaves the last correction in ``solver.correction_s``, like the per-step loop."""
     if not cnn_supported(model, solver, u0):
         raise ValueError("burgers_cnn_rollout: needs a PeriodicCNN1D(32, 5, 4) corrector, a fixed-dt "
