@@ -60,7 +60,7 @@ INC_DEV void cell_products(float (&acc)[KW], const float* dr, const float* ar, i
     }
 }
 
-constexpr int EDGE = 2 * C * KW + C + 1;  // dW1, dW4, db1, db4 of one block
+constexpr int EDGE = 2 * C * KW + C + 2;  // dW1, dW4, db1, db4 (high and low part) of one block
 constexpr int HID = C * C * KW + C;       // one hidden layer's dW and db
 
 struct AdjArgs {
@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
     make_ctx<1, N>(a, src, g, true, cx);
     cx.has_s = true;
     int parity = 0;
-    float g1[KW], g4[KW], gb1 = 0.f, gb4 = 0.f;  // this warp's cells, lane = channel
+    float g1[KW], g4[KW], gb1 = 0.f;  // this warp's cells, lane = channel
+    double gb4 = 0.0;  // this cell's share of db4: one scalar, whose terms cancel
 #pragma unroll
     for (int k = 0; k < KW; ++k) g1[k] = g4[k] = 0.f;
     float gu = (a.g_final && valid) ? __ldg(a.g_final + (int64_t)row * N + g) : 0.f;
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         if (c.g_corr && valid) gs += __ldg(c.g_corr + at);
         put_row(S.u[rl], u);
         put_row(S.d[rl], gs);
+        gb4 += gs;
         __syncthreads();  // (also: the solver's rows are free)
         // ---- layer 4: gelu(z3) by channel for dW4; dz3 = (W4^T s_bar) gelu'(z3)
         {
@@ -215,7 +217,6 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         }
         __syncthreads();
         cell_products(g4, S.d[pr], S.o.ch[pr][lane], px);
-        gb4 += cell_sum(S.d[pr], px);
         // ---- layer 3: dz3 out, dz2 = (W3^T dz3) gelu'(z2)
         float z2[C];
         {
@@ -353,7 +354,10 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
             p[KW + k] = g4[k];
         }
         p[2 * KW] = gb1;
-        p[2 * KW + 1] = gb4;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
+        const float high = (float)gb4;
+        p[2 * KW + 1] = lane == 0 ? high : (float)(gb4 - high);  // (lane 1: the rest)
     }
     tc::fence_before();
     __syncthreads();
@@ -371,7 +375,12 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
             e[C * KW + lane * KW + k] = s[KW + k];
         }
         e[2 * C * KW + lane] = s[2 * KW];
-        if (lane == 0) e[2 * C * KW + C] = s[2 * KW + 1];
+        double b4 = 0.0;
+        for (int q = 0; q < T / 32; ++q) b4 += (double)S.sums[q][0][2 * KW + 1] + S.sums[q][1][2 * KW + 1];
+        if (lane == 0) {
+            e[2 * C * KW + C] = fail ? nan : (float)b4;
+            e[2 * C * KW + C + 1] = (float)(b4 - (float)b4);
+        }
         tc::tmem_free(S.tmem, Cfg::COLS);
     }
 }
@@ -648,10 +657,10 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
     __syncthreads();
 }
 
-// g[i] in the packed order from the blocks' partial sums: 32 outputs x 32 slices per block
+// g[i] in the packed order from the blocks' partial sums, in FP64: 32 outputs x 32 slices per block
 __global__ void __launch_bounds__(1024) k_cnn_grad_sum(const float* __restrict__ edge, int edges,
                                                        const float* __restrict__ hid, int hids, float* __restrict__ g) {
-    __shared__ float s[32][33];
+    __shared__ double s[32][33];
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     const float* src = nullptr;
     int count = 0;
@@ -663,16 +672,18 @@ __global__ void __launch_bounds__(1024) k_cnn_grad_sum(const float* __restrict__
     else if (i < OFF_B4) { src = edge + C * KW + i - OFF_W4; count = edges; }
     else if (i == OFF_B4) { src = edge + 2 * C * KW + C; count = edges; }
     stride = (i >= OFF_W2 && i < OFF_W4) ? HID : EDGE;
-    float v = 0.f;
+    double v = 0.0;
 #pragma unroll 4
     for (int p = slice; p < count; p += 32) v += __ldg(src + p * stride);
+    if (i == OFF_B4)
+        for (int p = slice; p < count; p += 32) v += __ldg(src + 1 + p * stride);
     s[slice][lane] = v;
     __syncthreads();
     if (threadIdx.x < 32 && i < W_FLOATS) {
-        float t[4] = {0.f, 0.f, 0.f, 0.f};
+        double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
         for (int q = 0; q < 32; ++q) t[q & 3] += s[q][lane];
-        g[i] = (t[0] + t[1]) + (t[2] + t[3]);
+        g[i] = (float)((t[0] + t[1]) + (t[2] + t[3]));
     }
 }
 

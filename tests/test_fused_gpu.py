@@ -373,3 +373,33 @@ def test_fused_cnn_rows_of_different_magnitude(cuda, N):
     for r in (0, 1, 3, 4, 5):
         assert rel_l2(corr[r], ref_c[r]) < TOL, r
         assert rel_l2(frames[r], ref_f[r]) < TOL, r
+
+
+@pytest.mark.parametrize("B,N,steps", [(35, 128, 27), (10, 512, 5), (9, 64, 12), (3, 256, 6)])
+def test_fused_training_last_bias_gradient(cuda, B, N, steps):
+    """The last layer's bias gradient is one sum over every row, step and cell whose terms
+    cancel: it is formed in FP64, so it is as far off as the terms themselves, a few FP32
+    roundings (2^-24) of their root sum of squares, not of every partial sum.  Compared
+    with the sum, in FP64, of the corrections' gradients that the per-step loop's autograd gives."""
+    from inc_b200.correctors import PeriodicCNN1D
+    from inc_b200.fused import burgers_cnn_rollout
+    from inc_b200.solvers import BurgersSolverTorch
+    torch.manual_seed(B + N)
+    net = PeriodicCNN1D().to(cuda)
+    u0 = torch.as_tensor(_u0(B, N, 3), dtype=torch.float32, device=cuda)
+    w = torch.randn(B, steps, N, device=cuda) / N
+    sp = _sim_params(_params(N), B, "ssprk3", cuda)
+    frames, _ = burgers_cnn_rollout(net, BurgersSolverTorch(sp), u0, steps)
+    (frames * w).sum().backward()
+    got = net.convs[3].bias.grad.double().item()
+    s, u, loss, terms = BurgersSolverTorch(sp), u0, 0.0, []
+    for k in range(steps):
+        c = net(u)
+        c.retain_grad()
+        terms.append(c)
+        s.correction_s = c
+        u = s.step(u)
+        loss = loss + (u * w[:, k]).sum()
+    loss.backward()
+    g = torch.stack([c.grad for c in terms]).double()
+    assert abs(got - g.sum().item()) < 64 * 2.0 ** -24 * g.square().sum().sqrt().item() * steps ** 0.5
