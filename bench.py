@@ -877,9 +877,9 @@ def bench_diff(args, dev, world, which):
     extra["error"].update(forward_steps=extra["checks"]["forward_steps"], rows=extra["checks"]["rows"],
                           tol={"forward": 1e-5, "grad": 1e-4},
                           vs="FP64 loop on the host (torch corrector in float64, oracle step), FP64 central FD")
-    if which == "ks_diff":  # the FNO's spectral convolution layer against the HBM peak
+    if which == "ks_diff":  # the general path's spectral convolution layer against the HBM peak
         extra["roofline"] = spectral_layer_roofline(dev, B, N)
-    if which == "burgers_diff":  # the fused corrector rollout against the FP32 FMA peak
+    if which == "burgers_diff":  # the fused corrector rollout's FP32 work against the FP32 FMA peak
         from inc_b200.roofline import burgers_cnn_flops_per_cell_step
         fpc = burgers_cnn_flops_per_cell_step(cfg["scheme"])
         achieved = cells * fpc / (ms(t_fwd) * 1e-3) / 1e12
@@ -887,6 +887,7 @@ def bench_diff(args, dev, world, which):
         extra["fused_inference_roofline"] = {
             "kernel": "inc_burgers_cnn_rollout (k_cnn_rollout<256>)", "bound": "fp32", "achieved": achieved,
             "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None, "flops_per_cell_step": fpc,
+            "note": "FP32 work; the hidden layers' part runs on the tensor cores, so this can exceed 1",
             "peak_source": "FP32 FMA loop (inc_bench_fma) measured in this run"}
     cfg = dict(name=which, B=B, N=N, steps=steps, scheme=cfg["scheme"],
                corrector=("PeriodicCNN1D(4x32ch,k5,GELU)" if which == "burgers_diff" else "FNO1D(L=100, modes=16, width=64), the reference's corrector"))
@@ -1132,9 +1133,8 @@ def diff_line(args, world, cfg, cells, times, extra):
                    "checkpoint_every": extra.get("graph_ckpt"),
                    "checkpoint_note": ("solver adjoint replays its own states; the corrector's activations "
                                        "are kept (None) or recomputed every 8 steps" if cfg["name"] == "ks_diff"
-                                       else "solver adjoint replays its states from checkpoints every 8 steps; "
-                                       "the fused forward records the CNN's hidden pre-activations (537 MB) "
-                                       "and the fused backward reads them"),
+                                       else "the fused forward records every state and the CNN's hidden "
+                                       "pre-activations (537 MB); the backward reads them and replays nothing"),
                    "value_is": "whole training step (rollout, loss, backward, Adam) in one CUDA graph",
                    "l2": "inputs and activations exceed L2 (not flushed)" if cfg["name"] == "ks_diff"
                    else "not flushed (the recorded pre-activations, 537 MB, exceed L2)",
