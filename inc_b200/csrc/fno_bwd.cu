@@ -490,9 +490,12 @@ int run_wgrad(WgradArgs a, int* blocks, cudaStream_t st) {
 
 // ---- Fourier weight gradients -------------------------------------------------------------
 // dW[c][o][k] = (c_k / n) sum_b conj(X[k][b][c]) G[k][b][o] (c_0 = 1, c_k = 2; torch's convention for
-// complex gradients), all four layers: block = mode, layer, 32 of the o; thread: 4 c x 2 o, the
+// complex gradients), all four layers: block = mode, layer, 16 of the o; thread: 4 c x 1 o, the
 // factors Re X and Im X in separate packed accumulators (two packed operations per complex
-// product), the next 16 trajectories loaded while these are multiplied.
+// product), the next 32 trajectories loaded while these are multiplied.  67 MB are read (10.4 us
+// at the copy rate for 256 trajectories of 64 channels and 16 modes); bound by the loads' and
+// barriers' latency: 23.2 us with four warps a scheduler, 27.4 with two (32 of the o per
+// block, 16 trajectories a time).
 struct ModesGradArgs {
     const float2* x;  // [4][modes][batch][W]
     const float2* g;  // [4][modes][batch][W]
@@ -501,11 +504,11 @@ struct ModesGradArgs {
 };
 template <int W>
 __global__ void __launch_bounds__(W * 4) k_fno_modes_grad(ModesGradArgs a) {
-    constexpr int TB = 16, T = W * 4, LX = TB * W / T, LG = TB * 32 / T;
-    __shared__ float2 X[TB][W], G[TB][32];
-    const int k = blockIdx.x, l = blockIdx.y, o0 = blockIdx.z * 32;
+    constexpr int TB = 32, T = W * 4, LX = TB * W / T, LG = TB * 16 / T;
+    __shared__ float2 X[TB][W], G[TB][16];
+    const int k = blockIdx.x, l = blockIdx.y, o0 = blockIdx.z * 16;
     const int64_t base = ((int64_t)l * a.modes + k) * a.batch * W;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx, tx + 16; c: ty + i W / 4
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx; c: ty + i W / 4
     float2 rx[LX], rg[LG];
     auto load = [&](int b0) {
 #pragma unroll
@@ -515,15 +518,14 @@ __global__ void __launch_bounds__(W * 4) k_fno_modes_grad(ModesGradArgs a) {
         }
 #pragma unroll
         for (int i = 0; i < LG; ++i) {
-            const int e = threadIdx.x + i * T, b = b0 + e / 32;
-            rg[i] = b < a.batch ? __ldg(a.g + base + (int64_t)b * W + o0 + e % 32) : make_float2(0.f, 0.f);
+            const int e = threadIdx.x + i * T, b = b0 + e / 16;
+            rg[i] = b < a.batch ? __ldg(a.g + base + (int64_t)b * W + o0 + e % 16) : make_float2(0.f, 0.f);
         }
     };
-    float2 tre[4][2], tim[4][2];
+    float2 tre[4], tim[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) tre[i][j] = tim[i][j] = make_float2(0.f, 0.f);
+        tre[i] = tim[i] = make_float2(0.f, 0.f);
     load(0);
     for (int b0 = 0; b0 < a.batch; b0 += TB) {
         __syncthreads();
@@ -533,39 +535,32 @@ __global__ void __launch_bounds__(W * 4) k_fno_modes_grad(ModesGradArgs a) {
         for (int i = 0; i < LG; ++i) (&G[0][0])[threadIdx.x + i * T] = rg[i];
         __syncthreads();
         if (b0 + TB < a.batch) load(b0 + TB);
-        float2 re[4][2], im[4][2];  // (a chunk's sum first: shorter chains)
+        float2 re[4], im[4];  // (a chunk's sum first: shorter chains)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) re[i][j] = im[i][j] = make_float2(0.f, 0.f);
+            re[i] = im[i] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int b = 0; b < TB; ++b) {
-            const float2 g[2] = {G[b][tx], G[b][tx + 16]};
+            const float2 g = G[b][tx];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float2 x = X[b][ty + i * (W / 4)];
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    re[i][j] = __ffma2_rn(make_float2(x.x, x.x), g[j], re[i][j]);
-                    im[i][j] = __ffma2_rn(make_float2(x.y, x.y), g[j], im[i][j]);
-                }
+                re[i] = __ffma2_rn(make_float2(x.x, x.x), g, re[i]);
+                im[i] = __ffma2_rn(make_float2(x.y, x.y), g, im[i]);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                tre[i][j] = __fadd2_rn(tre[i][j], re[i][j]);
-                tim[i][j] = __fadd2_rn(tim[i][j], im[i][j]);
-            }
+        for (int i = 0; i < 4; ++i) {
+            tre[i] = __fadd2_rn(tre[i], re[i]);
+            tim[i] = __fadd2_rn(tim[i], im[i]);
+        }
     }
     const float s = (k == 0 ? 1.f : 2.f) / (float)a.n;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)  // conj(x) g = (x.x g.x + x.y g.y, x.x g.y - x.y g.x)
-            a.out[l][((int64_t)(ty + i * (W / 4)) * W + o0 + tx + 16 * j) * a.modes + k] =
-                make_float2((tre[i][j].x + tim[i][j].y) * s, (tre[i][j].y - tim[i][j].x) * s);
+        // conj(x) g = (x.x g.x + x.y g.y, x.x g.y - x.y g.x)
+        a.out[l][((int64_t)(ty + i * (W / 4)) * W + o0 + tx) * a.modes + k] =
+            make_float2((tre[i].x + tim[i].y) * s, (tre[i].y - tim[i].x) * s);
 }
 
 // ---- the blocks' partial sums, added in a fixed order ---------------------------------------
@@ -757,7 +752,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
     mg.batch = B;
     mg.modes = M;
     mg.n = n;
-    k_fno_modes_grad<W><<<dim3(M, 4, W / 32), W * 4, 0, st>>>(mg);
+    k_fno_modes_grad<W><<<dim3(M, 4, W / 16), W * 4, 0, st>>>(mg);
     return check_launch("fno gradients");
 }
 
