@@ -609,7 +609,7 @@ struct ModesArgs {
 struct ModesSmem {
     alignas(128) unsigned char ft[64 * F_PLANE];
     alignas(128) unsigned char a[2][3 * 8 * A_PITCH];
-    uint64_t bar_images, bar[2], bar_tile;
+    uint64_t bar_images, bar[2];
     uint32_t tmem;
 };
 
