@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
     __syncthreads();
     tc::fence_after();
     // this warp's lanes of its tile's accumulators
-    const uint32_t acc = S.tmem + 96 * tile + ((uint32_t)(t & 96) << 16);
+    const uint32_t acc = S.tmem + 128 * tile + ((uint32_t)(t & 96) << 16);
     Ctx<1> cx;
     make_ctx<1, N>(a, valid ? row : 0, g, true, cx);
     cx.has_s = true;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
                 tc::fence_after();
 #pragma unroll
                 for (int q = 0; q < Cfg::TILES; ++q) {
-                    issue_layer<N>(S.tmem + 96 * q, S.act, S.w[l], q);
+                    issue_layer<N>(S.tmem + 128 * q, S.act, S.w[l], q);
                     tc::commit(&S.bar[q]);
                 }
             }

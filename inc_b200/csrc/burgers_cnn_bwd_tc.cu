@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t acc = S.tmem + 96 * tile + ((uint32_t)(t & 96) << 16);
+    const uint32_t acc = S.tmem + 128 * tile + ((uint32_t)(t & 96) << 16);
     uint32_t phase = 0;
     bool fail = false;  // a wait for the tensor cores ran out: the gradients turn to NaN
     Ctx<1> cx;
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         __syncthreads();
         if (issuer && tc::elect()) {
             tc::fence_after();
-            issue_layer<N>(S.tmem + 96 * tile, S.act, S.w[l], tile);
+            issue_layer<N>(S.tmem + 128 * tile, S.act, S.w[l], tile);
             tc::commit(&S.bar[tile]);
         }
         return s * (1.f / 256.f) * ws[l];
@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
 // A unit is 256 cells at one step (R rows of N <= 256 cells, or half a row of 512), a group
 // GROUP steps of the same cells: its products accumulate in tensor memory with one pair of
 // scales (the maxima over the group), then the sums are read once.  Lanes are (piece of dz,
-// co), columns (tap, piece of a, ci); the useful six of the nine piece pairs are added in
-// registers.  dz is scaled to 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
+// co), columns (tap, piece of a, ci); the nine piece pairs are added in registers, each with its
+// order's power of two.  dz is scaled to 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
 // Even blocks take layer 2 (a = gelu(z1), z1 from the recorded state), odd ones layer 3.
 // The bias gradient is one more block of columns (a = 1).  16 warps prepare the two operand
 // tiles (two buffers), a 17th issues.  Bound by the preparation (about 5,500 clocks a unit: two
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
 #pragma unroll
         for (int q = 0; q < 2; ++q)
             *reinterpret_cast<uint4*>(S.buf[q].a + 12 * PL + i * 16) =
-                make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+                make_uint4(0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u);
     tc::fence_smem();
     tc::fence_before();
     __syncthreads();
@@ -561,7 +561,8 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
         tc::fence_after();
         // (every lane reads the same columns: loads under a branch cost a few hundred clocks each)
         const float f = fail ? __int_as_float(0x7fffffff) : f_done;
-        const float f1 = lane_q < 2 ? f : 0.f, f2 = lane_q < 1 ? f : 0.f;
+        const float order = lane_q == 0 ? 1.f : (lane_q == 1 ? tc::DOWN : tc::DOWN * tc::DOWN);  // of dz's piece
+        const float f0 = f * order, f1 = f0 * tc::DOWN, f2 = f1 * tc::DOWN;
         const uint32_t dl = d + ((uint32_t)(tid & 96) << 16) + 8 * colq;
         float ones[8];
         tc::tmem_ld8(d + ((uint32_t)(tid & 96) << 16) + ONES, ones);
@@ -573,9 +574,9 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
             tc::tmem_ld8(dl + tap_col(k) + 64, q2);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[k][i] += fmaf(q0[i], f, fmaf(q1[i], f1, q2[i] * f2));
+            for (int i = 0; i < 8; ++i) acc[k][i] += fmaf(q0[i], f0, fmaf(q1[i], f1, q2[i] * f2));
         }
-        gb += ones[0] * (fail ? f : fb_done);
+        gb += ones[0] * ((fail ? f : fb_done) * order);
         tc::fence_before();
         wg_sync();  // read everywhere before the next group's products
     };

@@ -6,11 +6,11 @@
 // shifted by one cell.  Activations sit in shared memory in the core-matrix layout of
 // tc.cuh, one slot (16 bytes per 8 channels and piece) per cell, with the two halo
 // cells of each side stored, so a tap is a start address 16 bytes further.  The
-// weights' three pieces are stacked as 96 columns: the activations' hi piece takes
-// all 96 in one instruction, mid 64 (hi, mid) and lo 32 (hi), so the accumulator
-// columns are hi.hi | first-order | second-order sums (see tc.cuh).  One instruction of
+// weights' three pieces are stacked as 96 columns: the activations' hi and mid pieces take
+// all 96 in one instruction each, lo 64 (hi, mid), each 32 columns further, so the 128
+// accumulator columns are the sums of orders 0 to 3 (see tc.cuh).  One instruction of
 // N = 96 issues in 56 cycles, N = 64 in 48, N = 32 in 45 (measured, M = 128, K = 16):
-// 1,490 cycles for a layer of 128 cells against 6,550 on the FP32 pipes at their peak.
+// 1,640 cycles for a layer of 128 cells against 6,550 on the FP32 pipes at their peak.
 #pragma once
 #include "burgers_cnn.cuh"
 #include "gelu.cuh"
@@ -30,7 +30,7 @@ struct TcCfg {
     static constexpr int SLOTS = R * (N + 4);        // cells with halos
     static constexpr int PLANE = SLOTS * 16;         // bytes of 8 channels of one piece
     static constexpr int TILES = N < 128 ? R : N / 128;
-    static constexpr int COLS = TILES <= 1 ? 128 : TILES <= 2 ? 256 : 512;  // 96 used per tile
+    static constexpr int COLS = 128 * TILES;
     static constexpr int WARPS_PER_ROW = N / 32;
 };
 constexpr int W_TAP = 96 * 32 * 2;             // bytes of one tap's stacked weight pieces
@@ -95,7 +95,7 @@ INC_DEV void store_cell(unsigned char* act, const float (&v)[C], float inv, int 
 }
 
 // One layer's products for one tile: 5 taps x 2 channel halves, accumulators at
-// columns d .. d + 95 of the tile's 128 lanes; one thread issues (tc::elect).
+// columns d .. d + 127 of the tile's 128 lanes; one thread issues (tc::elect).
 template <int N>
 INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned char* w, int tile) {
     constexpr int PL = TcCfg<N>::PLANE;
@@ -110,45 +110,54 @@ INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned ch
         for (int h = 0; h < 2; ++h) {
             const uint64_t b = tc::desc_at(bd, k * W_TAP + 2 * h * W_PLANE);
             const uint64_t a = tc::desc_at(ad, k * 16 + 2 * h * PL);
+            const uint64_t mid = tc::desc_at(a, 4 * PL), lo = tc::desc_at(a, 8 * PL);
             tc::mma(d, a, b, i96, k + h > 0);
-            tc::mma(d + 32, tc::desc_at(a, 4 * PL), b, i64, true);
-            tc::mma(d + 64, tc::desc_at(a, 8 * PL), b, i32, true);
+            if (k + h > 0) {
+                tc::mma(d + 32, mid, b, i96, true);
+            } else {  // (the first to write the last 32 columns)
+                tc::mma(d + 32, mid, b, i64, true);
+                tc::mma(d + 96, mid, tc::desc_at(b, 64 * 16), i32, false);
+            }
+            tc::mma(d + 64, lo, b, i64, true);
         }
     }
 }
 
-// 16 channels (c0 .. c0 + 15) of this thread's cell: bias + (hi.hi + (first + second order)) f
+// 16 channels (c0 .. c0 + 15) of this thread's cell, the four orders added up
+INC_DEV void read_orders16(uint32_t d, int c0, float2 (&z)[8]) {
+    const float2 down = f2s(tc::DOWN);
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) {
+        float v0[8], v1[8], v2[8], v3[8];
+        tc::tmem_ld8(d + c0 + h, v0);
+        tc::tmem_ld8(d + 32 + c0 + h, v1);
+        tc::tmem_ld8(d + 64 + c0 + h, v2);
+        tc::tmem_ld8(d + 96 + c0 + h, v3);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const float2 s = __ffma2_rn(f2(v3[i], v3[i + 1]), down, f2(v2[i], v2[i + 1]));
+            z[(h + i) / 2] = __ffma2_rn(__ffma2_rn(s, down, f2(v1[i], v1[i + 1])), down, f2(v0[i], v0[i + 1]));
+        }
+    }
+}
+
+// the same times f, plus bias
 INC_DEV void read_layer16(uint32_t d, int c0, float f, const float* bias, float2 (&z)[8]) {
-    float v0[16], v1[16], v2[16];
-    tc::tmem_ld16(d + c0, v0);
-    tc::tmem_ld16(d + 32 + c0, v1);
-    tc::tmem_ld16(d + 64 + c0, v2);
-    tc::tmem_ld_wait();
+    read_orders16(d, c0, z);
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
         const float4 b = lds4(bias + c0 + 2 * i);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int e = 2 * (i + j);
-            const float2 s = __fadd2_rn(f2(v0[e], v0[e + 1]), __fadd2_rn(f2(v1[e], v1[e + 1]), f2(v2[e], v2[e + 1])));
-            z[i + j] = __ffma2_rn(s, f2s(f), j == 0 ? f2(b.x, b.y) : f2(b.z, b.w));
-        }
+        z[i] = __ffma2_rn(z[i], f2s(f), f2(b.x, b.y));
+        z[i + 1] = __ffma2_rn(z[i + 1], f2s(f), f2(b.z, b.w));
     }
 }
 
 // the same without a bias
 INC_DEV void read_sums16(uint32_t d, int c0, float f, float2 (&z)[8]) {
-    float v0[16], v1[16], v2[16];
-    tc::tmem_ld16(d + c0, v0);
-    tc::tmem_ld16(d + 32 + c0, v1);
-    tc::tmem_ld16(d + 64 + c0, v2);
-    tc::tmem_ld_wait();
+    read_orders16(d, c0, z);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int e = 2 * i;
-        z[i] = __fmul2_rn(__fadd2_rn(f2(v0[e], v0[e + 1]), __fadd2_rn(f2(v1[e], v1[e + 1]), f2(v2[e], v2[e + 1]))),
-                          f2s(f));
-    }
+    for (int i = 0; i < 8; ++i) z[i] = __fmul2_rn(z[i], f2s(f));
 }
 
 // max |v| over this thread's channels and its row (a barrier of the CTA inside; fails

@@ -86,12 +86,12 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
             take_over();
             if (ok && tc::elect()) {  // hidden values: columns 0..127 and 128..255
                 tc::fence_after();
-                issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
+                issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w));
                 tc::commit(&S.bar);
             }
             __syncwarp();
 #pragma unroll 1
-            for (int h = 0; h < 2; ++h) {  // dL/dx += g1[64 h ..] w1, into columns 0.. and 128.., read by then
+            for (int h = 0; h < 2; ++h) {  // g1[64 h ..] w1, into columns 64 h .. and 128 + 64 h .., read by then
                 take_over();
                 if (ok && tc::elect()) {
                     tc::fence_after();
@@ -99,17 +99,28 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
                     const uint64_t w = tc::smem_desc(tc::smem_u32(S.w) + 64 * h * 16, 128, 384 * 16);
                     constexpr uint32_t id = tc::instr_desc(128, W, false, true);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint64_t a0 = tc::desc_at(x, 2 * k * 2048), a1 = tc::desc_at(a0, 8 * 2048);
-                        const uint64_t a2 = tc::desc_at(a0, 16 * 2048), b0 = tc::desc_at(w, 16 * k * 16);
-                        const uint64_t b1 = tc::desc_at(b0, 128 * 16), b2 = tc::desc_at(b0, 256 * 16);
-                        tc::mma(d, a0, b0, id, h + k > 0);
-                        tc::mma(d + 128, a1, b0, id, h + k > 0);
-                        tc::mma(d + 128, a0, b1, id, true);
-                        tc::mma(d + 128, a0, b2, id, true);
-                        tc::mma(d + 128, a1, b1, id, true);
-                        tc::mma(d + 128, a2, b0, id, true);
-                    }
+                    for (int stage = 3; stage > 0; --stage)  // (as issue_stage; the operand B is MN-major here)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t c0 = d + 64 * h, c1 = c0 + 128;
+                            const uint64_t a0 = tc::desc_at(x, 2 * k * 2048), a1 = tc::desc_at(a0, 8 * 2048);
+                            const uint64_t a2 = tc::desc_at(a0, 16 * 2048), b0 = tc::desc_at(w, 16 * k * 16);
+                            const uint64_t b1 = tc::desc_at(b0, 128 * 16), b2 = tc::desc_at(b0, 256 * 16);
+                            if (stage == 3) {
+                                tc::mma(c1, a1, b2, id, k > 0);
+                                tc::mma(c1, a2, b1, id, true);
+                            } else if (stage == 2) {
+                                if (k == 0) tc::mma_scaled(c1, a0, b2, id);
+                                else tc::mma(c1, a0, b2, id, true);
+                                tc::mma(c1, a1, b1, id, true);
+                                tc::mma(c1, a2, b0, id, true);
+                            } else {
+                                tc::mma(c0, a0, b0, id, k > 0);
+                                if (k == 0) tc::mma_scaled(c1, a0, b1, id);
+                                else tc::mma(c1, a0, b1, id, true);
+                                tc::mma(c1, a1, b0, id, true);
+                            }
+                        }
                     tc::commit(&S.bar);
                 }
                 __syncwarp();
@@ -170,8 +181,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
                     const int j = c + e;
                     const float2 bi = *reinterpret_cast<const float2*>(&S.b1[j0 + j]);
                     const float2 w2 = *reinterpret_cast<const float2*>(&S.w2[j0 + j]);
-                    const float2 z = __ffma2_rn(
-                        __fadd2_rn(make_float2(x0[e], x0[e + 1]), make_float2(x1[e], x1[e + 1])), f, bi);
+                    const float2 z = __ffma2_rn(join2(x0[e], x0[e + 1], x1[e], x1[e + 1]), f, bi);
                     float2 y, gp;
                     act::gelu_both2(z, y, gp);
                     const float2 gg = make_float2(gy, gy);
@@ -200,14 +210,16 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj_bwd(ProjBwdArgs a) {
         float m3 = 0.f;
         float* out = a.g_x + ((int64_t)b * W + half * C) * N + p;
 #pragma unroll
-        for (int c = 0; c < C; c += 16) {
-            float x0[16], x1[16];
-            tc::tmem_ld16(dl + half * C + c, x0);
-            tc::tmem_ld16(dl + 128 + half * C + c, x1);
+        for (int c = 0; c < C; c += 8) {
+            float x0[8], x1[8], y0[8], y1[8];
+            tc::tmem_ld8(dl + half * C + c, x0);
+            tc::tmem_ld8(dl + 128 + half * C + c, x1);
+            tc::tmem_ld8(dl + 64 + half * C + c, y0);
+            tc::tmem_ld8(dl + 192 + half * C + c, y1);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float r = (x0[e] + x1[e]) * fs;
+            for (int e = 0; e < 8; ++e) {
+                const float r = fmaf(x1[e] + y1[e], tc::DOWN, x0[e] + y0[e]) * fs;
                 m3 = fmaxf(m3, fabsf(r));
                 if (on) out[(c + e) * N] = fail ? __int_as_float(0x7fffffff) : r;
             }
@@ -259,8 +271,9 @@ int launch_proj_bwd(const ProjBwdArgs& a, int* blocks, cudaStream_t st) {
 // g: a unit is `seg` points of one trajectory, 64 per chunk.  The rows of g in three
 // stacked pieces are the accumulator lanes, those of x the columns:
 //   MO = 32:  lanes (hi, mid, lo) x columns (hi, mid, lo), one product;
-//   MO = 64:  lanes (hi, mid) x (hi, mid, lo), and lo x hi added to the columns of hi x lo;
-//   MO = 128: hi x (hi, mid, lo), mid x (hi, mid), lo x hi.
+//   MO = 64:  lanes (hi, lo) x (hi, mid, lo), and (mid, 64 rows of zeros) x the same, one order
+//             further, so that in either half of the lanes a column group is one order;
+//   MO = 128: hi x (hi, mid, lo), mid x (hi, mid, lo) one order further, lo x (hi, mid) two.
 // A unit's sums are read into registers (with its two scales) while the next unit's products
 // run into the other half of the columns, so no chain in the tensor cores is longer than a
 // row; g is scaled to 128 instead of 256, so that 512 full-scale terms stay below 2^24 (tc.cuh).
@@ -280,7 +293,8 @@ struct WgradArgs {
 constexpr int WG_WORKERS = 512;
 template <int MO, int W>
 struct WgradSmem {
-    static constexpr int GP = 3 * MO * 16 + 16, XP = 3 * W * 16 + 16;  // plane pitches
+    static constexpr int GP = (MO == 64 ? 4 : 3) * MO * 16 + 16, XP = 3 * W * 16 + 16;  // plane pitches
+    static constexpr int MID = (MO == 64 ? 2 : 1) * MO * 16, LO = (MO == 64 ? 1 : 2) * MO * 16;  // of g's rows
     struct Buf {
         alignas(128) unsigned char g[8 * GP];
         alignas(128) unsigned char x[8 * XP];
@@ -306,6 +320,11 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         tc::mbar_init(&S.bar[1], 1);
         tc::mbar_init_fence();
     }
+    if (MO == 64) {  // the rows of zeros of both buffers' 8 planes
+        for (int i = tid; i < 2 * 8 * 64; i += WG_WORKERS)
+            *reinterpret_cast<uint4*>(S.buf[i >> 9].g + (i >> 6 & 7) * GP + (192 + (i & 63)) * 16) = make_uint4(0, 0, 0, 0);
+        tc::fence_smem();
+    }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -321,13 +340,18 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         for (int k = 0; k < 4; ++k) {
             const uint64_t b = tc::desc_at(x, 2 * k * XP), gk = tc::desc_at(g, 2 * k * GP);
             const bool add = !first || k > 0;
-            tc::mma(du, gk, b, tc::instr_desc(128, 3 * W), add);
-            if (MO == 64) {
-                tc::mma(du + 2 * W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, W), true);
-            } else if (MO == 128) {
-                tc::mma(du + W, tc::desc_at(gk, 128 * 16), b, tc::instr_desc(128, 2 * W), true);
-                tc::mma(du + 2 * W, tc::desc_at(gk, 256 * 16), b, tc::instr_desc(128, W), true);
+            constexpr uint32_t i3 = tc::instr_desc(128, 3 * W), i2 = tc::instr_desc(128, 2 * W);
+            tc::mma(du, gk, b, i3, add);
+            if (MO >= 64) {
+                const uint64_t mid = tc::desc_at(gk, Smem::MID);
+                if (add) {
+                    tc::mma(du + W, mid, b, i3, true);
+                } else {  // (the first to write the last W columns)
+                    tc::mma(du + W, mid, b, i2, true);
+                    tc::mma(du + 3 * W, mid, tc::desc_at(b, 2 * W * 16), tc::instr_desc(128, W), false);
+                }
             }
+            if (MO == 128) tc::mma(du + 2 * W, tc::desc_at(gk, Smem::LO), b, i2, true);
         }
         tc::commit(&S.bar[n & 1]);
     };
@@ -338,6 +362,8 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
     // lane, quarter of the columns, piece of the lane
     constexpr int CQ = W / 4;
     const int t = tid & 127, quarter = tid >> 7, group = t / MO;
+    // of the lane's piece (MO = 64: the upper half is lo)
+    const float order = group == 0 ? 1.f : (MO == 32 && group == 1 ? tc::DOWN : tc::DOWN * tc::DOWN);
     float acc[CQ], rs[IT];
 #pragma unroll
     for (int i = 0; i < CQ; ++i) acc[i] = 0.f;
@@ -369,14 +395,21 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
         tc::fence_after();
         if (fail) f = __int_as_float(0x7fffffff);
         const uint32_t dl = d + (n / chunks & 1) * COLS + ((uint32_t)(t & 96) << 16) + quarter * CQ;
-        float q0[CQ], q1[CQ], q2[CQ];
-        tc::tmem_ld(dl, q0);
-        tc::tmem_ld(dl + W, q1);
-        tc::tmem_ld(dl + 2 * W, q2);
-        tc::tmem_ld_wait();
+        f *= order;
 #pragma unroll
-        for (int i = 0; i < CQ; ++i)
-            acc[i] += (q0[i] + ((group < 2 ? q1[i] : 0.f) + (group < 1 ? q2[i] : 0.f))) * f;
+        for (int c = 0; c < CQ; c += 8) {
+            float q0[8], q1[8], q2[8], q3[8];
+            tc::tmem_ld8(dl + c, q0);
+            tc::tmem_ld8(dl + c + W, q1);
+            tc::tmem_ld8(dl + c + 2 * W, q2);
+            if (MO >= 64) tc::tmem_ld8(dl + c + 3 * W, q3);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float s = MO >= 64 ? fmaf(q3[i], tc::DOWN, q2[i]) : q2[i];
+                acc[c + i] += fmaf(fmaf(s, tc::DOWN, q1[i]), tc::DOWN, q0[i]) * f;
+            }
+        }
     };
     auto chunk = [&](int n, int buf, float4(&w)[IT][2]) {
         const float f_prev = sg * (1.f / 128.f) * (sx * (1.f / 256.f));
@@ -413,10 +446,9 @@ __global__ void __launch_bounds__(WG_WORKERS, 1) k_fno_wgrad(WgradArgs a) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) tc::split2(e[j], make_float2(inv, inv), hi[j], mid[j], lo[j]);
                 unsigned char* s = is_g ? S.buf[buf].g + c8 * GP + r * 16 : S.buf[buf].x + c8 * XP + (r - MO) * 16;
-                const int piece = (is_g ? MO : W) * 16;
                 *reinterpret_cast<uint4*>(s) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(s + piece) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
-                *reinterpret_cast<uint4*>(s + 2 * piece) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                *reinterpret_cast<uint4*>(s + (is_g ? Smem::MID : W * 16)) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+                *reinterpret_cast<uint4*>(s + (is_g ? Smem::LO : 2 * W * 16)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
         load(n + DEPTH, w);

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
             take_over();
             if (ok && tc::elect()) {
                 tc::fence_after();
-                issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
+                issue_product<128, W>(d, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w));
                 tc::commit(&S.bar);
             }
             __syncwarp();
@@ -118,11 +118,9 @@ __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
 #pragma unroll
             for (int e = 0; e < 16; e += 4) {
                 const float4 bi = lds4(&S.b1[64 * half + j + e]), w2 = lds4(&S.w2[64 * half + j + e]);
-                const float2 z0 = __ffma2_rn(__fadd2_rn(make_float2(x0[e], x0[e + 1]), make_float2(x1[e], x1[e + 1])), f,
-                                             make_float2(bi.x, bi.y));
-                const float2 z1 = __ffma2_rn(
-                    __fadd2_rn(make_float2(x0[e + 2], x0[e + 3]), make_float2(x1[e + 2], x1[e + 3])), f,
-                    make_float2(bi.z, bi.w));
+                const float2 z0 = __ffma2_rn(join2(x0[e], x0[e + 1], x1[e], x1[e + 1]), f, make_float2(bi.x, bi.y));
+                const float2 z1 =
+                    __ffma2_rn(join2(x0[e + 2], x0[e + 3], x1[e + 2], x1[e + 3]), f, make_float2(bi.z, bi.w));
                 y0 = __ffma2_rn(act::gelu2(z0), make_float2(w2.x, w2.y), y0);
                 y1 = __ffma2_rn(act::gelu2(z1), make_float2(w2.z, w2.w), y1);
             }

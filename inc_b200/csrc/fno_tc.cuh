@@ -188,25 +188,49 @@ INC_DEV float point_max(const float2 (&v)[C / 2]) {
     for (int i = 0; i < C / 2; ++i) m = fmaxf(m, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
     return m;
 }
-// D[128 x N] at columns d .. d + N - 1 (hi.hi) and d + N .. d + 2N - 1 (the rest) = (or +=,
-// with `add`) A [128 x K] B[N x K]^T.  A: pieces of a point tile (planes of 2048 bytes,
-// pieces a_piece apart); B: stacked pieces [3 N][K].  One thread (tc::elect).
-template <int N, int K>
-INC_DEV void issue_product(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b, bool add) {
+// A [128 x K] B[N x K]^T, one stage of it.  A: pieces of a point tile (planes of 2048 bytes,
+// pieces a_piece apart); B: stacked pieces [3 N][K].  The stages 3, 2, 1 leave order 0 in
+// columns d .. d + N - 1 and, in d + N .. d + 2N - 1, order 1 + 2^-14 (order 2 + 2^-14 order 3).  FIRST: the first
+// product of the accumulators (several may add up, stage by stage).  One thread (tc::elect).
+template <int N, int K, int STAGE, bool FIRST>
+INC_DEV void issue_stage(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b) {
     constexpr uint32_t plane_b = 3 * N * 16;
     constexpr uint32_t i2 = tc::instr_desc(128, 2 * N), i1 = tc::instr_desc(128, N);
     const uint64_t ad = tc::smem_desc(a, 2048, 128), bd = tc::smem_desc(b, plane_b, 128);
 #pragma unroll
     for (int k = 0; k < K / 16; ++k) {
+        const bool first = FIRST && k == 0;
         const uint64_t a0 = tc::desc_at(ad, 2 * k * 2048), b0 = tc::desc_at(bd, 2 * k * plane_b);
         const uint64_t a1 = tc::desc_at(a0, a_piece), a2 = tc::desc_at(a0, 2 * a_piece);
         const uint64_t b1 = tc::desc_at(b0, N * 16), b2 = tc::desc_at(b0, 2 * N * 16);
-        tc::mma(d, a0, b0, i2, add || k > 0);  // hi.hi | hi.mid
-        tc::mma(d + N, a1, b0, i1, true);      // mid.hi
-        tc::mma(d + N, a0, b2, i1, true);      // hi.lo
-        tc::mma(d + N, a1, b1, i1, true);      // mid.mid
-        tc::mma(d + N, a2, b0, i1, true);      // lo.hi
+        if constexpr (STAGE == 3) {
+            tc::mma(d + N, a1, b2, i1, !first);  // mid.lo
+            tc::mma(d + N, a2, b1, i1, true);    // lo.mid
+        } else if constexpr (STAGE == 2) {
+            if (first) tc::mma_scaled(d + N, a0, b2, i1);  // hi.lo
+            else tc::mma(d + N, a0, b2, i1, true);
+            tc::mma(d + N, a1, b1, i1, true);  // mid.mid
+            tc::mma(d + N, a2, b0, i1, true);  // lo.hi
+        } else {
+            if (first) {  // hi.hi, hi.mid
+                tc::mma(d, a0, b0, i1, false);
+                tc::mma_scaled(d + N, a0, b1, i1);
+            } else {
+                tc::mma(d, a0, b0, i2, true);
+            }
+            tc::mma(d + N, a1, b0, i1, true);  // mid.hi
+        }
     }
+}
+template <int N, int K>
+INC_DEV void issue_product(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b) {
+    issue_stage<N, K, 3, true>(d, a, a_piece, b);
+    issue_stage<N, K, 2, true>(d, a, a_piece, b);
+    issue_stage<N, K, 1, true>(d, a, a_piece, b);
+}
+// the two accumulators of such a product added up
+INC_DEV float2 join2(float x0, float y0, float x1, float y1) {
+    return __ffma2_rn(make_float2(x1, y1), make_float2(tc::DOWN, tc::DOWN), make_float2(x0, y0));
 }
 
 // sums over the warp of each of C values: lane l is left with that of channel l / (32 / C)
@@ -329,8 +353,14 @@ __global__ void __launch_bounds__(layer_threads(MODE), 2) k_fno_layer(LayerArgs 
     const uint32_t d = S.tmem;
     auto products = [&](int buf) {  // one thread
         tc::fence_after();
-        issue_product<W, W>(d + 2 * W * buf, tc::smem_u32(S.x), W * 256, tc::smem_u32(S.w), false);
-        issue_product<W, 32>(d + 2 * W * buf, tc::smem_u32(S.gt), 8192, tc::smem_u32(S.m), true);
+        const uint32_t dt = d + 2 * W * buf, x = tc::smem_u32(S.x), w = tc::smem_u32(S.w);
+        const uint32_t gt = tc::smem_u32(S.gt), m = tc::smem_u32(S.m);
+        issue_stage<W, W, 3, true>(dt, x, W * 256, w);
+        issue_stage<W, 32, 3, false>(dt, gt, 8192, m);
+        issue_stage<W, W, 2, true>(dt, x, W * 256, w);
+        issue_stage<W, 32, 2, false>(dt, gt, 8192, m);
+        issue_stage<W, W, 1, true>(dt, x, W * 256, w);
+        issue_stage<W, 32, 1, false>(dt, gt, 8192, m);
         tc::commit(&S.bar_layer);
     };
     if (!kBwd && tid >= WORKERS) {  // ---- the issuing warp
@@ -503,8 +533,8 @@ __global__ void __launch_bounds__(layer_threads(MODE), 2) k_fno_layer(LayerArgs 
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const int e = i + 2 * j, ch = i0 + e;
-                    float2 z = __ffma2_rn(__fadd2_rn(make_float2(x0[e], x0[e + 1]), make_float2(x1[e], x1[e + 1])),
-                                          make_float2(fx, fx), j == 0 ? make_float2(bi.x, bi.y) : make_float2(bi.z, bi.w));
+                    float2 z = __ffma2_rn(join2(x0[e], x0[e + 1], x1[e], x1[e + 1]), make_float2(fx, fx),
+                                          j == 0 ? make_float2(bi.x, bi.y) : make_float2(bi.z, bi.w));
                     if constexpr (MODE == BWD) z = __fmul2_rn(z, act::gelu_grad2(zp[ch / 2]));
                     if constexpr (MODE == FWD) {
                         m = fmaxf(m, fmaxf(z.x, z.y));  // |gelu(z)| <= max(z, 0.17)
@@ -645,9 +675,16 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const uint64_t ak = tc::desc_at(x, 2 * k * A_PITCH), bd = tc::desc_at(f, 2 * k * F_PLANE);
-                        tc::mma(d, ak, bd, tc::instr_desc(128, 96), ch + k > 0);
-                        tc::mma(d + 32, tc::desc_at(ak, 8 * A_PITCH), bd, tc::instr_desc(128, 64), true);
-                        tc::mma(d + 64, tc::desc_at(ak, 16 * A_PITCH), bd, tc::instr_desc(128, 32), true);
+                        const uint64_t mid = tc::desc_at(ak, 8 * A_PITCH), lo = tc::desc_at(ak, 16 * A_PITCH);
+                        const bool add = ch + k > 0;
+                        tc::mma(d, ak, bd, tc::instr_desc(128, 96), add);
+                        if (add) {
+                            tc::mma(d + 32, mid, bd, tc::instr_desc(128, 96), true);
+                        } else {  // (the first to write the last 32 columns)
+                            tc::mma(d + 32, mid, bd, tc::instr_desc(128, 64), true);
+                            tc::mma(d + 96, mid, tc::desc_at(bd, 64 * 16), tc::instr_desc(128, 32), false);
+                        }
+                        tc::mma(d + 64, lo, bd, tc::instr_desc(128, 64), true);
                     }
                     tc::commit(&S.bar[n & 1]);
                 }
@@ -725,10 +762,11 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
         // 4 warps per 32 lanes: 8 of the 32 columns (4 modes) each
         const int lane_row = tid & 127, part = tid >> 7, row = i * 128 + lane_row;
         const uint32_t dl = d + ((uint32_t)(tid & 96) << 16) + 8 * part;
-        float q0[8], q1[8], q2[8];
+        float q0[8], q1[8], q2[8], q3[8];
         tc::tmem_ld8(dl, q0);
         tc::tmem_ld8(dl + 32, q1);
         tc::tmem_ld8(dl + 64, q2);
+        tc::tmem_ld8(dl + 96, q3);
         tc::tmem_ld_wait();
         tc::fence_before();
         worker_sync<MODES_WORKERS>();  // read everywhere before the next tile's products
@@ -737,10 +775,8 @@ __global__ void __launch_bounds__(MODES_WORKERS + 32, 1) k_fno_modes(ModesArgs a
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int k = 4 * part + j;
-                if (k < a.modes)
-                    a.part[(int64_t)k * a.rows + row] =
-                        make_float2((q0[2 * j] + (q1[2 * j] + q2[2 * j])) * f,
-                                    (q0[2 * j + 1] + (q1[2 * j + 1] + q2[2 * j + 1])) * f);
+                auto sum = [&](int e) { return fmaf(fmaf(fmaf(q3[e], tc::DOWN, q2[e]), tc::DOWN, q1[e]), tc::DOWN, q0[e]); };
+                if (k < a.modes) a.part[(int64_t)k * a.rows + row] = make_float2(sum(2 * j) * f, sum(2 * j + 1) * f);
             }
         }
     };

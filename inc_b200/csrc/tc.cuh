@@ -1,24 +1,32 @@
 // Fifth-generation tensor-core (tcgen05) helpers for FP32-accurate contractions.
 //
-// An FP32 operand is split into three bf16 pieces in fixed point: with a power of
-// two s >= max|x| of the operand's scale group (the elements that share one scale
-// along the contraction), x / s * 256 = hi + mid + lo, where hi is an integer of
-// magnitude <= 256, mid a multiple of 2^-9 of magnitude <= 1/2 and lo a multiple
-// of 2^-18 of magnitude <= 2^-10: all exact in bf16, the remainder at most 2^-19
-// (2^-27 of s).  Six of the nine piece products are accumulated (the dropped ones
-// are below 2^-27 of s_a s_b per term) in two FP32 accumulators: hi.hi alone, whose
-// partial sums are integers below 2^24 for up to 256 full-scale terms, so the
-// accumulator's truncation never acts on it; and the five others, 2^-9 smaller, on
-// which it acts at 2^-33.  The two are added once in FP32.  The result is a rounded
-// exact sum of products of 27-bit inputs; an FP32 fused multiply-add chain of the
-// same length rounds at every term.
+// An FP32 operand is split into three fp16 pieces.  With a power of two s >= max|x| of the
+// operand's scale group (the elements that share one scale along the contraction),
+//   x / s * 256 = hi + 2^-14 mid + 2^-28 lo:
+// hi is an integer of magnitude <= 256, mid the remainder (<= 1/2) rounded to fp16's 11 bits,
+// lo what mid leaves, rounded to 11 bits; the powers of two keep the lower pieces in fp16's
+// range.  An element x is represented to 2^-24 |x| (half a unit in the last place of FP32), whatever
+// its size beside the group's maximum, down to 2^-36 of it; below that to 2^-61 of the
+// maximum.  (Three bf16 pieces on the same grid, as these once were, keep 2^-27 of the maximum
+// above 1/512 of it and 16 bits below: an output whose terms are all small, such as one
+// fed by a channel of small activations, then lost up to 8 of FP32's 24 bits.)
 //
-// Operand tiles live in shared memory as [rows][K] bf16 in 8-row x 16-byte core
+// Eight of the nine piece products are accumulated, by order (the number of 2^-14): order 0 is
+// hi.hi alone, whose partial sums are integers below 2^24 for up to 256 full-scale terms, so
+// the accumulator's truncation never acts on it; order 1 hi.mid and mid.hi; order 2 hi.lo,
+// mid.mid and lo.hi; order 3 mid.lo and lo.mid.  The one left out, lo.lo, is below 2^-24 |a b|.
+// Truncation acts on the orders from 1 up, 2^-9 below order 0 for operands near their maxima
+// (2^-33 of the sum), and at FP32's level for operands so small that their hi is 0.  Orders
+// are kept in columns of their own, or gathered in one accumulator from the highest down
+// with its input scaled by 2^-14 at each step (mma_scaled).  Against an FP32 fused multiply-add
+// chain of the same length, which rounds at every term, the result is no further off.
+//
+// Operand tiles live in shared memory as [rows][K] fp16 in 8-row x 16-byte core
 // matrices without swizzle: element (r, k) at (k / 8) * plane + r * 16 + (k % 8) * 2
 // bytes, plane = rows * 16.  A row is 16 bytes from the next, so a tile shifted by
 // one row (a convolution tap) is the same tile with the start address moved by 16.
 #pragma once
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 
@@ -109,10 +117,10 @@ INC_DEV uint64_t smem_desc(uint32_t addr, uint32_t lead, uint32_t stride) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lead >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((stride >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
-// FP32 accumulator, bf16 operands, M x N tile; a_mn / b_mn: operand stored MN-major
+// FP32 accumulator, fp16 operands, M x N tile; a_mn / b_mn: operand stored MN-major
 __host__ __device__ constexpr uint32_t instr_desc(int M, int N, bool a_mn = false, bool b_mn = false) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+    return (1u << 4) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
 }
 // the same tile `bytes` further on (a multiple of 16; within shared memory)
 INC_DEV uint64_t desc_at(uint64_t d, uint32_t bytes) { return d + (bytes >> 4); }
@@ -135,6 +143,14 @@ INC_DEV void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumu
         "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
+// D[tmem] = 2^-14 D + A B^T: the step from one order of the pieces' products to the one below it
+INC_DEV void mma_scaled(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.eq.b32 p, 0, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %4, %4}, p, 14;\n}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(0)
+        : "memory");
+}
 // arrives on `b` when every matrix instruction this thread issued has finished
 INC_DEV void commit(uint64_t* b) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
@@ -150,22 +166,27 @@ INC_DEV float pow2_above(float m) {
     return fminf(fmaxf(__uint_as_float(e), 7.888609052210118e-31f), 1.7014118346046923e38f);
 }
 
-// two values packed as bf16, rounded to nearest (a in the low half)
-INC_DEV uint32_t cvt_bf16x2(float a, float b) {
+// two values packed as fp16, rounded to nearest (a in the low half)
+INC_DEV uint32_t cvt_f16x2(float a, float b) {
     uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
     return r;
 }
+// The step between two orders of the pieces, 2^14 up and down
+constexpr float UP = 16384.f, DOWN = 1.f / 16384.f;
 // x * inv (a power of two, |x * inv| <= 256) of two values -> their pieces, packed.
 // The products inside the fused operations are exact.
 INC_DEV void split2(float2 x, float2 inv, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const float2 M = make_float2(12582912.f, 12582912.f), m1 = make_float2(-1.f, -1.f);  // 1.5 * 2^23: to integers
-    const float2 h = __fadd2_rn(__ffma2_rn(x, inv, M), make_float2(-M.x, -M.y));
-    const float2 r = __ffma2_rn(h, m1, __fmul2_rn(x, inv));
-    hi = __byte_perm(__float_as_uint(h.x), __float_as_uint(h.y), 0x7632);  // integers <= 256: exact
-    mid = cvt_bf16x2(r.x, r.y);
-    const float2 q = __ffma2_rn(make_float2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), m1, r);
-    lo = cvt_bf16x2(q.x, q.y);
+    constexpr float M = 12582912.f;  // 1.5 * 2^23: to integers
+    const float2 y = __fmul2_rn(x, make_float2(inv.x * UP, inv.y * UP));
+    const float2 t = __ffma2_rn(y, make_float2(DOWN, DOWN), make_float2(M, M));
+    const float2 h = make_float2(t.x - M, t.y - M);
+    hi = cvt_f16x2(h.x, h.y);  // integers <= 256: exact
+    const float2 r = __ffma2_rn(h, make_float2(-UP, -UP), y);
+    mid = cvt_f16x2(r.x, r.y);
+    const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&mid));
+    const float2 q = __ffma2_rn(m, make_float2(-UP, -UP), make_float2(r.x * UP, r.y * UP));
+    lo = cvt_f16x2(q.x, q.y);
 }
 // eight values -> 16 bytes of each piece
 INC_DEV void split8(const float (&x)[8], float inv, uint4& hi, uint4& mid, uint4& lo) {

@@ -1,0 +1,134 @@
+"""The tensor-core products keep FP32's accuracy whatever the sizes of the operands beside
+each other: channels whose activations are a power of two smaller and whose next layer's weights
+are as much larger, cells far from one large cell, and short rows.  Errors are against
+FP64 and are bounded by those of FP32 arithmetic on the same inputs (torch's layers, the
+layer-by-layer FNO, the replaying CNN backward).  Factors: 4 for one tensor or channel against
+another evaluation's, whose rounding scatters; 1.25 where errors are averaged over seeds."""
+import copy
+
+import pytest
+import torch
+
+from inc_b200 import fused
+from inc_b200.correctors import FNO1D, PeriodicCNN1D, fp64_copy
+from tests.test_fused_gpu import _params, _sim_params, _u0, fp32_convs  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _err(a, ref):
+    """Relative L2 error."""
+    a, ref = (torch.view_as_real(t) if t.is_complex() else t for t in (a.detach().cpu(), ref.detach().cpu()))
+    return ((a.double() - ref.double()).norm() / ref.double().norm().clamp_min(1e-300)).item()
+
+
+def _fno_errors(net, ref, u, gy, cuda, native):
+    """Errors of y, dL/du and every parameter's gradient; those of the layers next to the
+    rescaled channels are the worst over these channels."""
+    net = copy.deepcopy(net).to(cuda)
+    if not native:
+        net.conv1.register_forward_hook(lambda *a: None)  # a hooked layer: layer by layer
+    uc = u.float().to(cuda).requires_grad_(True)
+    y = net(uc)
+    assert ("FNOFn" in type(y.grad_fn).__name__) == native
+    y.backward(gy.float().to(cuda))
+    ur = u.clone().requires_grad_(True)
+    yr = ref(ur)
+    grads = torch.autograd.grad(yr, [ur] + list(ref.parameters()), gy)
+    out = dict(y=_err(y, yr), u=_err(uc.grad, grads[0]))
+    axis = {"fc1.weight": 1, "conv3.weights1": 1, "w3.weight": 0}
+    for (name, p), g in zip(net.named_parameters(), grads[1:]):
+        if name in axis:
+            out[name] = max(_err(a, b) for a, b in zip(p.grad.unbind(axis[name]), g.unbind(axis[name])))
+        else:
+            out[name] = _err(p.grad, g)
+    return out
+
+
+@pytest.mark.parametrize("width,e", [(64, 6), (64, 20), (32, 10)])
+def test_fno_channels_of_different_size(cuda, width, e):
+    """Every second channel between the last layer and fc1 2^-e times as large, its weights in
+    fc1 2^e times: no GELU stands between them, so the function is the same and an FP32
+    evaluation rounds the same."""
+    torch.manual_seed(width)
+    net = FNO1D(L=20.0, modes=12, width=width)
+    g = torch.Generator().manual_seed(e)
+    u, gy = (torch.randn(7, 256, generator=g, dtype=torch.float64) for _ in range(2))
+    fp32 = _fno_errors(net, fp64_copy(net), u, gy, cuda, native=False)
+    scale = 2.0 ** (-e * (torch.arange(width) % 2).float())
+    with torch.no_grad():
+        net.conv3.weights1 *= scale[None, :, None]
+        net.w3.weight *= scale[:, None, None]
+        net.w3.bias *= scale
+        net.fc1.weight /= scale
+    for name, err in _fno_errors(net, fp64_copy(net), u, gy, cuda, native=True).items():
+        assert err <= 4 * fp32[name], name
+
+
+def _corrections(net, u, N, cuda, steps=1, dt=None):
+    """The corrections of every step, [B, steps, N]."""
+    from inc_b200.solvers import BurgersSolverTorch
+    params = _sim_params(_params(N, B=u.shape[0]), u.shape[0], "euler", cuda)
+    params.dt = params.dt if dt is None else dt
+    return fused.burgers_cnn_rollout(net, BurgersSolverTorch(params), u, steps)[1]
+
+
+@pytest.mark.parametrize("e", [6, 20])
+def test_cnn_hidden_channels_of_different_size(cuda, e):
+    N = 128
+    torch.manual_seed(e)
+    net = PeriodicCNN1D()
+    scale = 2.0 ** (-e * (torch.arange(32) % 2).float())
+    with torch.no_grad():
+        net.convs[1].weight *= scale[:, None, None]
+        net.convs[1].bias *= scale
+        net.convs[2].weight /= scale[:, None]
+    u = torch.tensor(_u0(4, N, seed=e), dtype=torch.float32)
+    with torch.no_grad():
+        ref = copy.deepcopy(net).double()(u.double())
+        fp32 = _err(net(u), ref)
+        assert _err(_corrections(net.to(cuda), u.to(cuda), N, cuda)[:, 0], ref) <= 4 * fp32
+
+
+@pytest.mark.parametrize("N,size", [(64, 1e3), (256, 1e6), (512, 1e9)])
+def test_cnn_cells_far_from_a_large_one(cuda, N, size):
+    torch.manual_seed(N)
+    net = PeriodicCNN1D()
+    u = torch.tensor(_u0(3, N, seed=N), dtype=torch.float32)
+    u[:, 20] = size
+    with torch.no_grad():
+        ref = copy.deepcopy(net).double()(u.double())
+        fp32 = net(u)
+        got = _corrections(net.to(cuda), u.to(cuda), N, cuda)[:, 0]
+    far = torch.arange(N)[40:]  # beyond the receptive field of cell 20
+    assert _err(got[:, far], ref[:, far]) <= 4 * _err(fp32[:, far], ref[:, far])
+
+
+def _hidden_gradients(net, u, w, cuda, monkeypatch, record):
+    """(native, FP64) gradients of the hidden weights of sum(w * corrections), steps that leave the
+    state as it is (dt = 1e-30): each is the network's at u."""
+    ref = copy.deepcopy(net).double()
+    (ref(u.double())[:, None] * w.double()).sum().backward()
+    net = copy.deepcopy(net).to(cuda)
+    with monkeypatch.context() as m:
+        if not record:
+            m.setattr(fused, "ACTS_BYTES_MAX", 0)
+        c = _corrections(net, u.to(cuda), u.shape[1], cuda, w.shape[1], 1e-30)
+        (c * w.to(cuda)).sum().backward()
+    return [(net.convs[i].weight.grad, ref.convs[i].weight.grad) for i in (1, 2)]
+
+
+def test_cnn_hidden_weight_gradients_of_one_short_row(cuda, monkeypatch):
+    """Their operands are rounded no more coarsely than the replaying backward's."""
+    N, steps = 64, 4
+    total = {}
+    for seed in range(8):
+        torch.manual_seed(seed)
+        net = PeriodicCNN1D()
+        u = torch.tensor(_u0(1, N, seed=seed), dtype=torch.float32)
+        w = torch.randn(1, steps, N, generator=torch.Generator().manual_seed(seed))
+        for record in (True, False):
+            for i, (a, r) in enumerate(_hidden_gradients(net, u, w, cuda, monkeypatch, record)):
+                total[record, i] = total.get((record, i), 0.0) + _err(a, r) ** 2
+    for i in range(2):
+        assert total[True, i] <= 1.25 ** 2 * total[False, i], i
