@@ -8,7 +8,7 @@
 //                  first layers per thread from registers, the hidden layers' input
 //                  adjoints as convolutions with the transposed weights and reversed
 //                  taps on the tensor cores (burgers_cnn_tc.cuh).  dL/dz2 and dL/dz3 of every
-//                  step go to memory with their row maxima.  No replay: every u_k is
+//                  step go to memory with the channels' maxima.  No replay: every u_k is
 //                  recorded.  Bound by the chain of a step (the solver's adjoint, four row
 //                  reductions and products waited for; issue slots half used at 16 warps an
 //                  SM, all its registers taken): 865 us at 256 rows x 256 cells x 32 steps.
@@ -70,7 +70,7 @@ struct AdjArgs {
     const float* g_corr;   // [rows][steps][N] or NULL
     const float* acts;     // [rows][steps][2][32][N]
     float* dz;             // [rows][steps][2][32][N]: dL/dz2, dL/dz3
-    float* mx;             // [4][rows][steps]: max |dL/dz2|, |dL/dz3|, and bounds of |gelu(z1)|, |gelu(z2)|
+    float* mx;             // [4][rows][steps][32]: max over the cells of |dL/dz2|, |dL/dz3|, |gelu(z1)|, |gelu(z2)|
     float* edge;           // [blocks][EDGE]
 };
 
@@ -90,29 +90,34 @@ struct AdjSmem {
     };
     alignas(16) float w1[KW][C], b1[C], w4[KW][C];
     alignas(16) float u[Cfg::R][RL], d[Cfg::R][RL];
-    float red[2][2][Cfg::T / 32];
+    alignas(16) uint16_t cm[Cfg::T / 32][C];  // the warps' channel maxima, for layer 3 (bf16, which leaves two CTAs
+                                              // per SM room); layer 2's take d's place, which layer 4 has read by then
+    static_assert(Cfg::R * RL * sizeof(float) >= (Cfg::T / 32) * C * sizeof(uint16_t), "layer 2's channel maxima");
     uint64_t bar[Cfg::TILES];
     uint32_t tmem;
 };
 
-// max over the row of two non-negative values (one barrier; `fail` or-ed over the CTA)
+// max |v| over the warp (NaN left out)
+INC_DEV float warp_absmax(float v) {
+    float r;
+    asm("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+// the warp's max |v| of 4 channels, as bf16 rounded down
+INC_DEV void put_max4(uint16_t* out, float2 v0, float2 v1) {
+    uint32_t m0, m1;
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(m0) : "f"(warp_absmax(v0.y)), "f"(warp_absmax(v0.x)));
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(m1) : "f"(warp_absmax(v1.y)), "f"(warp_absmax(v1.x)));
+    if ((threadIdx.x & 31) == 0) *reinterpret_cast<uint2*>(out) = make_uint2(m0, m1);
+}
+// channel `lane`'s max over the warps of row rl (at least; at most 2^-7 above)
 template <int N>
-INC_DEV float2 row_max2(float a, float b, float (&red)[2][TcCfg<N>::T / 32], bool& fail, int rl) {
-    a = group_max_nonneg<32>(a);
-    b = group_max_nonneg<32>(b);
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = a;
-        red[1][threadIdx.x >> 5] = b;
-    }
-    fail = __syncthreads_or(fail);
+INC_DEV float channel_max(const uint16_t (*m)[C], int rl) {
     constexpr int WPR = TcCfg<N>::WARPS_PER_ROW;
-    a = b = 0.f;
+    uint32_t r = 0;
 #pragma unroll
-    for (int i = 0; i < WPR; ++i) {
-        a = fmaxf(a, red[0][rl * WPR + i]);
-        b = fmaxf(b, red[1][rl * WPR + i]);
-    }
-    return make_float2(a, b);
+    for (int i = 0; i < WPR; ++i) r = max(r, (uint32_t)m[rl * WPR + i][threadIdx.x & 31]);
+    return __uint_as_float(r << 16) * 1.0078125f;
 }
 
 template <int N>
@@ -140,8 +145,8 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
     }
     if (t < C) S.b1[t] = __ldg(c.w + OFF_B1 + t);
     float ws[2];
-    ws[0] = stage_weights<T, true>(S.w[0], c.w + OFF_W2, S.red[0][0]);
-    ws[1] = stage_weights<T, true>(S.w[1], c.w + OFF_W3, S.red[0][0]);
+    ws[0] = stage_weights<T, true>(S.w[0], c.w + OFF_W2, reinterpret_cast<float*>(S.cm));
+    ws[1] = stage_weights<T, true>(S.w[1], c.w + OFF_W3, reinterpret_cast<float*>(S.cm));
     tc::fence_smem();
     tc::fence_before();
     __syncthreads();
@@ -152,6 +157,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
     Ctx<1> cx;
     make_ctx<1, N>(a, src, g, true, cx);
     cx.has_s = true;
+    uint16_t(*cm[2])[C] = {reinterpret_cast<uint16_t(*)[C]>(S.d), S.cm};  // by layer: of dz, then of its activations
     int parity = 0;
     float g1[KW], g4[KW], gb1 = 0.f;  // this warp's cells, lane = channel
     double gb4 = 0.0;  // this cell's share of db4: one scalar, whose terms cancel
@@ -224,34 +230,34 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
 #pragma unroll
             for (int i = 0; i < C; ++i) z2[i] = __ldg(p + i * N);
         }
-        float m = 0.f, mz = 0.17f;  // |gelu(z)| <= max(z, 0.17)
+        auto put_mx = [&](int kind, float m) {
+            if (g < 32 && valid) c.mx[(((int64_t)kind * a.rows + row) * a.steps + k) * C + lane] = m;
+        };
 #pragma unroll
-        for (int i = 0; i < C; ++i) {
-            m = fmaxf(m, fabsf(v[i]));
-            mz = fmaxf(mz, z2[i]);
-        }
-        if (!valid) m = 0.f;
-        float2 rm = row_max2<N>(m, mz, S.red[0], fail, rl);  // (also: S.o.ch is read)
+        for (int i = 0; i < C; i += 4) put_max4(&cm[1][w][i], f2(v[i], v[i + 1]), f2(v[i + 2], v[i + 3]));
+        fail = __syncthreads_or(fail);  // (also: S.o.ch is read)
         if (fail) break;
-        if (g == 0 && valid) {
-            c.mx[((int64_t)1 * a.rows + row) * a.steps + k] = rm.x;
-            c.mx[((int64_t)3 * a.rows + row) * a.steps + k] = rm.y;
-        }
+        float m = channel_max<N>(cm[1], rl);
+        put_mx(1, m);
         if (valid) {
             float* p = acts_tile(c.dz, row, a.steps, k, 1, 0, N) + g;
 #pragma unroll
             for (int i = 0; i < C; ++i) p[i * N] = v[i];
         }
-        float f = adjoint_layer(v, 1, rm.x);
-        // gelu'(z2) while the products run
+        float f = adjoint_layer(v, 1, warp_absmax(m));
+        // gelu'(z2), and gelu(z2)'s maxima, while the products run
+        auto grad_and_max = [&](float(&z)[C], uint16_t(&out)[C]) {
 #pragma unroll
-        for (int i = 0; i < C; i += 2) {
-            const float2 gp = act::gelu_grad2(f2(z2[i], z2[i + 1]));
-            z2[i] = gp.x;
-            z2[i + 1] = gp.y;
-        }
+            for (int i = 0; i < C; i += 4) {
+                float2 y0, y1, g0, g1;
+                act::gelu_both2(f2(z[i], z[i + 1]), y0, g0);
+                act::gelu_both2(f2(z[i + 2], z[i + 3]), y1, g1);
+                put_max4(&out[i], y0, y1);
+                z[i] = g0.x; z[i + 1] = g0.y; z[i + 2] = g1.x; z[i + 3] = g1.y;
+            }
+        };
+        grad_and_max(z2, cm[1][w]);
         wait_layer();
-        m = 0.f;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float2 s[8];
@@ -261,7 +267,6 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
                 const int e = 16 * h + 2 * i;
                 v[e] = s[i].x * z2[e];
                 v[e + 1] = s[i].y * z2[e + 1];
-                m = fmaxf(m, fmaxf(fabsf(v[e]), fabsf(v[e + 1])));
             }
         }
         tc::fence_before();
@@ -269,12 +274,11 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
             float* p = acts_tile(c.dz, row, a.steps, k, 0, 0, N) + g;
 #pragma unroll
             for (int i = 0; i < C; ++i) p[i * N] = v[i];
-        } else {
-            m = 0.f;
         }
+#pragma unroll
+        for (int i = 0; i < C; i += 4) put_max4(&cm[0][w][i], f2(v[i], v[i + 1]), f2(v[i + 2], v[i + 3]));
         // ---- layer 2: dz1 = (W2^T dz2) gelu'(z1), z1 from u
         float z1[C];
-        mz = 0.17f;
         {
             float2 uu[KW];
 #pragma unroll
@@ -284,24 +288,17 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
                 float2 z = lds2(&S.b1[i]);
 #pragma unroll
                 for (int q = 0; q < KW; ++q) z = __ffma2_rn(*reinterpret_cast<const float2*>(&S.w1[q][i]), uu[q], z);
-                mz = fmaxf(mz, fmaxf(z.x, z.y));
                 z1[i] = z.x;
                 z1[i + 1] = z.y;
             }
         }
-        rm = row_max2<N>(m, mz, S.red[1], fail, rl);  // (also: the products have read the tile)
+        fail = __syncthreads_or(fail);  // (also: the products have read the tile)
         if (fail) break;
-        if (g == 0 && valid) {
-            c.mx[(int64_t)row * a.steps + k] = rm.x;
-            c.mx[((int64_t)2 * a.rows + row) * a.steps + k] = rm.y;
-        }
-        f = adjoint_layer(v, 0, rm.x);
-#pragma unroll
-        for (int i = 0; i < C; i += 2) {
-            const float2 gp = act::gelu_grad2(f2(z1[i], z1[i + 1]));
-            z1[i] = gp.x;
-            z1[i + 1] = gp.y;
-        }
+        m = channel_max<N>(cm[0], rl);
+        put_mx(0, m);
+        put_mx(3, channel_max<N>(cm[1], rl));
+        f = adjoint_layer(v, 0, warp_absmax(m));
+        grad_and_max(z1, cm[0][w]);
         wait_layer();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -317,6 +314,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         tc::fence_before();
         fail = __syncthreads_or(fail);  // (also: every tile's products have read the tile)
         if (fail) break;
+        put_mx(2, channel_max<N>(cm[0], rl));
         // ---- layer 1: dz1 by channel for dW1, db1; the input adjoint by tap
         {
             float2 q[KW];
@@ -387,8 +385,11 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
 
 // ---- hidden layers' weight gradients ---------------------------------------------------
 // A unit is 256 cells at one step (R rows of N <= 256 cells, or half a row of 512), a group
-// GROUP steps of the same cells: its products accumulate in tensor memory with one pair of
-// scales (the maxima over the group), then the sums are read once.  Lanes are (piece of dz,
+// GROUP steps of the same cells: its products accumulate in tensor memory with one scale per
+// channel of dz and of a (the channel's maximum over the group), then the sums are read once.
+// (A scale per group alone leaves a small channel's sums in the orders from 1 up, where the
+// accumulator truncates at each of the 64 instructions: 1.3e-6 of the channel's gradient
+// against 1.3e-7 in FP32.)  Lanes are (piece of dz,
 // co), columns (tap, piece of a, ci); the nine piece pairs are added in registers, each with its
 // order's power of two.  dz is scaled to 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
 // Even blocks take layer 2 (a = gelu(z1), z1 from the recorded state), odd ones layer 3.
@@ -424,6 +425,7 @@ struct CnnWgradSmem {
         alignas(128) unsigned char a[(3 * 4 + 2) * WgCfg<N>::PLANE];  // two planes of ones follow the pieces
     } buf[2];  // (dz's lanes past 96 read on into a: not used)
     alignas(16) float w1[KW][C], b1[C];
+    alignas(16) float up[2][2][C], down[2][2][C];  // by a group's parity, operand (dz, a), channel: scales, inverses
     uint64_t bar[2];
     uint32_t tmem;
 };
@@ -432,13 +434,17 @@ INC_DEV void wg_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 INC_DEV void wg_hand_over(int buf) { asm volatile("bar.arrive %0, 544;" ::"r"(2 + buf) : "memory"); }
 INC_DEV void wg_take_over(int buf) { asm volatile("bar.sync %0, 544;" ::"r"(2 + buf) : "memory"); }
 
-// 16 channels (half of the planes) of one slot
-INC_DEV void store_half(unsigned char* tile, int plane, const float2 (&v)[8], float inv, int slot, int half) {
+// 16 channels (half of the planes) of one slot; up: the channels' scales
+INC_DEV void store_half(unsigned char* tile, int plane, const float2 (&v)[8], const float* up, int slot, int half) {
 #pragma unroll
     for (int c8 = 0; c8 < 2; ++c8) {
         uint32_t h[4], m[4], l[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tc::split2(v[4 * c8 + j], f2s(inv), h[j], m[j], l[j]);
+        for (int j = 0; j < 4; j += 2) {
+            const float4 s = lds4(up + 16 * half + 8 * c8 + 2 * j);
+            tc::split2(v[4 * c8 + j], f2(s.x, s.y), h[j], m[j], l[j]);
+            tc::split2(v[4 * c8 + j + 1], f2(s.z, s.w), h[j + 1], m[j + 1], l[j + 1]);
+        }
         unsigned char* d = tile + (2 * half + c8) * plane + slot * 16;
         *reinterpret_cast<uint4*>(d) = make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4*>(d + 4 * plane) = make_uint4(m[0], m[1], m[2], m[3]);
@@ -518,7 +524,7 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
         for (int i = 0; i < 8; ++i) acc[k][i] = 0.f;
     bool fail = false;
     uint32_t used = 0;
-    float f_done = 0.f, fb_done = 0.f;  // scales of the group whose sums are still in tensor memory (0: none)
+    bool pending = false;  // a group's sums are still in tensor memory
     // the layer's input (half of the channels) at cell xa of a row and step
     auto input = [&](int row, int k, int xa, float2(&v)[8]) {
         if (layer == 1) {
@@ -556,13 +562,31 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
                                    : acts_tile(const_cast<float*>(a.acts), row, a.steps, k, 0, ch, N);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p + place % H * U + line * 32));
     };
-    auto drain = [&](int last) {  // the finished group's sums; `last`: the buffer of its last unit
+    // a group's scales, by 64 threads: the channels' maxima over the unit's rows and the group's steps
+    auto scales = [&](int gi, int par) {
+        if (tid >= 64 || gi >= groups) return;
+        const int op = tid >> 5, k0 = gi / places * GROUP, len = min(GROUP, a.steps - k0), first = gi % places / H * R;
+        float m = 0.f;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int j = 0; j < GROUP; ++j)
+                if (first + r < a.rows && j < len)
+                    m = fmaxf(m, __ldg(a.mx + (((int64_t)(2 * op + layer) * a.rows + first + r) * a.steps + k0 + j) * C +
+                                       (tid & 31)));
+        const float s = tc::pow2_above(m), full = op == 0 ? 64.f : 256.f;
+        S.up[par][op][tid & 31] = full / s;
+        S.down[par][op][tid & 31] = s / full;
+    };
+    // the finished group's sums; `last`: the buffer of its last unit; par: its parity
+    auto drain = [&](int last, int par) {
         if (!fail) fail = !tc::mbar_wait(&S.bar[last], (used >> last) & 1);
         tc::fence_after();
         // (every lane reads the same columns: loads under a branch cost a few hundred clocks each)
-        const float f = fail ? __int_as_float(0x7fffffff) : f_done;
         const float order = lane_q == 0 ? 1.f : (lane_q == 1 ? tc::DOWN : tc::DOWN * tc::DOWN);  // of dz's piece
-        const float f0 = f * order, f1 = f0 * tc::DOWN, f2 = f1 * tc::DOWN;
+        const float fd = (fail ? __int_as_float(0x7fffffff) : S.down[par][0][tid & 31]) * order;
+        const float4 fa0 = lds4(&S.down[par][1][8 * colq]), fa1 = lds4(&S.down[par][1][8 * colq + 4]);
+        const float f[8] = {fd * fa0.x, fd * fa0.y, fd * fa0.z, fd * fa0.w, fd * fa1.x, fd * fa1.y, fd * fa1.z, fd * fa1.w};
         const uint32_t dl = d + ((uint32_t)(tid & 96) << 16) + 8 * colq;
         float ones[8];
         tc::tmem_ld8(d + ((uint32_t)(tid & 96) << 16) + ONES, ones);
@@ -574,28 +598,20 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
             tc::tmem_ld8(dl + tap_col(k) + 64, q2);
             tc::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[k][i] += fmaf(q0[i], f0, fmaf(q1[i], f1, q2[i] * f2));
+            for (int i = 0; i < 8; ++i)
+                acc[k][i] = fmaf(fmaf(fmaf(q2[i], tc::DOWN, q1[i]), tc::DOWN, q0[i]), f[i], acc[k][i]);
         }
-        gb += ones[0] * ((fail ? f : fb_done) * order);
+        gb = fmaf(ones[0], fd, gb);
         tc::fence_before();
         wg_sync();  // read everywhere before the next group's products
     };
-    int n = 0;
-    for (int gi = me; gi < groups; gi += blocks) {
+    int n = 0, par = 0;
+    scales(me, 0);
+    for (int gi = me; gi < groups; gi += blocks, par ^= 1) {
+        wg_sync();  // this group's scales are there
         const int k0 = gi / places * GROUP, len = min(GROUP, a.steps - k0), place = gi % places;
         const int row = place / H * R + rl, x0 = place % H * U + x;
         const bool valid = row < a.rows;
-        float md = 0.f, ma = 0.f;  // over the unit's rows and the group's steps
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int rr = place / H * R + r;
-            if (rr < a.rows)
-                for (int j = 0; j < len; ++j) {
-                    md = fmaxf(md, __ldg(a.mx + ((int64_t)layer * a.rows + rr) * a.steps + k0 + j));
-                    ma = fmaxf(ma, __ldg(a.mx + ((int64_t)(2 + layer) * a.rows + rr) * a.steps + k0 + j));
-                }
-        }
-        const float sd = tc::pow2_above(md), sa = tc::pow2_above(ma);
         for (int j = 0; j < len; ++j, ++n) {
             const int buf = n & 1, k = k0 + j;
             if (n >= 2) {
@@ -612,29 +628,29 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
                     v[i].y = valid ? __ldg(p + (2 * i + 1) * N) : 0.f;
                 }
             }
-            store_half(S.buf[buf].dz, PL, v, 64.f / sd, slot, half);
+            store_half(S.buf[buf].dz, PL, v, S.up[par][0], slot, half);
             if (valid) {
                 input(row, k, x0, v);
             } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = f2s(0.f);
             }
-            store_half(S.buf[buf].a, PL, v, 256.f / sa, slot, half);
-            if (halo != 0) store_half(S.buf[buf].a, PL, v, 256.f / sa, slot + halo, half);
+            store_half(S.buf[buf].a, PL, v, S.up[par][1], slot, half);
+            if (halo != 0) store_half(S.buf[buf].a, PL, v, S.up[par][1], slot + halo, half);
             if (H > 1 && x < 4) {  // half a row: the neighbours' cells on either side
                 const int xh = x < 2 ? x - 2 : U + x - 2;
                 input(row, k, (place % H * U + xh + N) & (N - 1), v);
-                store_half(S.buf[buf].a, PL, v, 256.f / sa, xh + 2, half);
+                store_half(S.buf[buf].a, PL, v, S.up[par][1], xh + 2, half);
             }
             tc::fence_smem();
             tc::fence_before();
-            if (j == 0 && f_done != 0.f) drain(buf ^ 1);
+            if (j == 0 && pending) drain(buf ^ 1, par ^ 1);
             wg_hand_over(buf);
+            if (j == 0) scales(gi + blocks, par ^ 1);  // (the group before this one is read: its place is free)
         }
-        fb_done = sd * (1.f / 64.f);
-        f_done = fb_done * (sa * (1.f / 256.f));
+        pending = true;
     }
-    if (f_done != 0.f) drain((n - 1) & 1);
+    if (pending) drain((n - 1) & 1, par ^ 1);
     // the pieces of a lane's co added up, in the packed order [ci][co][k]
     float* s = reinterpret_cast<float*>(S.buf[0].dz);  // [3][32][161]; every product is done
     wg_sync();
@@ -698,7 +714,7 @@ struct BwdTcWork {
             return r;
         };
         dz = take(rows * steps * 2 * C * n);
-        mx = take(4 * rows * steps);
+        mx = take(4 * rows * steps * C);
         edge = take(rows * EDGE);
         part = take((int64_t)sm_count() * HID);
         total = at;
