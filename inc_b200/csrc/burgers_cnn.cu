@@ -40,7 +40,7 @@ struct FwdSmem {
             WideSmem<1, N> sh[Cfg::R];  // the solver's rows
         } o;
     };
-    float w1[KW][C], b[3][C], w4[KW][C];               // tap-major: channels contiguous
+    alignas(16) float w1[KW][C], b[3][C], w4[KW][C], ws[2][C];  // tap-major: channels contiguous
     float u[Cfg::R][N + 4];
     float red[2][Cfg::T / 32];
     uint64_t bar[Cfg::TILES];
@@ -75,9 +75,11 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
         S.b[1][t] = __ldg(wts + OFF_B2 + t);
         S.b[2][t] = __ldg(wts + OFF_B3 + t);
     }
-    float ws[2];
-    ws[0] = stage_weights<T, false>(S.w[0], wts + OFF_W2, S.red[0]);
-    ws[1] = stage_weights<T, false>(S.w[1], wts + OFF_W3, S.red[0]);
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const float s = stage_weights<T, false>(S.w[l], wts + (l == 0 ? OFF_W2 : OFF_W3));
+        if (t < C) S.ws[l][t] = s;
+    }
     const float b4 = __ldg(wts + OFF_B4);
     tc::fence_smem();
     tc::fence_before();
@@ -141,24 +143,24 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2)
             fail = !tc::mbar_wait(&S.bar[tile], phase);
             phase ^= 1;
             tc::fence_after();
-            const float f = s * (1.f / 256.f) * ws[l];
+            const float f = s * (1.f / 256.f);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float2 z[8];
-                read_layer16(acc, 16 * h, f, S.b[l + 1], z);
+            for (int c = 0; c < C; c += 8) {
+                float2 z[4];
+                read_layer8(acc, c, f, S.ws[l], S.b[l + 1], z);
                 if (acts && valid) {
-                    float* p = acts_tile(acts, row, a.steps, k, l, 16 * h, N) + g;
+                    float* p = acts_tile(acts, row, a.steps, k, l, c, N) + g;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         p[(int64_t)(2 * i) * N] = z[i].x;
                         p[(int64_t)(2 * i + 1) * N] = z[i].y;
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     const float2 y = act::gelu2(z[i]);
-                    v[16 * h + 2 * i] = y.x;
-                    v[16 * h + 2 * i + 1] = y.y;
+                    v[c + 2 * i] = y.x;
+                    v[c + 2 * i + 1] = y.y;
                 }
             }
             tc::fence_before();  // the accumulators are read before the next layer overwrites them

@@ -144,9 +144,9 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         S.w4[i / C][i % C] = __ldg(c.w + OFF_W4 + (i % C) * KW + i / C);
     }
     if (t < C) S.b1[t] = __ldg(c.w + OFF_B1 + t);
-    float ws[2];
-    ws[0] = stage_weights<T, true>(S.w[0], c.w + OFF_W2, reinterpret_cast<float*>(S.cm));
-    ws[1] = stage_weights<T, true>(S.w[1], c.w + OFF_W3, reinterpret_cast<float*>(S.cm));
+    float ws[2];  // the weight rows' scales, lane = channel
+    ws[0] = stage_weights<T, true>(S.w[0], c.w + OFF_W2);
+    ws[1] = stage_weights<T, true>(S.w[1], c.w + OFF_W3);
     tc::fence_smem();
     tc::fence_before();
     __syncthreads();
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
             issue_layer<N>(S.tmem + 128 * tile, S.act, S.w[l], tile);
             tc::commit(&S.bar[tile]);
         }
-        return s * (1.f / 256.f) * ws[l];
+        return s * (1.f / 256.f);
     };
     auto wait_layer = [&] {
         if (!fail) fail = !tc::mbar_wait(&S.bar[tile], phase);
@@ -245,28 +245,29 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
             for (int i = 0; i < C; ++i) p[i * N] = v[i];
         }
         float f = adjoint_layer(v, 1, warp_absmax(m));
-        // gelu'(z2), and gelu(z2)'s maxima, while the products run
-        auto grad_and_max = [&](float(&z)[C], uint16_t(&out)[C]) {
+        // gelu'(z2) times the weight rows' scales, and gelu(z2)'s maxima, while the products run
+        auto grad_and_max = [&](float(&z)[C], uint16_t(&out)[C], float scale) {
 #pragma unroll
             for (int i = 0; i < C; i += 4) {
                 float2 y0, y1, g0, g1;
                 act::gelu_both2(f2(z[i], z[i + 1]), y0, g0);
                 act::gelu_both2(f2(z[i + 2], z[i + 3]), y1, g1);
                 put_max4(&out[i], y0, y1);
+                g0 = __fmul2_rn(g0, f2(shfl<32>(scale, i), shfl<32>(scale, i + 1)));
+                g1 = __fmul2_rn(g1, f2(shfl<32>(scale, i + 2), shfl<32>(scale, i + 3)));
                 z[i] = g0.x; z[i + 1] = g0.y; z[i + 2] = g1.x; z[i + 3] = g1.y;
             }
         };
-        grad_and_max(z2, cm[1][w]);
+        grad_and_max(z2, cm[1][w], ws[1]);
         wait_layer();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float2 s[8];
-            read_sums16(acc, 16 * h, f, s);
+        for (int i = 0; i < C; i += 8) {
+            float2 s[4];
+            read_sums8(acc, i, f, s);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int e = 16 * h + 2 * i;
-                v[e] = s[i].x * z2[e];
-                v[e + 1] = s[i].y * z2[e + 1];
+            for (int e = 0; e < 4; ++e) {
+                v[i + 2 * e] = s[e].x * z2[i + 2 * e];
+                v[i + 2 * e + 1] = s[e].y * z2[i + 2 * e + 1];
             }
         }
         tc::fence_before();
@@ -298,17 +299,16 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         put_mx(0, m);
         put_mx(3, channel_max<N>(cm[1], rl));
         f = adjoint_layer(v, 0, warp_absmax(m));
-        grad_and_max(z1, cm[0][w]);
+        grad_and_max(z1, cm[0][w], ws[0]);
         wait_layer();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float2 s[8];
-            read_sums16(acc, 16 * h, f, s);
+        for (int i = 0; i < C; i += 8) {
+            float2 s[4];
+            read_sums8(acc, i, f, s);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int e = 16 * h + 2 * i;
-                v[e] = s[i].x * z1[e];
-                v[e + 1] = s[i].y * z1[e + 1];
+            for (int e = 0; e < 4; ++e) {
+                v[i + 2 * e] = s[e].x * z1[i + 2 * e];
+                v[i + 2 * e + 1] = s[e].y * z1[i + 2 * e + 1];
             }
         }
         tc::fence_before();

@@ -39,17 +39,23 @@ constexpr int W_PLANE = 96 * 16;
 
 // Packed FP32 weights of a hidden layer ([ci][co][k]) -> stacked pieces, tap-major:
 // tap k holds rows (piece, co), contraction ci.  TRANS: the layer's adjoint, rows
-// (piece, ci), contraction co, taps reversed.  Returns 2^e / 256 with 2^e >= max|w|.
+// (piece, ci), contraction co, taps reversed.  Each row has a scale of its own, so that
+// the products of a row of small weights lie in order 0 as well; returns 2^e / 256 with 2^e >=
+// the max |w| of row threadIdx.x % 32.  Three barriers; dst is scratch before the last.
 template <int T, bool TRANS>
-INC_DEV float stage_weights(unsigned char* dst, const float* __restrict__ w, float* red) {
+INC_DEV float stage_weights(unsigned char* dst, const float* __restrict__ w) {
+    const int row = threadIdx.x % C, warp = threadIdx.x / C;
+    float* part = reinterpret_cast<float*>(dst);
     float m = 0.f;
-    for (int i = threadIdx.x; i < C * C * KW; i += T) m = fmaxf(m, fabsf(__ldg(w + i)));
-    m = group_max_nonneg<32>(m);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    for (int c = warp; c < C; c += T / C)
+#pragma unroll
+        for (int k = 0; k < KW; ++k)
+            m = fmaxf(m, fabsf(__ldg(w + ((TRANS ? row : c) * C + (TRANS ? c : row)) * KW + k)));
+    part[threadIdx.x] = m;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < T / 32; ++i) m = fmaxf(m, red[i]);
-    __syncthreads();  // red is free again
+    for (int i = 0; i < T / C; ++i) m = fmaxf(m, part[i * C + row]);
+    __syncthreads();
     const float s = tc::pow2_above(m), inv = 256.f / s;
     // item: tap k, row r (the product's output channel), 8 contraction channels c8
     for (int i = threadIdx.x; i < KW * C * (C / 8); i += T) {
@@ -123,41 +129,38 @@ INC_DEV void issue_layer(uint32_t d, const unsigned char* act, const unsigned ch
     }
 }
 
-// 16 channels (c0 .. c0 + 15) of this thread's cell, the four orders added up
-INC_DEV void read_orders16(uint32_t d, int c0, float2 (&z)[8]) {
+// 8 channels (c0 .. c0 + 7) of this thread's cell, the four orders added up
+INC_DEV void read_orders8(uint32_t d, int c0, float2 (&z)[4]) {
     const float2 down = f2s(tc::DOWN);
-#pragma unroll
-    for (int h = 0; h < 16; h += 8) {
-        float v0[8], v1[8], v2[8], v3[8];
-        tc::tmem_ld8(d + c0 + h, v0);
-        tc::tmem_ld8(d + 32 + c0 + h, v1);
-        tc::tmem_ld8(d + 64 + c0 + h, v2);
-        tc::tmem_ld8(d + 96 + c0 + h, v3);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            const float2 s = __ffma2_rn(f2(v3[i], v3[i + 1]), down, f2(v2[i], v2[i + 1]));
-            z[(h + i) / 2] = __ffma2_rn(__ffma2_rn(s, down, f2(v1[i], v1[i + 1])), down, f2(v0[i], v0[i + 1]));
-        }
-    }
-}
-
-// the same times f, plus bias
-INC_DEV void read_layer16(uint32_t d, int c0, float f, const float* bias, float2 (&z)[8]) {
-    read_orders16(d, c0, z);
+    float v0[8], v1[8], v2[8], v3[8];
+    tc::tmem_ld8(d + c0, v0);
+    tc::tmem_ld8(d + 32 + c0, v1);
+    tc::tmem_ld8(d + 64 + c0, v2);
+    tc::tmem_ld8(d + 96 + c0, v3);
+    tc::tmem_ld_wait();
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
-        const float4 b = lds4(bias + c0 + 2 * i);
-        z[i] = __ffma2_rn(z[i], f2s(f), f2(b.x, b.y));
-        z[i + 1] = __ffma2_rn(z[i + 1], f2s(f), f2(b.z, b.w));
+        const float2 s = __ffma2_rn(f2(v3[i], v3[i + 1]), down, f2(v2[i], v2[i + 1]));
+        z[i / 2] = __ffma2_rn(__ffma2_rn(s, down, f2(v1[i], v1[i + 1])), down, f2(v0[i], v0[i + 1]));
     }
 }
 
-// the same without a bias
-INC_DEV void read_sums16(uint32_t d, int c0, float f, float2 (&z)[8]) {
-    read_orders16(d, c0, z);
+// the same times f and the weight rows' scales ws, plus bias
+INC_DEV void read_layer8(uint32_t d, int c0, float f, const float* ws, const float* bias, float2 (&z)[4]) {
+    read_orders8(d, c0, z);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) z[i] = __fmul2_rn(z[i], f2s(f));
+    for (int i = 0; i < 4; i += 2) {
+        const float4 b = lds4(bias + c0 + 2 * i), r = lds4(ws + c0 + 2 * i);
+        z[i] = __ffma2_rn(__fmul2_rn(z[i], f2(r.x, r.y)), f2s(f), f2(b.x, b.y));
+        z[i + 1] = __ffma2_rn(__fmul2_rn(z[i + 1], f2(r.z, r.w)), f2s(f), f2(b.z, b.w));
+    }
+}
+
+// the same times f alone
+INC_DEV void read_sums8(uint32_t d, int c0, float f, float2 (&z)[4]) {
+    read_orders8(d, c0, z);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[i] = __fmul2_rn(z[i], f2s(f));
 }
 
 // max |v| over this thread's channels and its row (a barrier of the CTA inside; fails

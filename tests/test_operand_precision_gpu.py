@@ -157,6 +157,27 @@ def test_cnn_hidden_weight_gradients_by_channel(cuda, monkeypatch, B, N, steps, 
         assert rms[True][i] <= 2 * rms[False][i], i
 
 
+def test_cnn_hidden_gradients_with_weight_rows_of_different_size(cuda, monkeypatch):
+    """The same scaling under a loss of one sign (truncation adds up over cells), each channel
+    on its own, averaged over seeds."""
+    N, e = 256, 12
+    scale = 2.0 ** (-e * (torch.arange(32) % 2).float())
+    total = {True: [0.0, 0.0], False: [0.0, 0.0]}
+    for seed in range(6):
+        torch.manual_seed(seed)
+        net = PeriodicCNN1D()
+        with torch.no_grad():
+            net.convs[1].weight *= scale[:, None, None]
+            net.convs[1].bias *= scale
+            net.convs[2].weight /= scale[:, None]
+        u = torch.tensor(_u0(4, N, seed=seed), dtype=torch.float32)
+        for record in (True, False):
+            for axis, (a, r) in enumerate(_hidden_gradients(net, u, torch.ones(4, 4, N), cuda, monkeypatch, record)):
+                total[record][axis] += sum(_err(a.select(axis, c), r.select(axis, c)) ** 2 for c in range(32))
+    for i in range(2):
+        assert total[True][i] <= 1.25 ** 2 * total[False][i], i
+
+
 def _one_channel(bias):
     """A network of channel 0 alone, centre taps of 1 (every sum is one value), `bias` before
     the second and third GELU."""
