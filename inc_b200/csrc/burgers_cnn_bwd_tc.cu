@@ -103,9 +103,12 @@ INC_DEV float warp_absmax(float v) {
     asm("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
-// the warp's max |v| of 4 channels, as bf16 rounded down
+// the warp's max |v| of 4 channels, of the finite values (x + 0 x: an infinite one to NaN), as
+// bf16 rounded down
 INC_DEV void put_max4(uint16_t* out, float2 v0, float2 v1) {
     uint32_t m0, m1;
+    v0 = __ffma2_rn(v0, f2s(0.f), v0);
+    v1 = __ffma2_rn(v1, f2s(0.f), v1);
     asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(m0) : "f"(warp_absmax(v0.y)), "f"(warp_absmax(v0.x)));
     asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(m1) : "f"(warp_absmax(v1.y)), "f"(warp_absmax(v1.x)));
     if ((threadIdx.x & 31) == 0) *reinterpret_cast<uint2*>(out) = make_uint2(m0, m1);
@@ -116,7 +119,10 @@ INC_DEV float channel_max(const uint16_t (*m)[C], int rl) {
     constexpr int WPR = TcCfg<N>::WARPS_PER_ROW;
     uint32_t r = 0;
 #pragma unroll
-    for (int i = 0; i < WPR; ++i) r = max(r, (uint32_t)m[rl * WPR + i][threadIdx.x & 31]);
+    for (int i = 0; i < WPR; ++i) {
+        const uint32_t e = m[rl * WPR + i][threadIdx.x & 31];
+        r = e < 0x7f80u ? max(r, e) : r;  // (a warp without a finite value has NaN)
+    }
     return __uint_as_float(r << 16) * 1.0078125f;
 }
 

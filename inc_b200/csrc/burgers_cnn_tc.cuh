@@ -163,14 +163,21 @@ INC_DEV void read_sums8(uint32_t d, int c0, float f, float2 (&z)[4]) {
     for (int i = 0; i < 4; ++i) z[i] = __fmul2_rn(z[i], f2s(f));
 }
 
-// max |v| over this thread's channels and its row (a barrier of the CTA inside; fails
-// is or-ed over the CTA)
+// max |v| over this thread's channels and its row, of the finite values: an infinite one or NaN
+// spoils the sums it enters, not the scale of the row's others (a barrier of the CTA inside;
+// fails is or-ed over the CTA)
 template <int N>
 INC_DEV float row_absmax(const float (&v)[C], float* red, bool& fail, int rl) {
     float m = 0.f;
 #pragma unroll
     for (int c = 0; c < C; ++c) m = fmaxf(m, fabsf(v[c]));
     m = group_max_nonneg<32>(m);
+    if (isinf(m)) {
+        m = 0.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c) m = fmaxf(m, isinf(v[c]) ? 0.f : fabsf(v[c]));
+        m = group_max_nonneg<32>(m);
+    }
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     fail = __syncthreads_or(fail);
     constexpr int WPR = TcCfg<N>::WARPS_PER_ROW;

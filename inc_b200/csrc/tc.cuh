@@ -160,10 +160,10 @@ INC_DEV void commit(uint64_t* b) {
 // ---- the three-piece split -----------------------------------------------------------
 // A power of two >= m (m >= 0): the scale s of a group with max|x| = m.  Groups below
 // 2^-100 use that (a product of two such groups is below FP32's smallest normal number);
-// above 2^127, and for a non-finite m, 2^127, so that 256 / s stays a normal number.
+// above 2^127, and for an infinite m or NaN, 2^127, so that 256 / s stays a normal number.
 INC_DEV float pow2_above(float m) {
-    const uint32_t e = (__float_as_uint(m) + 0x007FFFFFu) & 0x7F800000u;
-    return fminf(fmaxf(__uint_as_float(e), 7.888609052210118e-31f), 1.7014118346046923e38f);
+    const uint32_t e = (__float_as_uint(fminf(m, 1.7014118346046923e38f)) + 0x007FFFFFu) & 0x7F800000u;
+    return fmaxf(__uint_as_float(e), 7.888609052210118e-31f);
 }
 
 // two values packed as fp16, rounded to nearest (a in the low half)

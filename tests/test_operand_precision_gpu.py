@@ -208,3 +208,46 @@ def test_gelu_derivative_has_no_systematic_error(cuda):
         error = (u.grad.double() - exact)
         assert error.abs().max() < 2e-7
         assert abs(error.mean().item()) < (4e-9 if -2 <= k < 2 else 1e-8), k
+
+
+def test_cnn_overflow_before_a_gelu(cuda):
+    """GELU is infinite at +infinity, as 0.5 z (1 + erf(z / sqrt 2)) is: the third layer's input
+    overflows in cell 20, which the last layer passes on, and to its neighbours with weight 0."""
+    N = 128
+    net = _one_channel(0.0).to(cuda)
+    u = torch.zeros(2, N, device=cuda)
+    u[:, 20] = 1e38
+    want = torch.zeros(2, N)
+    want[:, 18:23] = float("nan")
+    want[:, 20] = float("inf")
+    with torch.no_grad():
+        net.convs[2].weight[0, 0, 2] = 10.0
+        got = _corrections(net, u, N, cuda, 1, 1e-30)[:, 0].cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    keep = ~torch.isnan(want)
+    assert torch.equal(got[keep], want[keep])
+
+
+@pytest.mark.parametrize("N", [64, 256, 512])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_cnn_non_finite_cell_leaves_the_others(cuda, N, bad):
+    """A non-finite cell of the state, and of the adjoint, leaves cells beyond its reach as they are."""
+    torch.manual_seed(N)
+    net = PeriodicCNN1D()
+    g = torch.Generator().manual_seed(N)
+    u = torch.tensor(_u0(3, N, seed=N), dtype=torch.float32)
+    w = torch.randn(3, 1, N, generator=g)
+    far = torch.arange(N)[40:]
+    uc = u.to(cuda).requires_grad_(True)
+    net = net.to(cuda)
+    (_corrections(net, uc, N, cuda, 1, 1e-30) * w.to(cuda)).sum().backward()
+    want, uc.grad = uc.grad[:, far].clone(), None
+    w[:, :, 20] = bad
+    (_corrections(net, uc, N, cuda, 1, 1e-30) * w.to(cuda)).sum().backward()
+    assert not torch.isfinite(uc.grad[:, 20]).any()
+    assert _err(uc.grad[:, far], want) < 1e-6
+    with torch.no_grad():
+        clean = _corrections(net, u.to(cuda), N, cuda, 1, 1e-30)[:, 0, far]
+        u[:, 20] = bad
+        got = _corrections(net, u.to(cuda), N, cuda, 1, 1e-30)[:, 0]
+    assert not torch.isfinite(got[:, 20]).any() and _err(got[:, far], clean) < 1e-6
