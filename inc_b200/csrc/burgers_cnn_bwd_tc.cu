@@ -60,7 +60,7 @@ INC_DEV void cell_products(float (&acc)[KW], const float* dr, const float* ar, i
     }
 }
 
-constexpr int EDGE = 2 * C * KW + C + 2;  // dW1, dW4, db1, db4 (high and low part) of one block
+constexpr int EDGE = 2 * C * KW + C + 3;  // dW1, dW4, db1, db4 (high and low part) of one block, 1 if it gave up
 constexpr int HID = C * C * KW + C;       // one hidden layer's dW and db
 
 struct AdjArgs {
@@ -346,8 +346,7 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         gu += du;
         __syncthreads();  // the solver's rows take this memory again
     }
-    const float nan = __int_as_float(0x7fffffff);
-    if (valid) a.g_u[(int64_t)row * N + g] = fail ? nan : gu;
+    if (valid) a.g_u[(int64_t)row * N + g] = fail ? __int_as_float(0x7fffffff) : gu;
     // this block's first- and last-layer gradients: one partial per warp, added in order
     __syncthreads();
     {
@@ -375,15 +374,16 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
         float* e = c.edge + (int64_t)blockIdx.x * EDGE;
 #pragma unroll
         for (int k = 0; k < KW; ++k) {
-            e[lane * KW + k] = fail ? nan : s[k];
+            e[lane * KW + k] = s[k];
             e[C * KW + lane * KW + k] = s[KW + k];
         }
         e[2 * C * KW + lane] = s[2 * KW];
         double b4 = 0.0;
         for (int q = 0; q < T / 32; ++q) b4 += (double)S.sums[q][0][2 * KW + 1] + S.sums[q][1][2 * KW + 1];
         if (lane == 0) {
-            e[2 * C * KW + C] = fail ? nan : (float)b4;
+            e[2 * C * KW + C] = (float)b4;
             e[2 * C * KW + C + 1] = (float)(b4 - (float)b4);
+            e[2 * C * KW + C + 2] = fail ? 1.f : 0.f;
         }
         tc::tmem_free(S.tmem, Cfg::COLS);
     }
@@ -680,7 +680,9 @@ __global__ void __launch_bounds__(WG + 32, 1) k_cnn_wgrad(CnnWgradArgs a) {
     __syncthreads();
 }
 
-// g[i] in the packed order from the blocks' partial sums, in FP64: 32 outputs x 32 slices per block
+// g[i] in the packed order from the blocks' partial sums, in FP64: 32 outputs x 32 slices per block.
+// All of them are NaN when an adjoint block gave up on a wait: the weight gradients have read
+// steps that it did not write.
 __global__ void __launch_bounds__(1024) k_cnn_grad_sum(const float* __restrict__ edge, int edges,
                                                        const float* __restrict__ hid, int hids, float* __restrict__ g) {
     __shared__ double s[32][33];
@@ -700,6 +702,8 @@ __global__ void __launch_bounds__(1024) k_cnn_grad_sum(const float* __restrict__
     for (int p = slice; p < count; p += 32) v += __ldg(src + p * stride);
     if (i == OFF_B4)
         for (int p = slice; p < count; p += 32) v += __ldg(src + 1 + p * stride);
+    for (int p = slice; p < edges; p += 32)
+        if (__ldg(edge + (int64_t)p * EDGE + 2 * C * KW + C + 2) != 0.f) v = __longlong_as_double(0x7ff8000000000000ll);
     s[slice][lane] = v;
     __syncthreads();
     if (threadIdx.x < 32 && i < W_FLOATS) {
