@@ -45,33 +45,51 @@ class BurgersRolloutFn(torch.autograd.Function):
         return g_u0, g_s, None, None, None, None
 
 
-# Largest tape (bytes) a checkpointed KS rollout takes in place of its checkpoints.  The tape's
-# backward has 9 row-pair transforms a step against 17 for replay and adjoint: forward and
-# backward of 512 x 512, 64 steps 574 -> 424 us (268 MB), 1024 x 256, 40 steps 352 -> 276 us,
-# 37 x 64, 40 steps 167 -> 122 us; no measured shape was slower.  Longer rollouts of large
-# batches keep the checkpoints, whose memory does not grow as fast (1 / (4 ckpt_every) of it).
+class _CkptDefault(int):
+    """ckpt_every that the caller left to the rollout."""
+
+
+CKPT_DEFAULT = _CkptDefault(8)
+# Largest tape (bytes) a KS rollout takes in place of the checkpoints that it would keep by
+# default.  The tape's backward has 9 row-pair transforms a step against 17 for replay and
+# adjoint: forward and backward of 512 x 512, 64 steps 574 -> 424 us (268 MB), 1024 x 256, 40
+# steps 352 -> 276 us, 37 x 64, 40 steps 167 -> 122 us; no measured shape was slower.  Longer
+# rollouts of large batches keep the checkpoints, whose memory does not grow as fast
+# (1 / (4 ckpt_every) of it).  A ckpt_every that the caller gives bounds the memory: then only
+# a tape too small to matter takes the checkpoints' place.
 KS_TAPE_BYTES_MAX = 1 << 30
+KS_TAPE_BYTES_SMALL = 16 << 20
 
 
 class KSRolloutFn(torch.autograd.Function):
     """ckpt_every > 0: checkpoints every ckpt_every steps, segments replayed in the
     backward, or a tape of every step's states (no replay, more memory) where that is at most
-    KS_TAPE_BYTES_MAX; ckpt_every == 0: the tape."""
+    KS_TAPE_BYTES_MAX (CKPT_DEFAULT) or KS_TAPE_BYTES_SMALL and there is room for it;
+    ckpt_every == 0: the tape."""
 
     @staticmethod
     def forward(ctx, u0, s, plan, steps, ckpt_every, want_grad):
         B, N = u0.shape
         frames = torch.empty(B, steps, N, device=u0.device, dtype=u0.dtype)
-        tape = want_grad and (ckpt_every == 0 or (ckpt_every > 0 and steps > 0
-                                                      and plan.tape_size(steps) <= KS_TAPE_BYTES_MAX))
-        if tape:
+        saved = None
+        if want_grad and ckpt_every == 0:
             saved = torch.empty(plan.tape_size(steps), dtype=torch.uint8, device=u0.device)
+        elif want_grad and ckpt_every > 0 and steps > 0:
+            most = KS_TAPE_BYTES_MAX if ckpt_every is CKPT_DEFAULT else min(KS_TAPE_BYTES_MAX, KS_TAPE_BYTES_SMALL)
+            size = plan.tape_size(steps)
+            if size <= most:
+                try:
+                    saved = torch.empty(size, dtype=torch.uint8, device=u0.device)
+                except torch.OutOfMemoryError:
+                    pass  # the checkpoints may still fit
+        tape = saved is not None
+        if tape:
             plan.rollout_tape(u0, s, steps, frames, None, saved)
         else:
-            k = ckpt_every if ckpt_every > 0 else 8
+            k = int(ckpt_every) if ckpt_every > 0 else 8
             saved = torch.empty(B, _nseg(steps, k), N, device=u0.device, dtype=u0.dtype) if want_grad else None
             plan.rollout(u0, s, steps, frames, None, k, saved)
-        ctx.plan, ctx.steps, ctx.k, ctx.has_s = plan, steps, (0 if tape else ckpt_every), s is not None
+        ctx.plan, ctx.steps, ctx.k, ctx.has_s = plan, steps, (0 if tape else int(ckpt_every)), s is not None
         ctx.shape = (B, N)
         if want_grad:
             ctx.save_for_backward(saved, s if s is not None else u0.new_empty(0))
@@ -111,13 +129,15 @@ def burgers_rollout(solver: BurgersSolverTorch, u0, steps, s=None, ckpt_every=8)
     return frames
 
 
-def ks_rollout(solver: KSSolverTorch, u0, steps, domain_size, s=None, ckpt_every=8):
+def ks_rollout(solver: KSSolverTorch, u0, steps, domain_size, s=None, ckpt_every=CKPT_DEFAULT):
     """Frames [B, steps, N] of `steps` KS step() calls in one launch (s held constant).
 
     Differentiable w.r.t. u0 and s.  The backward replays ckpt_every-step segments from
     checkpoints; ckpt_every=0 records every step's states in a tape instead (32 bytes per
-    row pair, cell and step) and the backward reads them, with no replay.  A tape of at most
-    KS_TAPE_BYTES_MAX is taken for any ckpt_every: the same gradients to rounding, faster."""
+    row pair, cell and step) and the backward reads them, with no replay.  Without a ckpt_every
+    the tape is taken up to KS_TAPE_BYTES_MAX, checkpoints every 8 steps above: the same gradients
+    to rounding, faster.  A given one bounds the memory: its checkpoints, or a tape of at most
+    KS_TAPE_BYTES_SMALL."""
     _check_state(u0, solver.resolution)
     u0 = u0.contiguous()
     s = _contig(s)
@@ -127,7 +147,8 @@ def ks_rollout(solver: KSSolverTorch, u0, steps, domain_size, s=None, ckpt_every
         return u0.unsqueeze(1).expand(0, int(steps), u0.shape[1]).clone()
     plan = solver.plan_for(u0, domain_size)
     want = torch.is_grad_enabled() and (u0.requires_grad or (s is not None and s.requires_grad))
-    return KSRolloutFn.apply(u0, s, plan, int(steps), int(ckpt_every), want)
+    k = ckpt_every if ckpt_every is CKPT_DEFAULT else int(ckpt_every)
+    return KSRolloutFn.apply(u0, s, plan, int(steps), k, want)
 
 
 def simulate_rollout(model, solver, u_initial, mstep, correction_term, L=None, checkpoint_every=None):
@@ -138,7 +159,8 @@ def simulate_rollout(model, solver, u_initial, mstep, correction_term, L=None, c
     solver.correction_s = None
     if correction_term is None:
         if isinstance(solver, KSSolverTorch) and solver.correction_u is None:
-            return ks_rollout(solver, u_initial, mstep, L), None
+            k = CKPT_DEFAULT if checkpoint_every is None else 8  # a caller who checkpoints bounds the memory
+            return ks_rollout(solver, u_initial, mstep, L, ckpt_every=k), None
         if isinstance(solver, BurgersSolverTorch) and solver.adaptive_CFL is None:
             return burgers_rollout(solver, u_initial, mstep), None
     elif correction_term != "INC":

@@ -422,3 +422,29 @@ def test_rollout_gradients_tape_in_place_of_checkpoints(cuda, monkeypatch, B, N,
             monkeypatch.undo()
         for a, b in zip(*got):
             assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
+
+
+def test_rollout_given_checkpoints_bound_the_memory(cuda):
+    """A caller's ckpt_every keeps its checkpoints where the tape would be large (34 MB here, 32 times
+    them); left to the rollout the tape is taken; simulate_rollout's checkpoint_every bounds it too."""
+    from inc_b200 import rollout as ro
+    B, N, steps = 128, 256, 64
+    ds = torch.full((B,), 56.0, device=cuda)
+    solver = _solver(N, 0.1, "ETRK2", [56.0] * B)
+    u = torch.rand(B, N, device=cuda, requires_grad=True)
+    solver.plan_for(u, ds)
+
+    def peak(call):
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated(cuda)
+        torch.cuda.reset_peak_memory_stats(cuda)
+        k = call().grad_fn.k
+        return k, torch.cuda.max_memory_allocated(cuda) - base
+
+    frames, tape = B * steps * N * 4, 16 * B * steps * N
+    k, used = peak(lambda: ro.ks_rollout(solver, u, steps, ds, ckpt_every=8))
+    assert k == 8 and used < frames + tape // 16
+    k, used = peak(lambda: ro.simulate_rollout(None, solver, u, steps, None, L=ds, checkpoint_every=4)[0])
+    assert k == 8 and used < frames + tape // 16
+    k, used = peak(lambda: ro.ks_rollout(solver, u, steps, ds))
+    assert k == 0 and used >= frames + tape
