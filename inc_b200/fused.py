@@ -6,7 +6,7 @@ u = solver.step(u); results[:, k] = u``) for a ``PeriodicCNN1D`` corrector in
 one launch of ``inc_burgers_cnn_rollout``: the four convolutions run from
 shared memory before every step, so no per-step corrector launches remain.
 With gradients on (rows of 64, 128, 256 or 512 cells), the rollout is one autograd node.
-While the hidden layers' pre-activations of every step fit ``ACTS_BYTES_MAX``, the
+While the hidden layers' pre-activations of every step, twice, fit ``ACTS_BYTES_MAX``, the
 forward records them and every state, and the backward is
 ``inc_burgers_cnn_rollout_bwd_states``: the solver's and the network's adjoint in
 reverse, then the weight gradients over all cells and steps, on the tensor cores,
@@ -68,10 +68,10 @@ def pack_cnn_weights(model, device=None) -> torch.Tensor:
 
 CNN_TRAIN_N = CNN_N
 MAX_CKPT_EVERY = 32
-# Largest record of the hidden layers' pre-activations the training path keeps (bytes):
-# 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps; the backward
-# takes as much again while it runs.  That training step is 1.85 ms with the record, 3.76 with
-# the replay (4.47 when the replay's forward ran on the FP32 pipes).
+# Largest memory (bytes) that the training path takes for the hidden layers' pre-activations: the
+# record, 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps, and as
+# much again for the layers' adjoints while the backward runs.  That training step is 1.99 ms
+# with the record, 3.80 with the replay (4.47 when the replay's forward ran on the FP32 pipes).
 ACTS_BYTES_MAX = 4 << 30
 
 
@@ -117,9 +117,10 @@ class BurgersCNNRolloutFn(torch.autograd.Function):
         frames = torch.empty(B, steps, N, device=u0.device, dtype=torch.float32)
         corr = torch.empty_like(frames)
         # the hidden layers' pre-activations and the state of every step, kept for the backward
-        # when they fit ACTS_BYTES_MAX (else the backward replays segments and recomputes them)
+        # when they and their adjoints fit ACTS_BYTES_MAX (else the backward replays segments and
+        # recomputes them)
         acts = None
-        if B * steps * 2 * 32 * N * 4 <= ACTS_BYTES_MAX:
+        if 2 * (B * steps * 2 * 32 * N * 4) <= ACTS_BYTES_MAX:
             acts = torch.empty(B, steps, 2, 32, N, device=u0.device, dtype=torch.float32)
             ckpt_every = 1
         nseg = (steps + ckpt_every - 1) // ckpt_every

@@ -403,3 +403,26 @@ def test_fused_training_last_bias_gradient(cuda, B, N, steps):
     loss.backward()
     g = torch.stack([c.grad for c in terms]).double()
     assert abs(got - g.sum().item()) < 64 * 2.0 ** -24 * g.square().sum().sqrt().item() * steps ** 0.5
+
+
+def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
+    """ACTS_BYTES_MAX bounds the record and what the backward adds to it: a rollout whose record alone
+    would fit (25 of 40 MB) is replayed, one of half its rows is recorded."""
+    from inc_b200 import fused
+    from inc_b200.solvers import BurgersSolverTorch
+    N, steps = 256, 24
+    monkeypatch.setattr(fused, "ACTS_BYTES_MAX", 40 * 10 ** 6)
+    for B, recorded in ((16, False), (8, True)):
+        net = _net(2).float().to(cuda)
+        solver = BurgersSolverTorch(_sim_params(_params(N, B=B), B, "ssprk3", cuda))
+        u0 = torch.tensor(_u0(B, N, seed=1), dtype=torch.float32, device=cuda, requires_grad=True)
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated(cuda)
+        torch.cuda.reset_peak_memory_stats(cuda)
+        f, _ = fused.burgers_cnn_rollout(net, solver, u0, steps)
+        record = B * steps * 2 * 32 * N * 4
+        assert (torch.cuda.memory_allocated(cuda) - base >= record) == recorded
+        f.sum().backward()
+        # beside them: frames, corrections, states and their adjoints, weight-gradient scratch
+        small = 6 * B * steps * N * 4 + 200 * 4 * fused.nat.INC_CNN_WEIGHT_FLOATS
+        assert torch.cuda.max_memory_allocated(cuda) - base < fused.ACTS_BYTES_MAX + small
