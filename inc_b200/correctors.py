@@ -301,20 +301,20 @@ class FNOFn(torch.autograd.Function):
         d = FNOFn._desc(u, grid, params)
         need = ctx.needs_input_grad
         gu = torch.empty_like(u) if need[0] else None
-        grads = [torch.empty_like(p) for p in params]
+        grads = [torch.empty_like(p) if wanted else None for p, wanted in zip(params, need[3:])]  # (frozen: None)
         g = nat.FNOGrads()
         g.u = nat.ptr(gu)
-        g.fc0_w, g.fc0_b = grads[0].data_ptr(), grads[1].data_ptr()
+        g.fc0_w, g.fc0_b = nat.ptr(grads[0]), nat.ptr(grads[1])
         for i in range(4):
-            g.modes_w[i], g.w[i], g.b[i] = (grads[j].data_ptr() for j in (2 + i, 6 + 2 * i, 7 + 2 * i))
-        g.fc1_w, g.fc1_b, g.fc2_w, g.fc2_b = (t.data_ptr() for t in grads[14:])
+            g.modes_w[i], g.w[i], g.b[i] = (nat.ptr(grads[j]) for j in (2 + i, 6 + 2 * i, 7 + 2 * i))
+        g.fc1_w, g.fc1_b, g.fc2_w, g.fc2_b = map(nat.ptr, grads[14:])
         lib = nat.lib()
         with nat.on_device(u.device):
             work = u.new_empty(lib.inc_fno_backward_work_size(C.byref(d)))
             rc = lib.inc_fno_backward(C.byref(d), u.data_ptr(), gy.data_ptr(), z.data_ptr(), xm.data_ptr(),
                                       tmax.data_ptr(), C.byref(g), work.data_ptr(), nat.stream_of(u.device))
         nat.check(rc, "inc_fno_backward")
-        return (gu, None, None) + tuple(t if need[3 + i] else None for i, t in enumerate(grads))
+        return (gu, None, None, *grads)
 
 
 class FNO1D(nn.Module):

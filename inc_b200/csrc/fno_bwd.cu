@@ -531,7 +531,7 @@ int run_wgrad(WgradArgs a, int* blocks, cudaStream_t st) {
 struct ModesGradArgs {
     const float2* x;  // [4][modes][batch][W]
     const float2* g;  // [4][modes][batch][W]
-    float2* out[4];   // [W][W][modes]
+    float2* out[4];   // [W][W][modes] (NULL: not wanted)
     int batch, modes, n;
 };
 template <int W>
@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(W * 4) k_fno_modes_grad(ModesGradArgs a) {
     constexpr int TB = 32, T = W * 4, LX = TB * W / T, LG = TB * 16 / T;
     __shared__ float2 X[TB][W], G[TB][16];
     const int k = blockIdx.x, l = blockIdx.y, o0 = blockIdx.z * 16;
+    if (!a.out[l]) return;
     const int64_t base = ((int64_t)l * a.modes + k) * a.batch * W;
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // o: tx; c: ty + i W / 4
     float2 rx[LX], rg[LG];
@@ -627,7 +628,8 @@ __global__ void __launch_bounds__(1024) k_fno_reduce(ReduceArgs a) {
 }
 
 // Layer 0 and the lift from the six sums per channel: s[0..2][o] = sum dL/dz {u, grid, 1},
-// s[3..5][c] = sum dL/dh {u, grid, 1}, with h[c] = w[c][0] u + w[c][1] grid + b[c].
+// s[3..5][c] = sum dL/dh {u, grid, 1}, with h[c] = w[c][0] u + w[c][1] grid + b[c].  Outputs
+// that are NULL are not wanted.
 template <int W>
 __global__ void __launch_bounds__(256) k_fno_lift_grad(const float* __restrict__ s, const float* __restrict__ w,
                                                        const float* __restrict__ bias, float* __restrict__ g_w0,
@@ -635,12 +637,14 @@ __global__ void __launch_bounds__(256) k_fno_lift_grad(const float* __restrict__
                                                        float* __restrict__ g_fc0_b) {
     for (int i = blockIdx.x * 256 + threadIdx.x; i < W * W; i += gridDim.x * 256) {
         const int o = i / W, c = i % W;
-        g_w0[i] = fmaf(w[2 * c], s[o], fmaf(w[2 * c + 1], s[W + o], bias[c] * s[2 * W + o]));
+        if (g_w0) g_w0[i] = fmaf(w[2 * c], s[o], fmaf(w[2 * c + 1], s[W + o], bias[c] * s[2 * W + o]));
         if (c == 0) {
-            g_b0[o] = s[2 * W + o];
-            g_fc0_w[2 * o] = s[3 * W + o];
-            g_fc0_w[2 * o + 1] = s[4 * W + o];
-            g_fc0_b[o] = s[5 * W + o];
+            if (g_b0) g_b0[o] = s[2 * W + o];
+            if (g_fc0_w) {
+                g_fc0_w[2 * o] = s[3 * W + o];
+                g_fc0_w[2 * o + 1] = s[4 * W + o];
+            }
+            if (g_fc0_b) g_fc0_b[o] = s[5 * W + o];
         }
     }
 }
@@ -702,6 +706,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
     if (rc) return rc;
     ReduceArgs ra{};
     auto job = [&](const float* src, float* dst, int stride, int count, int len) {
+        if (!dst) return;
         const int j = ra.jobs++;
         ra.src[j] = src;
         ra.dst[j] = dst;
@@ -725,19 +730,33 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
         job(work + o.sums + 128, gr->fc2_b, 132, blocks, 1);
         float* part = work + o.part;
         float* rows = work + o.rows;
-        rc = run_wgrad<128, W>(WgradArgs{work + o.g1, work + o.g1max, z + 3 * state, tmax + 3 * nq * B, part, rows, B, n, 0}, &blocks, st);
-        if (rc) return rc;
-        job(part, gr->fc1_w, 128 * W, blocks, 128 * W);
-        job(rows, gr->fc1_b, 128, blocks, 128);
+        if (gr->fc1_w || gr->fc1_b) {
+            rc = run_wgrad<128, W>(WgradArgs{work + o.g1, work + o.g1max, z + 3 * state, tmax + 3 * nq * B, part, rows, B, n, 0}, &blocks, st);
+            if (rc) return rc;
+            job(part, gr->fc1_w, 128 * W, blocks, 128 * W);
+            job(rows, gr->fc1_b, 128, blocks, 128);
+        }
     }
-    for (int l = 3; l >= 0; --l) {
+    // only what is asked for: the lift's gradients and layer 0's come from its adjoint's sums; the
+    // chain of adjoints ends at the lowest layer that something asks of
+    const bool lift = gr->u || gr->w[0] || gr->b[0] || gr->fc0_w || gr->fc0_b;
+    int lowest = 0;
+    while (lowest < 4 && !(lowest == 0 && lift) && !gr->modes_w[lowest] && !gr->w[lowest] && !gr->b[lowest]) ++lowest;
+    bool modes_wanted = false;
+    for (int l = 0; l < 4; ++l) modes_wanted = modes_wanted || gr->modes_w[l];
+    for (int l = 3; l >= lowest; --l) {
+        const bool on = l > lowest || (l == 0 && lift);  // the adjoint goes on below this layer
         const float* g = gz + (l & 1) * state;
         const float* gmx = gzmax + (l & 1) * nq * B;
-        rc = run_modes<W, false>(ModesArgs{g, gmx, prep->transform, gm + l * modes, B * W, B, M}, n, st);
-        if (rc) return rc;
-        rc = run_mix<W>(gm + l * modes, wt + (int64_t)l * M * W * W, mixed, work + o.mmax + l * B, B, n, M, st);
-        if (rc) return rc;
-        if (l > 0) {
+        if (on || gr->modes_w[l]) {
+            rc = run_modes<W, false>(ModesArgs{g, gmx, prep->transform, gm + l * modes, B * W, B, M}, n, st);
+            if (rc) return rc;
+        }
+        if (on) {
+            rc = run_mix<W>(gm + l * modes, wt + (int64_t)l * M * W * W, mixed, work + o.mmax + l * B, B, n, M, st);
+            if (rc) return rc;
+        }
+        if (l > 0 && (gr->w[l] || gr->b[l])) {
             float* part = work + o.part + most * (128 * W + (l - 1) * W * W);
             float* rows = work + o.rows + most * (128 + (l - 1) * W);
             rc = run_wgrad<W, W>(WgradArgs{g, gmx, z + (l - 1) * state, tmax + (int64_t)(l - 1) * nq * B, part, rows, B, n,
@@ -746,6 +765,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
             job(part, gr->w[l], W * W, blocks, W * W);
             job(rows, gr->b[l], W, blocks, W);
         }
+        if (!on) break;
         LayerArgs a{};
         a.x = g;
         a.xmax = gmx;
@@ -773,10 +793,12 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
         }
         if (rc) return rc;
     }
-    job(work + o.six + 6 * W, work + o.six, 6 * W, tile_grid(B, nq), 6 * W);
-    k_fno_reduce<<<ra.first[ra.jobs], 1024, 0, st>>>(ra);
-    k_fno_lift_grad<W><<<W * W / 256, 256, 0, st>>>(work + o.six, d->fc0_w, d->fc0_b, gr->w[0], gr->b[0], gr->fc0_w,
-                                                   gr->fc0_b);
+    const bool six = gr->w[0] || gr->b[0] || gr->fc0_w || gr->fc0_b;
+    if (six) job(work + o.six + 6 * W, work + o.six, 6 * W, tile_grid(B, nq), 6 * W);
+    if (ra.jobs) k_fno_reduce<<<ra.first[ra.jobs], 1024, 0, st>>>(ra);
+    if (six)
+        k_fno_lift_grad<W><<<W * W / 256, 256, 0, st>>>(work + o.six, d->fc0_w, d->fc0_b, gr->w[0], gr->b[0], gr->fc0_w,
+                                                       gr->fc0_b);
     ModesGradArgs mg{};
     mg.x = reinterpret_cast<const float2*>(xm);
     mg.g = gm;
@@ -784,7 +806,7 @@ int run_backward(const inc_fno_desc* d, const float* u, const float* g_y, const 
     mg.batch = B;
     mg.modes = M;
     mg.n = n;
-    k_fno_modes_grad<W><<<dim3(M, 4, W / 16), W * 4, 0, st>>>(mg);
+    if (modes_wanted) k_fno_modes_grad<W><<<dim3(M, 4, W / 16), W * 4, 0, st>>>(mg);
     return check_launch("fno gradients");
 }
 
@@ -805,10 +827,8 @@ extern "C" int inc_fno_backward(const inc_fno_desc* d, const float* u, const flo
     const int rc = fno::check_fno(d);
     if (rc) return rc;
     bool ok = u && g_y && z && x_modes && tmax && g && work && (reinterpret_cast<uintptr_t>(work) & 15u) == 0 &&
-              (reinterpret_cast<uintptr_t>(z) & 15u) == 0 &&
-              g->fc0_w && g->fc0_b && g->fc1_w && g->fc1_b && g->fc2_w && g->fc2_b;
-    for (int l = 0; ok && l < 4; ++l)
-        ok = g->modes_w[l] && g->w[l] && g->b[l] && (reinterpret_cast<uintptr_t>(g->modes_w[l]) & 7u) == 0;
+              (reinterpret_cast<uintptr_t>(z) & 15u) == 0;
+    for (int l = 0; ok && l < 4; ++l) ok = (reinterpret_cast<uintptr_t>(g->modes_w[l]) & 7u) == 0;
     if (!ok) {
         set_error("fno_backward: bad arguments");
         return INC_E_INVALID;

@@ -436,10 +436,10 @@ int64_t inc_fno_work_size(const inc_fno_desc* d, int32_t train);
 int inc_fno_forward(const inc_fno_desc* d, const float* u, float* y, float* z, float* x_modes,
                     float* tmax, float* work, void* stream);
 
-/* Its backward: the gradients of every parameter (torch's layouts; complex ones in
- * torch's convention) and, when u is not NULL, of u, from g_y [rows][n] and what the
- * forward recorded.  work: inc_fno_backward_work_size floats (for the current
- * device); z and work 16-byte aligned.                                          */
+/* Its backward: the gradients of the parameters (torch's layouts; complex ones in
+ * torch's convention) and of u, from g_y [rows][n] and what the forward recorded.  A
+ * NULL gradient is not wanted, and the work for it is left out.  work:
+ * inc_fno_backward_work_size floats (for the current device); z and work 16-byte aligned. */
 typedef struct inc_fno_grads {
     float* u;
     float* fc0_w;

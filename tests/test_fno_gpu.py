@@ -136,3 +136,38 @@ def test_fno_pending_conjugation_is_not_read_raw(cuda):
     net = FNO1D(L=16.0, modes=8, width=32).to(cuda)
     net.conv1.weights1 = torch.nn.Parameter(net.conv1.weights1.detach().conj())
     assert net.conv1.weights1.is_conj() and not net._fused(torch.randn(2, 64, device=cuda), 16.0)
+
+
+@pytest.mark.parametrize("wanted", ["u", "fc2.bias", "fc1.bias", "conv3.weights1", "w3.bias", "conv1.weights1",
+                                    "w1.weight", "conv0.weights1", "w0.weight", "fc0.bias"])
+def test_fno_backward_leaves_out_what_is_frozen(cuda, monkeypatch, wanted):
+    """With one gradient asked for, the backward is given that one alone (NULL for the others,
+    whose kernels it leaves out) and its bits are those of the full backward."""
+    from inc_b200 import _native as nat
+    net = _net(32, 8).to(cuda)
+    u = torch.randn(5, 128, generator=torch.Generator().manual_seed(3)).to(cuda).requires_grad_(True)
+    net(u).square().sum().backward()
+    full = dict({n: p.grad.clone() for n, p in net.named_parameters()}, u=u.grad.clone())
+    net.zero_grad()
+    u = u.detach().requires_grad_(wanted == "u")
+    for n, p in net.named_parameters():
+        p.requires_grad_(n == wanted)
+    given = []
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def inc_fno_backward(self, *args):
+            g = args[6]._obj
+            for field, _ in g._fields_:
+                v = getattr(g, field)
+                given.extend([v] if v is None or isinstance(v, int) else list(v))
+            return lib.inc_fno_backward(*args)
+
+    lib = nat.lib()
+    monkeypatch.setattr(nat, "lib", lambda: Lib())
+    net(u).square().sum().backward()
+    assert sum(v is not None for v in given) == 1 and len(given) == 19
+    got = u.grad if wanted == "u" else dict(net.named_parameters())[wanted].grad
+    assert torch.equal(got, full[wanted])
