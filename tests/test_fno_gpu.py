@@ -171,3 +171,86 @@ def test_fno_backward_leaves_out_what_is_frozen(cuda, monkeypatch, wanted):
     assert sum(v is not None for v in given) == 1 and len(given) == 19
     got = u.grad if wanted == "u" else dict(net.named_parameters())[wanted].grad
     assert torch.equal(got, full[wanted])
+
+
+def _ks(B, n, cuda):
+    from types import SimpleNamespace
+
+    from inc_b200.solvers import KSSolverTorch
+    L = torch.linspace(0.2, 0.3, B).mul(n).to(cuda)
+    return KSSolverTorch(SimpleNamespace(resolution=n, dt=0.1, device=cuda, domain_size=L,
+                                         alpha=torch.zeros(B, device=cuda), time_scheme="ETRK2")), L
+
+
+@pytest.mark.parametrize("checkpoint_every", [None, 2])
+def test_fno_in_the_ks_loop(cuda, monkeypatch, checkpoint_every):
+    """simulate_rollout's unrolled training step through FNOFn (each row its own domain size, every
+    parameter used at every step) against the same loop layer by layer."""
+    from inc_b200 import correctors
+    from inc_b200.rollout import simulate_rollout
+    B, n, steps = 5, 128, 4
+    g = torch.Generator().manual_seed(4)
+    u0, target = torch.randn(B, n, generator=g).to(cuda), torch.randn(B, steps, n, generator=g).to(cuda)
+    calls = []
+    apply = correctors.FNOFn.apply
+    monkeypatch.setattr(correctors.FNOFn, "apply", lambda *a: (calls.append(1), apply(*a))[1])
+    got = []
+    for native in (True, False):
+        net = _net(32, 8).to(cuda)
+        if not native:
+            net.conv2.register_forward_hook(lambda *a: None)
+        solver, L = _ks(B, n, cuda)
+        u = u0.clone().requires_grad_(True)
+        del calls[:]
+        frames, corrections = simulate_rollout(net, solver, u, steps, "INC", L=L, checkpoint_every=checkpoint_every)
+        (((frames - target) ** 2).mean() + corrections.square().mean()).backward()
+        assert len(calls) == (0 if not native else steps if checkpoint_every is None else 2 * steps)
+        got.append([frames, corrections, u.grad] + [p.grad for p in net.parameters()])
+    for a, b in zip(*got):
+        assert _rel(a, b.detach().to(torch.complex128 if b.is_complex() else torch.float64)) < 1e-5
+
+
+def test_fno_training_step_in_a_graph(cuda):
+    """Forward and backward captured in one CUDA graph and replayed for new states: the eager bits."""
+    net = _net(64, 16).to(cuda)
+    g = torch.Generator().manual_seed(5)
+    states = [torch.randn(7, 256, generator=g).to(cuda) for _ in range(2)]
+    static = states[0].clone()
+    params = list(net.parameters())
+
+    def step(u):
+        y = net(u)
+        assert _fused(y)
+        return [y.detach()] + list(torch.autograd.grad(y.square().mean(), params))
+
+    side = torch.cuda.Stream(cuda)
+    side.wait_stream(torch.cuda.current_stream(cuda))
+    with torch.cuda.stream(side):
+        step(static)
+    torch.cuda.current_stream(cuda).wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step(static)
+    for u in (states[1], states[0]):
+        static.copy_(u)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(out, step(u)):
+            assert torch.equal(a, b)
+
+
+def test_fno_evaluation_in_a_graphed_rollout(cuda):
+    from inc_b200.graphs import GraphedRollout
+    from inc_b200.rollout import simulate_rollout
+    B, n, steps = 6, 64, 5
+    net = _net(32, 8).to(cuda)
+    g = torch.Generator().manual_seed(6)
+    a, b = (torch.randn(B, n, generator=g).to(cuda) for _ in range(2))
+    solver, L = _ks(B, n, cuda)
+    assert net._fused(a, L)
+    replay = GraphedRollout(net, solver, a, steps, domain_size=L)
+    for u in (b, a):
+        frames, corrections = replay(u)
+        with torch.no_grad():
+            want = simulate_rollout(net, _ks(B, n, cuda)[0], u, steps, "INC", L=L)
+        assert torch.equal(frames, want[0]) and torch.equal(corrections, want[1])

@@ -251,3 +251,17 @@ def test_cnn_non_finite_cell_leaves_the_others(cuda, N, bad):
         u[:, 20] = bad
         got = _corrections(net, u.to(cuda), N, cuda, 1, 1e-30)[:, 0]
     assert not torch.isfinite(got[:, 20]).any() and _err(got[:, far], clean) < 1e-6
+
+
+@pytest.mark.parametrize("B,n", [(600, 512), (1200, 256), (592, 512)])
+def test_fno_gradients_of_large_batches(cuda, B, n):
+    """Past 16 SM counts of tiles the weight gradients take whole rows at a time (592 rows of 512 on 148
+    SMs are the last that do not): sums of up to 512 full-scale terms in the accumulators."""
+    torch.manual_seed(B)
+    net = FNO1D(L=20.0, modes=16, width=32)
+    g = torch.Generator().manual_seed(n)
+    u, gy = (torch.randn(B, n, generator=g, dtype=torch.float64).to(cuda) for _ in range(2))
+    ref = fp64_copy(net).to(cuda)
+    fp32 = _fno_errors(net, ref, u, gy, cuda, native=False)
+    for name, err in _fno_errors(net, ref, u, gy, cuda, native=True).items():
+        assert err <= 4 * fp32[name], name
