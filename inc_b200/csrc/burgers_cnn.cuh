@@ -1,8 +1,8 @@
 // Periodic CNN corrector (PeriodicCNN1D: Conv1d 1 -> 32 -> 32 -> 32 -> 1,
-// kernel 5, circular padding 2, erf GELU between layers) evaluated from shared
-// memory inside the Burgers rollout kernels: constants, the packed weight
-// layout, the activation row layout and the convolution stages shared by the
-// forward rollout (burgers_cnn.cu) and its backward (burgers_cnn_bwd.cu).
+// kernel 5, circular padding 2, erf GELU between layers) inside the Burgers rollout
+// kernels: constants, the packed weight layout, the layouts of the activation rows and of
+// the forward's record (burgers_cnn.cu, burgers_cnn_bwd_tc.cu), and the convolution stages
+// on the FP32 pipes of the replaying backward (burgers_cnn_bwd.cu).
 // torch's Conv1d is a cross-correlation:
 //   out[co][x] = b[co] + sum_ci sum_k W[co][ci][k] in[ci][(x + k - 2) mod N].
 #pragma once
@@ -28,7 +28,6 @@ constexpr int OFF_B3 = OFF_W3 + C * C * KW;
 constexpr int OFF_W4 = OFF_B3 + C;
 constexpr int OFF_B4 = OFF_W4 + C * KW;
 constexpr int W_FLOATS = OFF_B4 + 1;
-constexpr int W_SMEM = (W_FLOATS + 3) / 4 * 4;
 static_assert(INC_CNN_WEIGHT_FLOATS == W_FLOATS, "packed weight size");
 static_assert(OFF_W2 % 4 == 0 && OFF_W3 % 4 == 0 && OFF_B1 % 4 == 0 && OFF_B2 % 4 == 0 && OFF_B3 % 4 == 0,
               "float4 weight loads");
@@ -36,15 +35,6 @@ static_assert(OFF_W2 % 4 == 0 && OFF_W3 % 4 == 0 && OFF_B1 % 4 == 0 && OFF_B2 % 
 INC_DEV constexpr int apad(int p) { return p + ((p >> 5) << 2); }
 template <int N>
 INC_DEV constexpr int row_len() { return (apad(N + 3) + 1 + 3) / 4 * 4; }
-template <int N>
-INC_DEV constexpr int rows_per_cta() { return N >= 512 ? 1 : 512 / N; }
-
-template <int N>
-struct Smem {
-    float w[W_SMEM];
-    float act[2][rows_per_cta<N>()][C][row_len<N>()];
-    WideSmem<1, N> sh[rows_per_cta<N>()];
-};
 
 // torch.nn.functional.gelu, approximate='none'
 INC_DEV float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
@@ -176,16 +166,7 @@ INC_DEV float* acts_tile(float* acts, int64_t row, int steps, int k, int layer, 
     return acts + ((((row * steps + k) * 2 + layer) * C + ch) * (int64_t)n);
 }
 
-// this thread's 4-channel x 8-cell tile to / from the record (two float4 a channel)
-INC_DEV void put_acts(float* acts, int64_t row, int steps, int k, int layer, const float (&acc)[4][8], int cg,
-                      int L, int n) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float4* p = reinterpret_cast<float4*>(acts_tile(acts, row, steps, k, layer, 4 * cg + c, n) + 8 * L);
-        p[0] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
-        p[1] = make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
-    }
-}
+// this thread's 4-channel x 8-cell tile from the record (two float4 a channel)
 INC_DEV void get_acts(const float* __restrict__ acts, int64_t row, int steps, int k, int layer, float (&acc)[4][8],
                       int cg, int L, int n) {
 #pragma unroll
@@ -196,31 +177,6 @@ INC_DEV void get_acts(const float* __restrict__ acts, int64_t row, int steps, in
         acc[c][0] = v0.x; acc[c][1] = v0.y; acc[c][2] = v0.z; acc[c][3] = v0.w;
         acc[c][4] = v1.x; acc[c][5] = v1.y; acc[c][6] = v1.z; acc[c][7] = v1.w;
     }
-}
-
-// Layer 4: channels 4 cg .. 4 cg + 3 -> partial sums of the single output
-// channel, stored in row cg of `part` (the other buffer); no bias, no GELU.
-template <int N>
-INC_DEV void conv_last_partial(const float* w4, float (*in)[row_len<N>()], float (*part)[row_len<N>()], int cg,
-                               int L) {
-    float acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int ci = 4 * cg + c;
-        float a[12];
-        load12(a, in[ci], L);
-#pragma unroll
-        for (int k = 0; k < KW; ++k) {
-            const float wk = w4[ci * KW + k];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = fmaf(wk, a[j + k], acc[j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float2*>(part[cg] + apad(8 * L + 2 + 2 * i)) = make_float2(acc[2 * i], acc[2 * i + 1]);
 }
 
 }  // namespace cnn

@@ -181,13 +181,6 @@ INC_DEV void store_point(unsigned char* x, const float2 (&v)[C / 2], float inv, 
         *reinterpret_cast<uint4*>(d + 2 * (W / 8) * 2048) = make_uint4(l[0], l[1], l[2], l[3]);
     }
 }
-template <int C>
-INC_DEV float point_max(const float2 (&v)[C / 2]) {
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < C / 2; ++i) m = fmaxf(m, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
-    return m;
-}
 // A [128 x K] B[N x K]^T, one stage of it.  A: pieces of a point tile (planes of 2048 bytes,
 // pieces a_piece apart); B: stacked pieces [3 N][K].  The stages 3, 2, 1 leave order 0 in
 // columns d .. d + N - 1 and, in d + N .. d + 2N - 1, order 1 + 2^-14 (order 2 + 2^-14 order 3).  FIRST: the first

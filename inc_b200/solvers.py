@@ -153,7 +153,8 @@ class _BurgersLaunch:
 
     def cnn_rollout(self, weights, u0, steps, frames, corrections, u_final, ckpt_every=0, ckpts=None, acts=None):
         """The fused CNN-corrected rollout; with ``acts`` ([rows, steps, 2, 32, n] float32) it
-        also records the hidden layers' pre-activations for cnn_rollout_bwd."""
+        also records the hidden layers' pre-activations, for cnn_rollout_bwd_states (with
+        ckpt_every = 1) or cnn_rollout_bwd."""
         lib = nat.lib()
         args = (C.byref(self.desc), weights.data_ptr(), u0.data_ptr(), nat.ptr(self.t_rows), self.t0, steps,
                 nat.ptr(frames), nat.ptr(corrections), nat.ptr(u_final), int(ckpt_every), nat.ptr(ckpts))
@@ -166,7 +167,8 @@ class _BurgersLaunch:
 
     def cnn_rollout_bwd(self, weights, ckpts, corrections, steps, ckpt_every, g_frames, g_corrections, g_final,
                         g_u0, g_weights, work, acts=None):
-        """Its backward; ``acts`` (the forward's record) replaces recomputing z2 and z3."""
+        """Its backward by replay; ``acts`` (the forward's record) replaces recomputing z2 and z3
+        (segments of any length beside the record; cnn_rollout_bwd_states wants every state)."""
         lib = nat.lib()
         args = (C.byref(self.desc), weights.data_ptr(), ckpts.data_ptr(), corrections.data_ptr(),
                 nat.ptr(self.t_rows), self.t0, steps, ckpt_every, nat.ptr(g_frames), nat.ptr(g_corrections),

@@ -426,3 +426,34 @@ def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
         # beside them: frames, corrections, states and their adjoints, weight-gradient scratch
         small = 6 * B * steps * N * 4 + 200 * 4 * fused.nat.INC_CNN_WEIGHT_FLOATS
         assert torch.cuda.max_memory_allocated(cuda) - base < fused.ACTS_BYTES_MAX + small
+
+
+@pytest.mark.parametrize("N,B,K", [(64, 9, 4), (256, 5, 1), (512, 2, 8)])
+def test_replaying_backward_reads_the_record(cuda, N, B, K):
+    """inc_burgers_cnn_rollout_bwd_acts: the replaying backward with the forward's pre-activations in
+    place of recomputing them, against the same without and against the one that replays nothing."""
+    from inc_b200 import _native as nat
+    from inc_b200.fused import pack_cnn_weights
+    from inc_b200.solvers import BurgersSolverTorch
+    steps = 11
+    w = pack_cnn_weights(_net(3).float(), cuda)
+    u0 = torch.tensor(_u0(B, N, seed=14), dtype=torch.float32, device=cuda)
+    launch = BurgersSolverTorch(_sim_params(_params(N, B=B), B, "ssprk3", cuda)).launch_for(u0)
+    gen = torch.Generator().manual_seed(5)
+    gf, gc = (torch.randn(B, steps, N, generator=gen).to(cuda) for _ in range(2))
+    frames, corr = torch.empty_like(gf), torch.empty_like(gf)
+    acts = torch.empty(B, steps, 2, 32, N, device=cuda)
+    out = []
+    for every in (K, 1):
+        ck = torch.empty(B, (steps + every - 1) // every, N, device=cuda)
+        launch.cnn_rollout(w, u0, steps, frames, corr, None, every, ck, acts=acts)
+        for record in (acts, None):
+            gu, gw = torch.empty_like(u0), torch.empty_like(w)
+            if every == 1 and record is not None:
+                launch.cnn_rollout_bwd_states(w, ck, corr, steps, gf, gc, None, gu, gw, acts)
+            else:
+                work = torch.empty(B, nat.INC_CNN_WEIGHT_FLOATS, device=cuda)
+                launch.cnn_rollout_bwd(w, ck, corr, steps, every, gf, gc, None, gu, gw, work, acts=record)
+            out.append((gu.cpu().numpy(), gw.cpu().numpy()))
+    for gu, gw in out[1:]:
+        assert rel_l2(gu, out[0][0]) < 1e-5 and rel_l2(gw, out[0][1]) < 1e-5
