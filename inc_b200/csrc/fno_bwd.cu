@@ -827,7 +827,7 @@ extern "C" int inc_fno_backward(const inc_fno_desc* d, const float* u, const flo
     const int rc = fno::check_fno(d);
     if (rc) return rc;
     bool ok = u && g_y && z && x_modes && tmax && g && work && (reinterpret_cast<uintptr_t>(work) & 15u) == 0 &&
-              (reinterpret_cast<uintptr_t>(z) & 15u) == 0;
+              (reinterpret_cast<uintptr_t>(z) & 15u) == 0 && (reinterpret_cast<uintptr_t>(x_modes) & 7u) == 0;
     for (int l = 0; ok && l < 4; ++l) ok = (reinterpret_cast<uintptr_t>(g->modes_w[l]) & 7u) == 0;
     if (!ok) {
         set_error("fno_backward: bad arguments");

@@ -271,7 +271,8 @@ extern "C" int inc_fno_forward(const inc_fno_desc* d, const float* u, float* y, 
     const int rc = fno::check_fno(d);
     if (rc) return rc;
     if (!u || !y || !work || (z != nullptr) != (x_modes != nullptr) || (z != nullptr) != (tmax != nullptr) ||
-        (reinterpret_cast<uintptr_t>(work) & 15u) != 0 || (reinterpret_cast<uintptr_t>(x_modes) & 15u) != 0) {
+        (reinterpret_cast<uintptr_t>(work) & 15u) != 0 || (reinterpret_cast<uintptr_t>(x_modes) & 15u) != 0 ||
+        (reinterpret_cast<uintptr_t>(z) & 15u) != 0) {  // (read four values at a time)
         set_error("fno_forward: bad arguments");
         return INC_E_INVALID;
     }

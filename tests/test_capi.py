@@ -123,3 +123,66 @@ def test_new_entry_points_check_arguments_without_gpu(lib):
     assert lib.inc_ks_fft_rows(fake, fake, 4, 96, 1, None) == nat.INC_E_UNSUPPORTED
     p.npairs = 0
     assert lib.inc_ks_substep(C.byref(p), fake, None, fake, None) == nat.INC_E_INVALID
+
+
+def _fno_desc(nat, width=32, n=64, modes=8, rows=4):
+    d = nat.FNODesc()
+    d.rows, d.n, d.width, d.modes, d.grid_stride = rows, n, width, modes, n
+    for field in ("grid", "fc0_w", "fc0_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b"):
+        setattr(d, field, 4096)  # never dereferenced: every call below is rejected on the host
+    for i in range(4):
+        d.modes_w[i] = d.w[i] = d.b[i] = 4096
+    return d
+
+
+def test_fno_entry_points_check_arguments_without_gpu(lib):
+    from inc_b200 import _native as nat
+    ok, odd, call = C.c_void_p(4096), C.c_void_p(4100), nat.INC_E_INVALID
+    d = _fno_desc(nat)
+
+    def forward(d, u=ok, y=ok, z=ok, modes=ok, tmax=ok, work=ok):
+        return lib.inc_fno_forward(C.byref(d), u, y, z, modes, tmax, work, None)
+
+    def backward(d, u=ok, g_y=ok, z=ok, modes=ok, tmax=ok, grads=True, work=ok):
+        g = nat.FNOGrads()
+        g.modes_w[1] = 4096 if grads is True else grads
+        return lib.inc_fno_backward(C.byref(d), u, g_y, z, modes, tmax, C.byref(g) if grads else None, work, None)
+
+    for kw in (dict(u=None), dict(y=None), dict(work=None), dict(z=None), dict(modes=None), dict(tmax=None),
+               dict(work=odd), dict(modes=odd), dict(z=odd)):
+        assert forward(d, **kw) == call, kw
+    for kw in (dict(u=None), dict(g_y=None), dict(z=None), dict(modes=None), dict(tmax=None), dict(grads=False),
+               dict(work=None), dict(work=odd), dict(z=odd), dict(modes=odd), dict(grads=4100)):
+        assert backward(d, **kw) == call, kw
+    for field, bad in (("rows", 0), ("grid", None), ("fc1_w", None), ("grid_stride", -1)):
+        d = _fno_desc(nat)
+        setattr(d, field, bad)
+        assert forward(d) == call and backward(d) == call, field
+    d = _fno_desc(nat)
+    d.modes_w[2] = 4100  # complex: 8-byte aligned
+    assert forward(d) == call and backward(d) == call
+    for kw in (dict(width=48), dict(n=32), dict(n=96), dict(modes=0), dict(modes=17)):
+        d = _fno_desc(nat, **kw)
+        assert forward(d) == nat.INC_E_UNSUPPORTED and backward(d) == nat.INC_E_UNSUPPORTED
+        assert lib.inc_fno_work_size(C.byref(d), 1) == -1 and lib.inc_fno_backward_work_size(C.byref(d)) == -1
+
+
+def test_cnn_states_backward_checks_arguments_without_gpu(lib):
+    from inc_b200 import _native as nat
+    ok = C.c_void_p(4096)
+    d = nat.BurgersDesc()
+    d.rows, d.n, d.dx, d.dt, d.scheme = 2, 64, 0.1, 0.01, nat.INC_TS_SSPRK3
+
+    def call(n=64, steps=3, **none):
+        d.n = n
+        p = lambda name: None if name in none else ok  # noqa: E731
+        return lib.inc_burgers_cnn_rollout_bwd_states(
+            C.byref(d), p("weights"), p("states"), p("corrections"), None, 0.0, steps, ok, None, None, p("g_u0"),
+            p("g_weights"), p("acts"), p("work"), None)
+
+    for name in ("weights", "states", "corrections", "g_u0", "g_weights", "acts", "work"):
+        assert call(**{name: True}) == nat.INC_E_INVALID, name
+    assert call(steps=0) == nat.INC_E_INVALID
+    assert call(n=32) == nat.INC_E_UNSUPPORTED
+    size = lib.inc_burgers_cnn_rollout_bwd_states_work_size
+    assert size(2, 32, 3) == -1 and size(0, 64, 3) == -1 and size(2, 64, 0) == -1
