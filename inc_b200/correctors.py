@@ -28,6 +28,7 @@ import ctypes as C
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd.function import once_differentiable
 
 from . import _native as nat
 
@@ -295,6 +296,7 @@ class FNOFn(torch.autograd.Function):
         return y
 
     @staticmethod
+    @once_differentiable  # its gradients are kernels' outputs: a second derivative raises, not 0
     def backward(ctx, gy):
         u, grid, z, xm, tmax, *params = ctx.saved_tensors
         gy = gy.resolve_neg().contiguous()

@@ -254,3 +254,13 @@ def test_fno_evaluation_in_a_graphed_rollout(cuda):
         with torch.no_grad():
             want = simulate_rollout(net, _ks(B, n, cuda)[0], u, steps, "INC", L=L)
         assert torch.equal(frames, want[0]) and torch.equal(corrections, want[1])
+
+
+def test_fno_second_derivative_is_refused(cuda):
+    """A penalty on dL/du needs what the native backward does not record: an error, not a term that
+    silently contributes nothing."""
+    net = _net(32, 8).to(cuda)
+    u = torch.randn(2, 64, device=cuda, requires_grad=True)
+    (gu,) = torch.autograd.grad(net(u).square().sum(), u, create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        (net(u).square().sum() + gu.square().sum()).backward()
