@@ -412,7 +412,8 @@ def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
     from inc_b200.solvers import BurgersSolverTorch
     N, steps = 256, 24
     monkeypatch.setattr(fused, "ACTS_BYTES_MAX", 40 * 10 ** 6)
-    for B, recorded in ((16, False), (8, True)):
+
+    def step(B, recorded):
         net = _net(2).float().to(cuda)
         solver = BurgersSolverTorch(_sim_params(_params(N, B=B), B, "ssprk3", cuda))
         u0 = torch.tensor(_u0(B, N, seed=1), dtype=torch.float32, device=cuda, requires_grad=True)
@@ -420,12 +421,14 @@ def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
         base = torch.cuda.memory_allocated(cuda)
         torch.cuda.reset_peak_memory_stats(cuda)
         f, _ = fused.burgers_cnn_rollout(net, solver, u0, steps)
-        record = B * steps * 2 * 32 * N * 4
-        assert (torch.cuda.memory_allocated(cuda) - base >= record) == recorded
+        assert (f.grad_fn.saved_tensors[3] is not None) == recorded
         f.sum().backward()
-        # beside them: frames, corrections, states and their adjoints, weight-gradient scratch
+        # beside the bound: frames, corrections, states and their adjoints, weight-gradient scratch
         small = 6 * B * steps * N * 4 + 200 * 4 * fused.nat.INC_CNN_WEIGHT_FLOATS
         assert torch.cuda.max_memory_allocated(cuda) - base < fused.ACTS_BYTES_MAX + small
+
+    step(16, False)
+    step(8, True)
 
 
 @pytest.mark.parametrize("N,B,K", [(64, 9, 4), (256, 5, 1), (512, 2, 8)])
