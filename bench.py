@@ -877,18 +877,16 @@ def bench_diff(args, dev, world, which):
     extra["error"].update(forward_steps=extra["checks"]["forward_steps"], rows=extra["checks"]["rows"],
                           tol={"forward": 1e-5, "grad": 1e-4},
                           vs="FP64 loop on the host (torch corrector in float64, oracle step), FP64 central FD")
-    if which == "ks_diff":  # the general path's spectral convolution layer against the HBM peak
-        extra["roofline"] = spectral_layer_roofline(dev, B, N)
-    if which == "burgers_diff":  # the fused corrector rollout's FP32 work against the FP32 FMA peak
-        from inc_b200.roofline import burgers_cnn_flops_per_cell_step
-        fpc = burgers_cnn_flops_per_cell_step(cfg["scheme"])
-        achieved = cells * fpc / (ms(t_fwd) * 1e-3) / 1e12
-        peak = fp32_peak_tflops(dev)
+    if which == "ks_diff":  # the corrector's evaluation against the HBM peak
+        extra["roofline"] = fno_forward_roofline(dev, net, B, N)
+    if which == "burgers_diff":  # the fused corrector rollout's matrix products against the tensor peak
+        from inc_b200.roofline import CNN_TENSOR_FLOPS_PER_CELL
+        achieved = cells * CNN_TENSOR_FLOPS_PER_CELL / (ms(t_fwd) * 1e-3) / 1e12
+        peak, src = tensor_peak_tflops()
         extra["fused_inference_roofline"] = {
-            "kernel": "inc_burgers_cnn_rollout (k_cnn_rollout<256>)", "bound": "fp32", "achieved": achieved,
-            "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None, "flops_per_cell_step": fpc,
-            "note": "FP32 work; the hidden layers' part runs on the tensor cores, so this can exceed 1",
-            "peak_source": "FP32 FMA loop (inc_bench_fma) measured in this run"}
+            "kernel": "inc_burgers_cnn_rollout (k_cnn_rollout<256>)", "bound": "tensor", "achieved": achieved,
+            "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
+            "flops_per_cell_step": CNN_TENSOR_FLOPS_PER_CELL, "peak_source": src}
     cfg = dict(name=which, B=B, N=N, steps=steps, scheme=cfg["scheme"],
                corrector=("PeriodicCNN1D(4x32ch,k5,GELU)" if which == "burgers_diff" else "FNO1D(L=100, modes=16, width=64), the reference's corrector"))
     del graph, graphed  # a CUDA graph holding NCCL calls must be released before the process group
@@ -920,46 +918,48 @@ def hbm_peak_gbs():
         return 6650.0, "fallback (6.65 TB/s, an earlier copy-bandwidth measurement on this pool)"
 
 
-def spectral_layer_roofline(dev, B, N, W=64, M=16):
-    """One FNO layer's spectral(x) + bias + 1x1 branch (inc_spectral_conv1d) at the workload's shape,
-    timed alone, against the HBM peak.  Algorithmic bytes: x, addend and y (12 B per point), the rfft
-    modes and the mixed modes each written and read (32 B per mode), the weights read, relaid and
-    read (24 B per weight entry).  Inputs exceed L2 (192 MB of activations); the calls are replayed from
-    a CUDA graph so that the time is the device's."""
+def tensor_peak_tflops():
+    """(dense 16-bit TFLOP/s, source): the driver-measured bf16 burst when MEASURED_PEAKS.json holds it, else
+    the pool's earlier measurement."""
+    path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")
+    try:
+        with open(path) as f:
+            v = float(json.load(f)["bf16_tflops"])
+        return v, "measured (MEASURED_PEAKS.json bf16_tflops)"
+    except (OSError, KeyError, ValueError, TypeError):
+        return 1590.0, "fallback (1.59 PFLOP/s, an earlier cuBLAS bf16 measurement on this pool)"
+
+
+def fno_forward_roofline(dev, net, B, N):
+    """The corrector's evaluation (inc_fno_forward) at the workload's shape, timed alone, against the HBM
+    peak.  Bytes: the [B, width, N] state's 11 passes (the first layer writes it, the other three read
+    and write it, the transforms to the modes read it three times, the projection once) and u
+    and y.  The state exceeds the L2; calls are replayed from a CUDA graph so that the time is
+    the device's."""
     import torch
-    from inc_b200.correctors import spectral_conv1d
-    g = torch.Generator(device=dev).manual_seed(0)
-    x = torch.randn(B, W, N, device=dev, generator=g)
-    add = torch.randn(B, W, N, device=dev, generator=g)
-    wr = torch.rand(W, W, M, device=dev, generator=g) / (W * W)
-    wi = torch.rand(W, W, M, device=dev, generator=g) / (W * W)
-    bias = torch.randn(W, device=dev, generator=g)
-    reps = 10  # layer calls per graph replay: device time without the host's per-call work
+    u = torch.randn(B, N, device=dev, generator=torch.Generator(device=dev).manual_seed(0))
+    reps = 10  # calls per graph replay: device time without the host's per-call work
     with torch.no_grad():
         side = torch.cuda.Stream(dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):
             for _ in range(3):
-                spectral_conv1d(x, wr, wi, M, bias=bias, addend=add)
+                net(u)
         torch.cuda.current_stream(dev).wait_stream(side)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             for _ in range(reps):
-                spectral_conv1d(x, wr, wi, M, bias=bias, addend=add)
+                net(u)
         graph.replay()
         torch.cuda.synchronize()
         t = event_time(graph.replay, 10)
     ms = sum(t) / len(t) / reps
-    nbytes = 12 * B * W * N + 32 * B * W * M + 24 * W * W * M
+    nbytes = 4 * B * N * (11 * net.width + 2)
     achieved = nbytes / (ms * 1e-3) / 1e9
     peak, src = hbm_peak_gbs()
-    # ncu dram__bytes_read.sum + dram__bytes_write.sum of the four kernels at this shape
-    # (profiles/fno_spectral_conv_b512_w64_n512_full.md); outputs still in L2 at the end of a
-    # launch are not counted there
-    traffic = 167.8e6 if (B, N, W, M) == (512, 512, 64, 16) else None
-    return {"kernel": "FNO spectral conv layer forward: k_sc_modes, k_sc_weights, k_sc_mix, k_sc_inverse",
+    return {"kernel": "inc_fno_forward: k_fno_prep, k_fno_modes, k_fno_mix, k_fno_layer, k_fno_proj",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "bytes_per_launch": nbytes, "ms_per_launch": ms, "peak_source": src}
+            "traffic": None, "bytes_per_launch": nbytes, "ms_per_launch": ms, "peak_source": src}
 
 
 def diff_checks(which, net, cfg, dev, rows=4, fwd_steps=10, grad_steps=8, directions=4, h=1e-6):

@@ -63,3 +63,7 @@ CNN_FLOPS_PER_CELL = 2 * (32 * 5 + 2 * 32 * 32 * 5 + 32 * 5)
 
 def burgers_cnn_flops_per_cell_step(scheme: str = "ssprk3") -> int:
     return CNN_FLOPS_PER_CELL + BURGERS_FLOPS[scheme]
+
+
+# The hidden layers on the tensor cores: eight products of 16-bit pieces for one FP32 product.
+CNN_TENSOR_FLOPS_PER_CELL = 8 * 2 * (2 * 32 * 32 * 5)
