@@ -10,9 +10,10 @@ While the hidden layers' pre-activations of every step, twice, fit ``ACTS_BYTES_
 forward records them and every state, and the backward is
 ``inc_burgers_cnn_rollout_bwd_states``: the solver's and the network's adjoint in
 reverse, then the weight gradients over all cells and steps, on the tensor cores,
-with no replay.  Longer records are not kept, and the backward is
-``inc_burgers_cnn_rollout_bwd``: segment replay from checkpoints, the activations
-recomputed in shared memory, everything in one kernel.  Weight gradients are summed in
+with no replay.  Up to twice as long a record is read by
+``inc_burgers_cnn_rollout_bwd_acts``, which needs no memory beside it: segment replay of
+the states from checkpoints, everything in one kernel.  Longer records are not kept, and
+``inc_burgers_cnn_rollout_bwd`` recomputes the activations as well.  Weight gradients are summed in
 a fixed order either way.  ``simulate_rollout`` dispatches here by
 itself when the model and solver qualify (``cnn_supported`` /
 ``cnn_train_supported``); otherwise it keeps the per-step loop.
@@ -68,10 +69,10 @@ def pack_cnn_weights(model, device=None) -> torch.Tensor:
 
 CNN_TRAIN_N = CNN_N
 MAX_CKPT_EVERY = 32
-# Largest memory (bytes) that the training path takes for the hidden layers' pre-activations: the
-# record, 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps, and as
-# much again for the layers' adjoints while the backward runs.  That training step is 1.99 ms
-# with the record, 3.80 with the replay (4.47 when the replay's forward ran on the FP32 pipes).
+# Largest memory (bytes) that the training path takes for the hidden layers' pre-activations.  The
+# record is 2 x 32 x n floats per row and step, 537 MB for 256 rows x 256 cells x 32 steps; the
+# tensor-core backward takes as much again for the layers' adjoints while it runs.  That training
+# step is 1.97 ms with both, 3.76 with the record alone (replayed states), 4.86 with neither.
 ACTS_BYTES_MAX = 4 << 30
 
 
@@ -116,18 +117,20 @@ class BurgersCNNRolloutFn(torch.autograd.Function):
         w = _pack_params(params, u0.device)
         frames = torch.empty(B, steps, N, device=u0.device, dtype=torch.float32)
         corr = torch.empty_like(frames)
-        # the hidden layers' pre-activations and the state of every step, kept for the backward
-        # when they and their adjoints fit ACTS_BYTES_MAX (else the backward replays segments and
-        # recomputes them)
-        acts = None
-        if 2 * (B * steps * 2 * 32 * N * 4) <= ACTS_BYTES_MAX:
+        # the hidden layers' pre-activations of every step, kept for the backward when they fit
+        # ACTS_BYTES_MAX, and every state when their adjoints fit it too (else the backward replays
+        # the states from checkpoints)
+        acts, size = None, B * steps * 2 * 32 * N * 4
+        states = 2 * size <= ACTS_BYTES_MAX
+        if size <= ACTS_BYTES_MAX:
             acts = torch.empty(B, steps, 2, 32, N, device=u0.device, dtype=torch.float32)
+        if states:
             ckpt_every = 1
         nseg = (steps + ckpt_every - 1) // ckpt_every
         ckpts = torch.empty(B, nseg, N, device=u0.device, dtype=torch.float32)
         launch.cnn_rollout(w, u0, steps, frames, corr, None, ckpt_every, ckpts, acts=acts)
         ctx.save_for_backward(ckpts, corr, w, acts)
-        ctx.launch, ctx.steps, ctx.ckpt_every, ctx.shape = launch, steps, ckpt_every, (B, N)
+        ctx.launch, ctx.steps, ctx.ckpt_every, ctx.shape, ctx.states = launch, steps, ckpt_every, (B, N), states
         return frames, corr
 
     @staticmethod
@@ -139,11 +142,12 @@ class BurgersCNNRolloutFn(torch.autograd.Function):
         g_w = torch.empty(nat.INC_CNN_WEIGHT_FLOATS, device=dev, dtype=torch.float32)
         gf = None if g_frames is None else g_frames.contiguous()
         gc = None if g_corr is None else g_corr.contiguous()
-        if acts is not None:
+        if ctx.states:
             ctx.launch.cnn_rollout_bwd_states(w, ckpts, corr, ctx.steps, gf, gc, None, g_u0, g_w, acts)
         else:
             work = torch.empty(B, nat.INC_CNN_WEIGHT_FLOATS, device=dev, dtype=torch.float32)
-            ctx.launch.cnn_rollout_bwd(w, ckpts, corr, ctx.steps, ctx.ckpt_every, gf, gc, None, g_u0, g_w, work)
+            ctx.launch.cnn_rollout_bwd(w, ckpts, corr, ctx.steps, ctx.ckpt_every, gf, gc, None, g_u0, g_w, work,
+                                       acts=acts)
         return (g_u0, None, None, None) + unpack_cnn_grads(g_w)
 
 
@@ -160,8 +164,8 @@ def burgers_cnn_rollout(model, solver, u0, steps, corrections=True, ckpt_every=8
 
     With gradients enabled (and u0 or the model's parameters requiring them) the
     result is differentiable through the fused backward (n = 64, 128, 256 or 512), which
-    replays ckpt_every-step segments where the record of every step is not kept
-    (``ACTS_BYTES_MAX``).  Advances ``solver.t`` by steps * dt and
+    replays ckpt_every-step segments where the record of every step and the backward's scratch
+    do not fit ``ACTS_BYTES_MAX``.  Advances ``solver.t`` by steps * dt and
     leaves the last correction in ``solver.correction_s``, like the per-step loop."""
     if not cnn_supported(model, solver, u0):
         raise ValueError("burgers_cnn_rollout: needs a PeriodicCNN1D(32, 5, 4) corrector, a fixed-dt "

@@ -406,14 +406,15 @@ def test_fused_training_last_bias_gradient(cuda, B, N, steps):
 
 
 def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
-    """ACTS_BYTES_MAX bounds the record and what the backward adds to it: a rollout whose record alone
-    would fit (25 of 40 MB) is replayed, one of half its rows is recorded."""
+    """ACTS_BYTES_MAX bounds the record and what the backward adds to it: with a record of 13 of 40 MB the
+    tensor-core backward runs, with 25 the one that replays beside the record, with 50 none is
+    kept."""
     from inc_b200 import fused
     from inc_b200.solvers import BurgersSolverTorch
     N, steps = 256, 24
     monkeypatch.setattr(fused, "ACTS_BYTES_MAX", 40 * 10 ** 6)
 
-    def step(B, recorded):
+    def step(B, recorded, states):
         net = _net(2).float().to(cuda)
         solver = BurgersSolverTorch(_sim_params(_params(N, B=B), B, "ssprk3", cuda))
         u0 = torch.tensor(_u0(B, N, seed=1), dtype=torch.float32, device=cuda, requires_grad=True)
@@ -421,14 +422,15 @@ def test_fused_training_memory_stays_within_its_bound(cuda, monkeypatch):
         base = torch.cuda.memory_allocated(cuda)
         torch.cuda.reset_peak_memory_stats(cuda)
         f, _ = fused.burgers_cnn_rollout(net, solver, u0, steps)
-        assert (f.grad_fn.saved_tensors[3] is not None) == recorded
+        assert (f.grad_fn.saved_tensors[3] is not None) == recorded and f.grad_fn.states == states
         f.sum().backward()
         # beside the bound: frames, corrections, states and their adjoints, weight-gradient scratch
         small = 6 * B * steps * N * 4 + 200 * 4 * fused.nat.INC_CNN_WEIGHT_FLOATS
         assert torch.cuda.max_memory_allocated(cuda) - base < fused.ACTS_BYTES_MAX + small
 
-    step(16, False)
-    step(8, True)
+    step(8, True, True)
+    step(16, True, False)
+    step(32, False, False)
 
 
 @pytest.mark.parametrize("N,B,K", [(64, 9, 4), (256, 5, 1), (512, 2, 8)])
