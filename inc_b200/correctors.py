@@ -327,7 +327,7 @@ class FNO1D(nn.Module):
     ``get_grid(x, L if L is not None else self.L)``.
 
     Calls that ``_fused`` accepts run as one native forward (``FNOFn``): 512 x 512, width 64,
-    16 modes 893 -> 340 us, forward and backward of 201 x 256 2,520 -> 650 us; every size it
+    16 modes 893 -> 359 us, forward and backward of 201 x 256 2,520 -> 650 us; every size it
     covers was faster than the general path, down to 2 x 64.  The others are
     computed with the hidden state kept [B, width, D]
     (contiguous) from the lift to the projection: the Linear layers act on the channel

@@ -11,18 +11,19 @@
 // Layout: one thread per cell, one row per CTA (two for rows of 64 cells).  The first
 // layer (5 products per channel) and the last (5 partial sums per cell, exchanged once)
 // run on the FP32 pipes from registers; the hidden layers are matrix products on the
-// tensor cores (burgers_cnn_tc.cuh), with three-piece operands whose rounding is below
-// that of an FP32 multiply-add chain (tc.cuh).  A thread turns its cell's 32
-// activations into pieces with one power-of-two scale per row (the row's max |a|, one
-// warp reduction and one barrier), one thread issues the products tile by tile, and each
-// thread reads its cell's 32 sums back from tensor memory.
+// tensor cores (burgers_cnn_tc.cuh), with three-piece operands that keep every element's
+// FP32 accuracy (tc.cuh).  A thread turns its cell's 32 activations into pieces with one
+// power-of-two scale per row (the largest finite |a| of the row, one warp reduction and one
+// barrier), one thread issues the products tile by tile, and each thread reads its
+// cell's 32 sums back from tensor memory.
 //
 // What bounds a step: a chain.  With two rows of 256 cells on an SM a step takes about
-// 27,000 clocks: 2 x 5,500 from issuing a layer's products to their end (1,490 per tile,
-// four tiles in turn), 2 x 2,200 in the split and its stores, 2 x 2,500 in reading and
-// GELU, 2,500 in the first layer and 4,000 in the solver's step.  256 x 256 x 32 steps:
-// 426 us, against 1,154 with all four layers on the FP32 pipes.  Issuing a layer's
-// products in two channel halves, the first beside the second's split, measured 429.
+// 28,700 clocks: the four tiles' products in turn (1,640 each, per layer), the split and its
+// stores (about 2 x 2,300), reading and GELU (2 x 2,800), 2,500 in the first layer and 4,000
+// in the solver's step.  256 x 256 x 32 steps: 467 us, against 1,154 with all four layers on
+// the FP32 pipes.  With bf16 pieces, six products and one scale per weight matrix it was 426,
+// and lost small operands' digits (tc.cuh).  Issuing a layer's products in two channel
+// halves, the first beside the second's split, measured no faster (429 against 426).
 #include "burgers_cnn_tc.cuh"
 
 namespace inc {

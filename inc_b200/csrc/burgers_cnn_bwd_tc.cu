@@ -11,7 +11,8 @@
 //                  step go to memory with the channels' maxima.  No replay: every u_k is
 //                  recorded.  Bound by the chain of a step (the solver's adjoint, four row
 //                  reductions and products waited for; issue slots half used at 16 warps an
-//                  SM, all its registers taken): 865 us at 256 rows x 256 cells x 32 steps.
+//                  SM, all its registers taken): 920 us at 256 rows x 256 cells x 32 steps
+//                  (865 with bf16 pieces, one scale per weight matrix and maxima by row).
 //   k_cnn_wgrad    the hidden layers' weight gradients, dW[co][ci][k] = sum dz[co][x] a[ci][x + k -
 //                  2] over all cells, steps and rows: cells are the contraction, so the
 //                  same tile layout serves read by columns, a tap is again a start
@@ -395,18 +396,19 @@ __global__ void __launch_bounds__(TcCfg<N>::T, N == 512 ? 1 : 2) k_cnn_adjoint(A
 // channel of dz and of a (the channel's maximum over the group), then the sums are read once.
 // (A scale per group alone leaves a small channel's sums in the orders from 1 up, where the
 // accumulator truncates at each of the 64 instructions: 1.3e-6 of the channel's gradient
-// against 1.3e-7 in FP32.)  Lanes are (piece of dz,
-// co), columns (tap, piece of a, ci); the nine piece pairs are added in registers, each with its
-// order's power of two.  dz is scaled to 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
+// against 1.3e-7 in FP32.)  Lanes are (piece of dz, co), columns (tap, piece of a, ci); the
+// nine piece pairs are added in registers, each with its order's power of two.  dz is scaled to
+// 64, so that a group's 1024 terms of hi.hi stay below 2^24 (tc.cuh).
 // Even blocks take layer 2 (a = gelu(z1), z1 from the recorded state), odd ones layer 3.
 // The bias gradient is one more block of columns (a = 1).  16 warps prepare the two operand
 // tiles (two buffers), a 17th issues.  Bound by the preparation (about 5,500 clocks a unit: two
 // loads' latency, the split, GELU and the stores) and the reading of a group's sums, which
-// the products of the group wait for; the products take 80 x 56 clocks.  709 us for 256 rows x
-// 256 cells x 32 steps in its first form; 629 with an elected issuer (tc::elect); 440 with
-// the sums read without branches and the bias gradient out of the registers; 432 with the
-// next unit's lines fetched to the L2.  Not faster: 8 warps with the next values held in
-// registers (432), 16 with them (478, spills), the sums kept in memory (707).
+// the products of the group wait for; the products take 80 x 56 clocks.  256 rows x 256 cells x 32
+// steps: 709 us in its first form; 629 with an elected issuer (tc::elect); 440 with the sums read
+// without branches and the bias gradient out of the registers; 432 with the next unit's
+// lines fetched to the L2; 475 with fp16 pieces (a longer split) and the channels' scales.  Not
+// faster, measured against 432: 8 warps with the next values held in registers (432), 16 with
+// them (478, spills), the sums kept in memory (707).
 constexpr int WG = 512;
 constexpr int GROUP = 4;
 struct CnnWgradArgs {

@@ -22,8 +22,9 @@ int check_fno(const inc_fno_desc* d);  // fno_fwd.cu
 
 // ---- projection -------------------------------------------------------------------------
 // Bound, like the forward's, by the GELUs (with their derivative) and three rounds of products
-// per tile, each waited for; 100 MB written.  51 us at 256 x 64 x 512.  Letting one of the
-// eight warps issue (128 registers in place of 96, no spills) measured 52.
+// per tile, each waited for; 100 MB written.  56 us at 256 x 64 x 512 (51 with six products of bf16
+// pieces; letting one of the eight warps issue, 128 registers in place of 96 and no spills,
+// measured 52 then).
 struct ProjBwdArgs {
     const float* x;      // z of the last layer [batch][W][N]
     const float* xmax;   // [tiles per row][batch]
@@ -280,7 +281,7 @@ int launch_proj_bwd(const ProjBwdArgs& a, int* blocks, cudaStream_t st) {
 // 16 warps split; the last of them also issues (8 or 12 instructions per chunk).  A 17th warp
 // for that cost every thread 32 registers (128 -> 96), and reading the sums before the next
 // unit started left the tensor cores idle: 33 -> 30 us (64 x 64) and 37 -> 35 us (128 x 64) at
-// 256 rows of 512 points.
+// 256 rows of 512 points (31.5 and 38.2 since fp16 pieces and their eight products).
 struct WgradArgs {
     const float* g;      // [batch][MO][n]
     const float* gmax;   // [tiles per row][batch]

@@ -11,7 +11,7 @@
 //
 // What bounds it: reading and writing the state (11 passes of 67 MB at 512 x 64 x 512, 114 us
 // at the measured copy rate) and, beside it, the splits and GELUs of every element and 13
-// launches' starts: 340 us there, against 893 for batched FP32 matmuls, spectral-convolution
+// launches' starts: 359 us there, against 893 for batched FP32 matmuls, spectral-convolution
 // kernels and elementwise passes on the same state.
 #include "fno_tc.cuh"
 
@@ -43,7 +43,7 @@ struct ProjSmem {
 // y[p] = b2 + sum_j w2[j] gelu(b1[j] + sum_c w1[j][c] x[c][p]): the 128 hidden values of a
 // point live in its tensor-memory lane and the registers of its two threads only.  Bound by
 // those GELUs on the FMA pipe (16,384 per tile: 850 clocks per 16 columns with two CTAs) and
-// the products (1,540 clocks per tile): 40 us at 512 x 64 x 512.
+// the products (2,050 clocks per tile): 44 us at 512 x 64 x 512.
 template <int W, int N>
 __global__ void __launch_bounds__(THREADS, 2) k_fno_proj(ProjArgs a) {
     extern __shared__ __align__(128) unsigned char fno_smem[];

@@ -4,8 +4,10 @@
 // The network's contractions are products over channels (the layers' 1x1 branches, the
 // projection) and, for the Fourier branch with its few kept modes, products with a
 // [2 modes x points] table of cosines and sines: a transform to the modes and back is a
-// thin matrix product beside the 1x1 branch's.  All of them are FP32-accurate
-// three-piece tcgen05 products (tc.cuh).
+// thin matrix product beside the 1x1 branch's.  All of them are three-piece tcgen05
+// products that keep FP32's accuracy (tc.cuh).  Two CTAs of an SM with two tiles each in
+// flight leave a tile 2 W accumulator columns, so the orders of the pieces' products from 1 up
+// share W of them (issue_stage).
 //
 // A tile of k_fno_layer is 128 points (64 for rows of 64) of one trajectory with all W
 // channels.  The [W][n] state puts a point's channels n apart: two threads per point
@@ -20,9 +22,11 @@
 //
 // What bounds a layer: the loads' latency at the start of a launch (4,000 to 12,000 clocks
 // until the first tile and the images are there), then the splits and GELUs beside the
-// loads.  512 x 64 x 512: 43.5 us for 134 MB read and written (20.8 us at the copy rate); a
-// batched FP32 matmul, a spectral convolution and a GELU pass took about 150.  Programmatic launch
-// overlap, an L2 prefetch of later tiles and 16 warps a CTA measured no faster.
+// loads, and the products (2,110 clocks per tile at W = 64).  512 x 64 x 512: 47.5 us for 134 MB
+// read and written (20.8 us at the copy rate; 43.5 with six products of bf16 pieces, which
+// lost small operands' digits); a batched FP32 matmul, a spectral convolution and a GELU pass
+// took about 150.  Programmatic launch overlap, an L2 prefetch of later tiles and 16 warps a CTA
+// measured no faster.
 //
 // The modes of a state are a launch of their own (k_fno_modes) with the points as the
 // contraction: taking them in the layer's epilogue instead (a second split and product per
@@ -309,7 +313,7 @@ struct LayerSmem {
 // Who issues: in the forward a ninth warp; in the adjoint the last of the eight, which leaves a
 // thread 128 registers in place of 96 and with them room to load zprev a tile ahead (256 x 64 x
 // 512: 33.2 -> 29.6 us, the first layer's 30.1 -> 24.8; the forward with the lift 18.0 -> 20.3 that
-// way, the others equal).
+// way, the others equal; 32.0 and 26.2 for the adjoints since the operands have fp16 pieces).
 constexpr int layer_threads(int mode) { return mode >= BWD ? WORKERS : THREADS; }
 
 template <int W, int N, bool LIFT, int MODE, bool TRAIN>
@@ -618,8 +622,8 @@ int run_layer(const LayerArgs& a, int n, cudaStream_t st) {
 // splits 8 consecutive points of a row at a time (float4 loads, 256 contiguous bytes per
 // 8 lanes); the planes' pitch of 2064 bytes makes their 16-byte stores conflict-free.
 // 16 warps split (and apply GELU), a 17th issues.  Bound by reading the state and the split:
-// 12.4 us at 256 x 64 x 512 (33.5 MB, 5.2 us at the copy rate; 128 tiles leave 20 SMs idle),
-// 13.9 with GELU, 21.7 at 512 x 64 x 512 (256 tiles on 148 SMs: a second round on 108).
+// 12.8 us at 256 x 64 x 512 (33.5 MB, 5.2 us at the copy rate; 128 tiles leave 20 SMs idle),
+// 14.7 with GELU, 22.1 at 512 x 64 x 512 (256 tiles on 148 SMs: a second round on 108).
 constexpr int MODES_WORKERS = 512;
 constexpr int A_PITCH = 2048 + 16;
 struct ModesArgs {
