@@ -919,15 +919,15 @@ def hbm_peak_gbs():
 
 
 def tensor_peak_tflops():
-    """(dense 16-bit TFLOP/s, source): the driver-measured bf16 burst when MEASURED_PEAKS.json holds it, else
-    the pool's earlier measurement."""
+    """(dense 16-bit TFLOP/s, source): the bf16 burst that MEASURED_PEAKS.json holds, else an earlier
+    measurement."""
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")
     try:
         with open(path) as f:
             v = float(json.load(f)["bf16_tflops"])
         return v, "measured (MEASURED_PEAKS.json bf16_tflops)"
     except (OSError, KeyError, ValueError, TypeError):
-        return 1590.0, "fallback (1.59 PFLOP/s, an earlier cuBLAS bf16 measurement on this pool)"
+        return 1590.0, "fallback (1.59 PFLOP/s, an earlier cuBLAS bf16 measurement)"
 
 
 def fno_forward_roofline(dev, net, B, N):
