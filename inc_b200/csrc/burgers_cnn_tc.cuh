@@ -41,7 +41,7 @@ constexpr int W_PLANE = 96 * 16;
 // tap k holds rows (piece, co), contraction ci.  TRANS: the layer's adjoint, rows
 // (piece, ci), contraction co, taps reversed.  Each row has a scale of its own, so that
 // the products of a row of small weights lie in order 0 as well; returns 2^e / 256 with 2^e >=
-// the max |w| of row threadIdx.x % 32.  Three barriers; dst is scratch before the last.
+// the max |w| of row threadIdx.x % 32.  Two barriers; dst is scratch before the second.
 template <int T, bool TRANS>
 INC_DEV float stage_weights(unsigned char* dst, const float* __restrict__ w) {
     const int row = threadIdx.x % C, warp = threadIdx.x / C;
